@@ -58,7 +58,10 @@ struct SpeciesND {
     float tb[3], sb[3];  // Boris t = hqmdt B and s = 2 t / (1 + t^2)
     float drift[3];    // dt / d_a: cell units per unit velocity
     float dep_fixed;   // dep * rho_scale
-    uint8_t* alive;    // runs with walls and an absorbing side: Particle::alive (null: all alive)
+    // runs with walls and an absorbing side: Particle::alive (null: all alive)
+    uint8_t* alive[2];
+    // FP64 form: Boris h = 0.5 qm dt, t = h B and s = 2 t / (1 + t^2) of a full step in the uniform B
+    double bh, bt[3], bs[3];
     int index;         // species index (loss ledger row)
 };
 
@@ -66,6 +69,7 @@ struct ParamsND {
     int dims;
     int n[3];
     double L[3], d[3];
+    double rd[3];  // 1 / d (cells_of)
     double dt, eps;
     double B[3];
     double rho_scale, inv_rho_scale;
@@ -128,8 +132,11 @@ __device__ __forceinline__ void field_b(const ParamsND& p, const double pos[3], 
 // stays below 2^32), so the density does not depend on particle order.
 constexpr float kWeightScale = 8388608.0f;  // 2^23
 
-// wrap_periodic, src/FieldSolver.cpp:15-17, with the exact fast branch for |x| < 2L
+// wrap_periodic, src/FieldSolver.cpp:15-17, with the exact fast branch for
+// |x| < 2L; a position already inside [0, L) stays as it is (the reference's
+// (x + L) - L rounds its last bits away)
 __device__ __forceinline__ double wrap_periodic(double x, double L) {
+    if (x >= 0.0 && x < L) return x;
     if (!(fabs(x) < 2.0 * L)) return fmod(fmod(x, L) + L, L);
     const double r = x >= L ? x - L : (x <= -L ? x + L : x);
     const double y = r + L;
@@ -141,38 +148,42 @@ struct Axis {
     double f;
 };
 
-// One axis of the periodic CIC stencil, src/Mesh2D.cpp:96-114, src/FieldSolver.cpp:936-960
-__device__ __forceinline__ Axis axis(double x, double L, double d, int n) {
+// One axis of the periodic CIC stencil, src/Mesh2D.cpp:96-114, src/FieldSolver.cpp:936-960.
+// The wrap leaves 0 <= x <= L, so the cell is at most n and i % n is a
+// compare (a NaN converts to cell 0); 64-bit remainders here were most of the
+// FP64 push's instructions.
+__device__ __forceinline__ Axis axis(double x, double L, double d, double rd, int n) {
     const double xp = wrap_periodic(x, L);
-    const double g = xp / d;
-    const unsigned long long i = (unsigned long long)floor(g);
+    const double g = cells_of(xp, d, rd);
+    const int i = (int)floor(g);
     Axis a;
     a.f = g - (double)i;
-    a.i0 = (int)(i % (unsigned long long)n);
-    a.i1 = (int)((i + 1) % (unsigned long long)n);
+    a.i0 = (unsigned)i < (unsigned)n ? i : 0;
+    a.i1 = a.i0 + 1 == n ? 0 : a.i0 + 1;
     return a;
 }
 
 // One axis of the CIC stencil on a wall axis: clamp into [0, L], cell
 // min(floor, n - 2), fraction clamped to [0, 1], src/Mesh2D.cpp:96-129,
 // src/FieldSolver.cpp:926-960
-__device__ __forceinline__ Axis axis_wall(double x, double L, double d, int n) {
+__device__ __forceinline__ Axis axis_wall(double x, double L, double d, double rd, int n) {
     const double c = x < 0.0 ? 0.0 : (L < x ? L : x);
-    const double g = c / d;
-    unsigned long long i = (unsigned long long)floor(g);
-    if (i > (unsigned long long)(n - 2)) i = (unsigned long long)(n - 2);
+    const double g = cells_of(c, d, rd);
+    int i = (int)floor(g);  // (a NaN converts to cell 0)
+    if (i > n - 2) i = n - 2;
     double f = g - (double)i;
     f = f < 0.0 ? 0.0 : (f > 1.0 ? 1.0 : f);
     Axis a;
-    a.i0 = (int)i;
-    a.i1 = (int)i + 1;
+    a.i0 = i;
+    a.i1 = i + 1;
     a.f = f;
     return a;
 }
 
 template <bool WALLS>
 __device__ __forceinline__ Axis axis2(const ParamsND& p, int a, double x) {
-    return (WALLS && p.wall[a]) ? axis_wall(x, p.L[a], p.d[a], p.n[a]) : axis(x, p.L[a], p.d[a], p.n[a]);
+    return (WALLS && p.wall[a]) ? axis_wall(x, p.L[a], p.d[a], p.rd[a], p.n[a])
+                                : axis(x, p.L[a], p.d[a], p.rd[a], p.n[a]);
 }
 
 // 1 / node_area (node_volume) relative to an interior node: 2 on each
@@ -237,38 +248,6 @@ __device__ __forceinline__ void boris(double v[3], const double E[3], const doub
     v[0] = vq0 + h * E[0];
     v[1] = vq1 + h * E[1];
     v[2] = vq2 + h * E[2];
-}
-
-template <int DIM>
-__device__ __forceinline__ void deposit(const ParamsND& p, const SpeciesND& S, const double pos[3]) {
-    const Axis ax = axis(pos[0], p.L[0], p.d[0], p.n[0]);
-    const Axis ay = axis(pos[1], p.L[1], p.d[1], p.n[1]);
-    const int nx = p.n[0];
-    if (DIM == 2) {
-        // q (1 - fx)(1 - fy) / node_area, src/Mesh2D.cpp:131-142 (reciprocal area inside the fixed-point rounding)
-        const double fx = ax.f, fy = ay.f;
-        const double c00 = S.dep * (1.0 - fx) * (1.0 - fy), c10 = S.dep * fx * (1.0 - fy);
-        const double c01 = S.dep * (1.0 - fx) * fy, c11 = S.dep * fx * fy;
-        atomicAdd(p.rho_acc + ay.i0 * nx + ax.i0, (unsigned long long)to_fixed(c00, p.rho_scale));
-        atomicAdd(p.rho_acc + ay.i0 * nx + ax.i1, (unsigned long long)to_fixed(c10, p.rho_scale));
-        atomicAdd(p.rho_acc + ay.i1 * nx + ax.i0, (unsigned long long)to_fixed(c01, p.rho_scale));
-        atomicAdd(p.rho_acc + ay.i1 * nx + ax.i1, (unsigned long long)to_fixed(c11, p.rho_scale));
-    } else {
-        // q_over_volume * shape, src/Mesh3D.cpp:110-122
-        const Axis az = axis(pos[2], p.L[2], p.d[2], p.n[2]);
-        const double wx[2] = {1.0 - ax.f, ax.f}, wy[2] = {1.0 - ay.f, ay.f}, wz[2] = {1.0 - az.f, az.f};
-        const int ii[2] = {ax.i0, ax.i1}, jj[2] = {ay.i0, ay.i1}, kk[2] = {az.i0, az.i1};
-#pragma unroll
-        for (int c = 0; c < 2; ++c)
-#pragma unroll
-            for (int b = 0; b < 2; ++b)
-#pragma unroll
-                for (int a = 0; a < 2; ++a) {
-                    const double shape = wx[a] * wy[b] * wz[c];
-                    atomicAdd(p.rho_acc + ((size_t)kk[c] * p.n[1] + jj[b]) * nx + ii[a],
-                              (unsigned long long)to_fixed(S.dep * shape, p.rho_scale));
-                }
-    }
 }
 
 // CIC deposit of a warp's particles with one atomic per node per run of lanes
@@ -359,9 +338,6 @@ __device__ __forceinline__ void deposit_warp(const ParamsND& p, const SpeciesND&
 
 enum : int { kPushStep = 0, kPushDepositOnly = 1, kPushInitHalf = 2, kPushSync = 3 };
 
-// One particle per thread.  Modes: a full step (kick, drift, wrap, deposit),
-// deposit only (initialize/resume), half-step initialisation from v
-// (initialize_{boris,leapfrog}_half_step) and synchronisation into v.
 // reflect_coordinate, src/Simulation2D.cpp:43-54 (a particle crosses at most a
 // few domain lengths per step; the bound only guards against runaway input)
 __device__ __forceinline__ void reflect_coordinate(double& c, double& v, double L) {
@@ -391,10 +367,13 @@ __device__ __forceinline__ int apply_walls(const ParamsND& p, double x[3], doubl
     return -1;
 }
 
+// One particle per thread.  Modes: deposit only (initialize/resume), half-step
+// initialisation from v (initialize_{boris,leapfrog}_half_step) and
+// synchronisation into v.  (The full step is k_push_run.)
 template <int DIM, bool BORIS, int MODE, bool WALLS = false>
 __global__ void __launch_bounds__(kThreads) k_push(ParamsND p, SpeciesND S, int buf) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
-    const bool valid = i < S.n && (!WALLS || !S.alive || S.alive[i]);
+    const bool valid = i < S.n && (!WALLS || !S.alive[buf] || S.alive[buf][i]);
     if (MODE == kPushInitHalf || MODE == kPushSync) {
         if (!valid) return;
     } else if (blockIdx.x * kThreads + (threadIdx.x & ~31u) >= S.n) {
@@ -434,35 +413,204 @@ __global__ void __launch_bounds__(kThreads) k_push(ParamsND p, SpeciesND S, int 
         for (int a = 0; a < 3; ++a) S.v[a][i] = vh[a];
         return;
     }
-    // kick_boris / kick_leapfrog + drift_leapfrog, src/Pusher.cpp:109-128, :162-174
-    if (BORIS) {
-        double Bp[3];
-        field_b(p, pos, Bp);
-        boris(vh, e, Bp, S.qm, p.dt);
-    } else {
-        for (int a = 0; a < DIM; ++a) vh[a] += S.qm * e[a] * p.dt;
-    }
-    bool absorbed = false;
-    if (WALLS) {
-        for (int a = 0; a < DIM; ++a) pos[a] = pos[a] + vh[a] * p.dt;
-        const int side = valid ? apply_walls<DIM>(p, pos, vh) : -1;
-        if (side >= 0) {
-            absorbed = true;
-            S.alive[i] = 0;
-            atomicAdd(p.losses + 6 * S.index + side, 1ull);
+}
+
+// boris_advance with the species' precomputed h, t and s (uniform B): the same
+// operations as boris(), whose t, s and division depend on B only
+__device__ __forceinline__ void boris_uniform(double v[3], const double E[3], const SpeciesND& S) {
+    const double h = S.bh;
+    const double vm0 = v[0] + h * E[0], vm1 = v[1] + h * E[1], vm2 = v[2] + h * E[2];
+    const double vp0 = vm0 + (vm1 * S.bt[2] - vm2 * S.bt[1]);
+    const double vp1 = vm1 + (vm2 * S.bt[0] - vm0 * S.bt[2]);
+    const double vp2 = vm2 + (vm0 * S.bt[1] - vm1 * S.bt[0]);
+    const double vq0 = vm0 + (vp1 * S.bs[2] - vp2 * S.bs[1]);
+    const double vq1 = vm1 + (vp2 * S.bs[0] - vp0 * S.bs[2]);
+    const double vq2 = vm2 + (vp0 * S.bs[1] - vp1 * S.bs[0]);
+    v[0] = vq0 + h * E[0];
+    v[1] = vq1 + h * E[1];
+    v[2] = vq2 + h * E[2];
+}
+
+enum : int { kNoField = 0, kUniformField = 1, kProfileField = 2 };
+
+// The FP64 step push: kick, drift, particle boundaries and CIC deposit of
+// kRunItems consecutive particles per thread.  Particles are sorted by cell,
+// so the field at a cell's nodes is fetched once per run of equal cells, the
+// fixed-point contributions of a run are summed in registers, a run that ends
+// inside the thread is committed with one atomic per node, and each lane's
+// last run joins a segmented sum over the lanes that end in the same cell.
+// The state moves as 16-byte vectors.  Contributions are integers, so the
+// density does not depend on how particles are grouped.
+// Against one particle per thread with 64-bit index remainders (both species, per
+// step): 2 x 1 M particles on 256 x 128, 81 -> 70 us; 2 x 4.2 M on 64^3,
+// 483 -> 437 us (bound by load latency at 2 CTAs an SM and, between sorts, by the
+// deposit's global atomics); walls, 2 x 2 M on 512 x 513, 161 -> 129 us and
+// 2 x 4.2 M on 129^3, 680 -> 545 us (these also sorted by cell now).
+constexpr int kRunItems = 2;
+
+template <int DIM, int BKIND, bool WALLS>
+__global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, int buf) {
+    constexpr int NN = DIM == 2 ? 4 : 8;
+    const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * kRunItems;
+    const int lane = threadIdx.x & 31;
+    if ((blockIdx.x * kThreads + (threadIdx.x & ~31u)) * kRunItems >= S.n) return;  // whole warp past the end
+    const int nx = p.n[0], ny = p.n[1];
+    double x[kRunItems][3], v[kRunItems][3];
+    bool live[kRunItems];
+    const bool full = first + kRunItems <= S.n;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        double2 q{0.0, 0.0}, w{0.0, 0.0};
+        if (full) {
+            if (a < DIM) q = __ldcs(reinterpret_cast<const double2*>(S.pos[buf][a] + first));
+            w = __ldcs(reinterpret_cast<const double2*>(S.vh[buf][a] + first));
+        } else if (first < S.n) {
+            if (a < DIM) q.x = S.pos[buf][a][first];
+            w.x = S.vh[buf][a][first];
         }
-    } else {
-        for (int a = 0; a < DIM; ++a) {
-            const double c = pos[a] + vh[a] * p.dt;
-            // periodic particle boundary: wrap only outside [0, L], src/Simulation2D.cpp:57-97
-            pos[a] = (c >= 0.0 && c <= p.L[a]) ? c : wrap_periodic(c, p.L[a]);
+        x[0][a] = q.x; x[1][a] = q.y;
+        v[0][a] = w.x; v[1][a] = w.y;
+    }
+#pragma unroll
+    for (int k = 0; k < kRunItems; ++k)
+        live[k] = first + k < S.n && (!WALLS || !S.alive[buf] || S.alive[buf][first + k]);
+    const unsigned kNoCell = 0xFFFFFFFFu;
+    unsigned gcell = kNoCell, rcell = kNoCell;  // cells of the cached field and of the current deposit run
+    double en[NN][DIM];
+    long long racc[NN];
+    unsigned rnode[3] = {0u, 0u, 0u};  // steps from the run's first node to its upper x, y, z neighbours
+#pragma unroll
+    for (int j = 0; j < NN; ++j) racc[j] = 0;
+    auto commit = [&]() {
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+            const unsigned node = rcell + ((j & 1) ? rnode[0] : 0u) + ((j & 2) ? rnode[1] : 0u) + ((j & 4) ? rnode[2] : 0u);
+            if (racc[j]) atomicAdd(p.rho_acc + node, (unsigned long long)racc[j]);
+        }
+    };
+#pragma unroll
+    for (int k = 0; k < kRunItems; ++k) {
+        if (!live[k]) continue;
+        const Axis gx = axis2<WALLS>(p, 0, x[k][0]), gy = axis2<WALLS>(p, 1, x[k][1]);
+        const Axis gz = DIM == 3 ? axis2<WALLS>(p, 2, x[k][DIM - 1]) : Axis{0, 0, 0.0};
+        const unsigned c0 = ((unsigned)gz.i0 * ny + gy.i0) * nx + gx.i0;
+        if (c0 != gcell) {
+            gcell = c0;
+#pragma unroll
+            for (int j = 0; j < NN; ++j) {
+                const unsigned g = ((unsigned)((j & 4) ? gz.i1 : gz.i0) * ny + ((j & 2) ? gy.i1 : gy.i0)) * nx +
+                                   ((j & 1) ? gx.i1 : gx.i0);
+                if (DIM == 2) {
+                    const double2 q = __ldg(reinterpret_cast<const double2*>(p.E) + g);
+                    en[j][0] = q.x; en[j][1] = q.y;
+                } else {
+                    const double2* E = reinterpret_cast<const double2*>(p.E) + 2 * (size_t)g;
+                    const double2 q = __ldg(E);
+                    en[j][0] = q.x; en[j][1] = q.y;
+                    en[j][DIM - 1] = __ldg(reinterpret_cast<const double*>(E + 1));
+                }
+            }
+        }
+        double e[3] = {0.0, 0.0, 0.0};
+        if (DIM == 2) {
+            const double fx = gx.f, fy = gy.f;
+            const double w00 = (1.0 - fx) * (1.0 - fy), w10 = fx * (1.0 - fy), w01 = (1.0 - fx) * fy, w11 = fx * fy;
+            e[0] = en[0][0] * w00 + en[1][0] * w10 + en[2][0] * w01 + en[3][0] * w11;
+            e[1] = en[0][1] * w00 + en[1][1] * w10 + en[2][1] * w01 + en[3][1] * w11;
+        } else {
+            // interpolate_electric(Mesh3D&), src/FieldSolver.cpp:978-1038: loops z, y, x
+            const double wx[2] = {1.0 - gx.f, gx.f}, wy[2] = {1.0 - gy.f, gy.f}, wz[2] = {1.0 - gz.f, gz.f};
+#pragma unroll
+            for (int j = 0; j < NN; ++j) {
+                const double shape = wx[j & 1] * wy[(j >> 1) & 1] * wz[(j >> 2) & 1];
+#pragma unroll
+                for (int a = 0; a < DIM; ++a) e[a] += en[j][a] * shape;
+            }
+        }
+        // kick_boris / kick_leapfrog + drift_leapfrog, src/Pusher.cpp:109-128, :162-174
+        if (BKIND == kUniformField) {
+            boris_uniform(v[k], e, S);
+        } else if (BKIND == kProfileField) {
+            double Bp[3];
+            field_b(p, x[k], Bp);
+            boris(v[k], e, Bp, S.qm, p.dt);
+        } else {
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) v[k][a] += S.qm * e[a] * p.dt;
+        }
+        if (WALLS) {
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) x[k][a] = x[k][a] + v[k][a] * p.dt;
+            const int side = apply_walls<DIM>(p, x[k], v[k]);
+            if (side >= 0) {
+                S.alive[buf][first + k] = 0;
+                atomicAdd(p.losses + 6 * S.index + side, 1ull);
+                continue;
+            }
+        } else {
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) {
+                const double c = x[k][a] + v[k][a] * p.dt;
+                // periodic particle boundary: wrap only outside [0, L], src/Simulation2D.cpp:57-97
+                x[k][a] = (c >= 0.0 && c <= p.L[a]) ? c : wrap_periodic(c, p.L[a]);
+            }
+        }
+        // deposit at the pushed position into the run of its cell (the contributions of deposit_warp)
+        const Axis ax = axis2<WALLS>(p, 0, x[k][0]), ay = axis2<WALLS>(p, 1, x[k][1]);
+        const Axis az = DIM == 3 ? axis2<WALLS>(p, 2, x[k][DIM - 1]) : Axis{0, 0, 0.0};
+        const unsigned c1 = ((unsigned)az.i0 * ny + ay.i0) * nx + ax.i0;
+        if (c1 != rcell) {
+            if (rcell != kNoCell) commit();
+            rcell = c1;
+            rnode[0] = (unsigned)(ax.i1 - ax.i0);
+            rnode[1] = (unsigned)((ay.i1 - ay.i0) * nx);
+            if (DIM == 3) rnode[2] = (unsigned)((az.i1 - az.i0) * ny * nx);
+#pragma unroll
+            for (int j = 0; j < NN; ++j) racc[j] = 0;
+        }
+        const double ux[2] = {1.0 - ax.f, ax.f}, uy[2] = {1.0 - ay.f, ay.f}, uz[2] = {1.0 - az.f, az.f};
+#pragma unroll
+        for (int j = 0; j < NN; ++j) {
+            double c = DIM == 2 ? S.dep * ux[j & 1] * uy[(j >> 1) & 1]
+                                : S.dep * (ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1]);
+            if (WALLS) {  // q shape / node volume over the wall nodes' half cells
+                double f = area_factor<WALLS>(p, 0, (j & 1) ? ax.i1 : ax.i0) *
+                           area_factor<WALLS>(p, 1, (j & 2) ? ay.i1 : ay.i0);
+                if (DIM == 3) f *= area_factor<WALLS>(p, 2, (j & 4) ? az.i1 : az.i0);
+                c *= f;
+            }
+            racc[j] += to_fixed(c, p.rho_scale);
         }
     }
-    if (valid) {
-        for (int a = 0; a < DIM; ++a) S.pos[buf][a][i] = pos[a];
-        for (int a = 0; a < 3; ++a) S.vh[buf][a][i] = vh[a];
+    // the state back, in place
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (full) {
+            if (a < DIM) __stcs(reinterpret_cast<double2*>(S.pos[buf][a] + first), make_double2(x[0][a], x[1][a]));
+            __stcs(reinterpret_cast<double2*>(S.vh[buf][a] + first), make_double2(v[0][a], v[1][a]));
+        } else if (first < S.n) {
+            if (a < DIM) S.pos[buf][a][first] = x[0][a];
+            S.vh[buf][a][first] = v[0][a];
+        }
     }
-    deposit_warp<DIM, WALLS>(p, S, pos, valid && !absorbed);
+    // each lane's last run, summed over segments of at most RSEG lanes that end in the same cell
+    constexpr int RSEG = DIM == 3 ? 4 : 8;
+    const unsigned prev = __shfl_up_sync(0xffffffffu, rcell, 1);
+    const bool head = (lane & (RSEG - 1)) == 0 || prev != rcell;
+    const unsigned heads = __ballot_sync(0xffffffffu, head);
+    const int start = 31 - __clz(heads & (0xFFFFFFFFu >> (31 - lane)));
+    const bool tail = lane == 31 || ((heads >> (lane + 1)) & 1u);
+#pragma unroll
+    for (int j = 0; j < NN; ++j) {
+        long long q = racc[j];
+#pragma unroll
+        for (int d = 1; d < RSEG; d <<= 1) {
+            const long long t = __shfl_up_sync(0xffffffffu, q, d);
+            if (lane - d >= start) q += t;
+        }
+        racc[j] = q;
+    }
+    if (tail && rcell != kNoCell) commit();
 }
 
 // walls: fixed-point density to FP64 (the accumulator is cleared for the
@@ -1054,7 +1202,7 @@ __global__ void k_to_fp32(ParamsND p, SpeciesND S, int buf) {
     if (i >= S.n) return;
     int ii[3] = {0, 0, 0};
     for (int a = 0; a < DIM; ++a) {
-        const Axis ax = axis(S.pos[buf][a][i], p.L[a], p.d[a], p.n[a]);
+        const Axis ax = axis(S.pos[buf][a][i], p.L[a], p.d[a], p.rd[a], p.n[a]);
         float f = (float)ax.f;
         int k = ax.i0;
         if (f >= 1.0f) { f = 0.0f; k = ax.i1; }
@@ -1136,24 +1284,33 @@ __global__ void k_cell_gather32(SpeciesND S, int from) {
 
 // ---- particle sort by cell -------------------------------------------------------
 
-template <int DIM>
+template <int DIM, bool WALLS>
 __device__ __forceinline__ unsigned cell_of(const ParamsND& p, const double pos[3]) {
-    const Axis ax = axis(pos[0], p.L[0], p.d[0], p.n[0]);
-    const Axis ay = axis(pos[1], p.L[1], p.d[1], p.n[1]);
+    const Axis ax = axis2<WALLS>(p, 0, pos[0]);
+    const Axis ay = axis2<WALLS>(p, 1, pos[1]);
     unsigned c = (unsigned)ay.i0 * p.n[0] + ax.i0;
     if (DIM == 3) {
-        const Axis az = axis(pos[2], p.L[2], p.d[2], p.n[2]);
+        const Axis az = axis2<WALLS>(p, 2, pos[2]);
         c += (unsigned)az.i0 * p.n[0] * p.n[1];
     }
     return c;
 }
 
-template <int DIM>
+// Runs with walls keep their absorbed particles (their positions can be read
+// back) in one bin after the last cell, so the push meets them in whole warps.
+template <int DIM, bool WALLS>
+__device__ __forceinline__ unsigned bin_of(const ParamsND& p, const SpeciesND& S, int buf, unsigned i,
+                                           const double pos[3]) {
+    if (WALLS && S.alive[buf] && !S.alive[buf][i]) return (unsigned)(p.n[0] * p.n[1] * (DIM == 3 ? p.n[2] : 1));
+    return cell_of<DIM, WALLS>(p, pos);
+}
+
+template <int DIM, bool WALLS>
 __global__ void k_cell_hist(ParamsND p, SpeciesND S, int buf, unsigned* count) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= S.n) return;
     const double pos[3] = {S.pos[buf][0][i], S.pos[buf][1][i], DIM == 3 ? S.pos[buf][2][i] : 0.0};
-    atomicAdd(count + cell_of<DIM>(p, pos), 1u);
+    atomicAdd(count + bin_of<DIM, WALLS>(p, S, buf, i, pos), 1u);
 }
 
 // exclusive scan of `count` (n entries) into `offset`, three launches
@@ -1217,7 +1374,7 @@ __global__ void k_scan_add(unsigned* offset, const unsigned* block_sums, unsigne
         if (base + k < n) offset[base + k] += add;
 }
 
-template <int DIM>
+template <int DIM, bool WALLS>
 __global__ void k_cell_scatter(ParamsND p, SpeciesND S, int from, unsigned* cursor) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i >= S.n) return;
@@ -1227,10 +1384,12 @@ __global__ void k_cell_scatter(ParamsND p, SpeciesND S, int from, unsigned* curs
     const double pos[3] = {S.pos[from][0][i], S.pos[from][1][i], DIM == 3 ? S.pos[from][2][i] : 0.0};
     const double vh[3] = {S.vh[from][0][i], S.vh[from][1][i], S.vh[from][2][i]};
     const unsigned id = S.id[from][i];
-    const unsigned o = atomicAdd(cursor + cell_of<DIM>(p, pos), 1u);
+    const uint8_t alive = WALLS && S.alive[from] ? S.alive[from][i] : 1;
+    const unsigned o = atomicAdd(cursor + bin_of<DIM, WALLS>(p, S, from, i, pos), 1u);
     for (int a = 0; a < DIM; ++a) S.pos[to][a][o] = pos[a];
     for (int a = 0; a < 3; ++a) S.vh[to][a][o] = vh[a];
     S.id[to][o] = id;
+    if (WALLS && S.alive[to]) S.alive[to][o] = alive;
 }
 
 // Device-side loading for large runs: uniform positions displaced by
@@ -1274,7 +1433,8 @@ __global__ void k_load_maxwellian(SpeciesND S, int buf, int dims, unsigned n, ui
 }
 
 // Read-back in load order: dst[id[i]] = src[i].
-__global__ void k_unpermute(const unsigned* id, const double* src, double* dst, unsigned n) {
+template <class T>
+__global__ void k_unpermute(const unsigned* id, const T* src, T* dst, unsigned n) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
     if (i < n) dst[id[i]] = src[i];
 }
@@ -1807,7 +1967,7 @@ constexpr size_t f256_smem(int mode) {
 // kinetic energy of v per species and field energy / charge_l1 of the grid;
 // per-block partials, the last block adds them in block order.
 constexpr int kSampleBlocks = 148;
-__global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, int dims, double* partial, unsigned* done,
+__global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, const uint8_t* alive, int dims, double* partial, unsigned* done,
                                                    double* out, const double* E, const double* rho,
                                                    long long N, double half_eps_vol, double vol, int species,
                                                    int last_species, int wall_x, int wall_y, int wall_z, int nx,
@@ -1817,7 +1977,7 @@ __global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, int dims, double
     const int tid = threadIdx.x;
     double ke = 0.0, fe = 0.0, l1 = 0.0;
     for (unsigned i = blockIdx.x * 256 + tid; i < S.n; i += gridDim.x * 256)
-        if (!S.alive || S.alive[i])
+        if (!alive || alive[i])
             ke += S.hmw * (S.v[0][i] * S.v[0][i] + S.v[1][i] * S.v[1][i] + S.v[2][i] * S.v[2][i]);
     if (last_species) {
         for (long long g = blockIdx.x * 256 + tid; g < N; g += gridDim.x * 256) {
@@ -2212,6 +2372,7 @@ struct SimND {
             // src/Mesh2D.cpp:57-62, src/Mesh3D.cpp:43-45
             const bool wall_a = walls && a < c.dims && (a < 2 ? c.wall_axis[a] != 0 : c.wall_axis_z != 0);
             p.d[a] = p.L[a] / (double)(wall_a ? p.n[a] - 1 : p.n[a]);
+            p.rd[a] = reciprocal_spacing(p.d[a]);
             p.B[a] = c.magnetic_field[a];
             N *= (size_t)p.n[a];
             if (a < c.dims) cellvol *= p.d[a];
@@ -2281,6 +2442,11 @@ struct SimND {
             for (int a = 0; a < 3; ++a) D.sb[a] = (float)(2.0 * hq * c.magnetic_field[a] / (1.0 + t2));
             for (int a = 0; a < 3; ++a) D.drift[a] = a < c.dims ? (float)(c.dt / p.d[a]) : 0.0f;
             D.dep_fixed = (float)(D.dep * p.rho_scale);
+            D.bh = hq;  // t and s of boris(), in its own order of operations
+            double bt2 = 0.0;
+            for (int a = 0; a < 3; ++a) { D.bt[a] = hq * c.magnetic_field[a]; bt2 += D.bt[a] * D.bt[a]; }
+            const double sf = 2.0 / (1.0 + bt2);
+            for (int a = 0; a < 3; ++a) D.bs[a] = sf * D.bt[a];
             D.index = s;
         }
         solver.allocs = &allocations;
@@ -2315,9 +2481,9 @@ struct SimND {
                 solver.F.acc_scale[s] = sp[s].dep / (double)kWeightScale;
             }
         }
-        cell_count = dalloc<unsigned>(N);
-        cell_offset = dalloc<unsigned>(N);
-        block_sums = dalloc<unsigned>((N + kScanBlock - 1) / kScanBlock + 1);
+        cell_count = dalloc<unsigned>(N + 1);
+        cell_offset = dalloc<unsigned>(N + 1);
+        block_sums = dalloc<unsigned>((N + kScanBlock) / kScanBlock + 1);
         sample_partial = dalloc<double>(3 * kSampleBlocks);
         sample_done = dalloc<unsigned>(1);
         sample_out = dalloc<double>(8);
@@ -2377,6 +2543,24 @@ struct SimND {
             APIC_CUDA(cudaGetLastError());
             return;
         }
+        if (MODE == kPushStep) {
+            const unsigned g = (S.n + kRunItems * kThreads - 1) / (kRunItems * kThreads);
+            const int kind = !boris ? kNoField : (p.prof_rows ? kProfileField : kUniformField);
+            auto run = [&](auto dim, auto wall) {
+                constexpr int D = decltype(dim)::value;
+                constexpr bool Wl = decltype(wall)::value;
+                if (kind == kNoField) k_push_run<D, kNoField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
+                else if (kind == kUniformField) k_push_run<D, kUniformField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
+                else k_push_run<D, kProfileField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
+            };
+            using D2 = std::integral_constant<int, 2>;
+            using D3 = std::integral_constant<int, 3>;
+            if (cfg.dims == 2) walls ? run(D2{}, std::true_type{}) : run(D2{}, std::false_type{});
+            else walls ? run(D3{}, std::true_type{}) : run(D3{}, std::false_type{});
+            APIC_CUDA(cudaGetLastError());
+            return;
+        }
+        if constexpr (MODE != kPushStep) {
         if (cfg.dims == 2 && walls) {
             if (boris) k_push<2, true, MODE, true><<<blocks, kThreads, 0, stream>>>(p, S, b);
             else k_push<2, false, MODE, true><<<blocks, kThreads, 0, stream>>>(p, S, b);
@@ -2391,28 +2575,35 @@ struct SimND {
             else k_push<3, false, MODE><<<blocks, kThreads, 0, stream>>>(p, S, b);
         }
         APIC_CUDA(cudaGetLastError());
+        }
     }
 
     void sort_species(int s) {
         SpeciesND& S = sp[s];
         if (S.n == 0) return;
         const unsigned blocks = (S.n + kThreads - 1) / kThreads;
-        const unsigned nb = (unsigned)((ncells + kScanBlock - 1) / kScanBlock);
-        APIC_CUDA(cudaMemsetAsync(cell_count, 0, ncells * sizeof(unsigned), stream));
+        const unsigned nbins = (unsigned)ncells + (walls ? 1u : 0u);  // with walls: one bin for the absorbed
+        const unsigned nb = (nbins + kScanBlock - 1) / kScanBlock;
+        APIC_CUDA(cudaMemsetAsync(cell_count, 0, nbins * sizeof(unsigned), stream));
         if (fp32) k_cell_hist32<<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
-        else if (cfg.dims == 2) k_cell_hist<2><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
-        else k_cell_hist<3><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
-        k_scan_local<<<nb, kThreads, 0, stream>>>(cell_count, cell_offset, block_sums, (unsigned)ncells);
+        else if (walls && cfg.dims == 2) k_cell_hist<2, true><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
+        else if (walls) k_cell_hist<3, true><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
+        else if (cfg.dims == 2) k_cell_hist<2, false><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
+        else k_cell_hist<3, false><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
+        k_scan_local<<<nb, kThreads, 0, stream>>>(cell_count, cell_offset, block_sums, nbins);
         k_scan_blocks<<<1, kThreads, 0, stream>>>(block_sums, nb);
-        k_scan_add<<<nb, kThreads, 0, stream>>>(cell_offset, block_sums, (unsigned)ncells);
+        k_scan_add<<<nb, kThreads, 0, stream>>>(cell_offset, block_sums, nbins);
         if (fp32) {
             k_cell_rank32<<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
             if (cfg.dims == 2) k_cell_gather32<2><<<blocks, kThreads, 0, stream>>>(S, buf[s]);
             else k_cell_gather32<3><<<blocks, kThreads, 0, stream>>>(S, buf[s]);
+        } else if (walls) {
+            if (cfg.dims == 2) k_cell_scatter<2, true><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
+            else k_cell_scatter<3, true><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
         } else if (cfg.dims == 2) {
-            k_cell_scatter<2><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
+            k_cell_scatter<2, false><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
         } else {
-            k_cell_scatter<3><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
+            k_cell_scatter<3, false><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
         }
         APIC_CUDA(cudaGetLastError());
         buf[s] ^= 1;
@@ -2442,7 +2633,7 @@ struct SimND {
         require(n <= cfg.species[s].capacity, "initial particle count exceeds max_particles_per_species",
                 APIC_ERR_CAPACITY);
         SpeciesND& S = sp[s];
-        if (S.alive && n) APIC_CUDA(cudaMemsetAsync(S.alive, 1, n, stream));
+        if (S.alive[buf[s]] && n) APIC_CUDA(cudaMemsetAsync(S.alive[buf[s]], 1, n, stream));
         const int b = buf[s];
         const size_t bytes = n * sizeof(double);
         for (int a = 0; a < cfg.dims; ++a)
@@ -2506,7 +2697,7 @@ struct SimND {
         bool absorbing = false;
         for (int k = 0; k < 2 * dims; ++k) absorbing = absorbing || p.pbc[k] == 1;
         for (int s = 0; s < c.nspecies; ++s)
-            sp[s].alive = absorbing ? dalloc<uint8_t>(c.species[s].capacity) : nullptr;
+            for (int b = 0; b < 2; ++b) sp[s].alive[b] = absorbing ? dalloc<uint8_t>(c.species[s].capacity) : nullptr;
         solver.F.dims = dims;
         solver.F.rho_acc = dalloc<unsigned long long>(N);
         solver.F.rho = dalloc<double>(N);
@@ -2720,7 +2911,7 @@ struct SimND {
         for (size_t it = 0; it < nsteps; ++it) {
             unsigned sort_mask = 0;
             for (int s = 0; s < cfg.nspecies; ++s)
-                if (!walls && since_sort[s] >= species_interval[s] && sp[s].n) sort_mask |= 1u << s;
+                if (since_sort[s] >= species_interval[s] && sp[s].n) sort_mask |= 1u << s;
             for (int s = 0; s < cfg.nspecies; ++s) {
                 if (since_sort[s] < species_interval[s]) continue;
                 since_sort[s] = 0;
@@ -2811,8 +3002,15 @@ struct SimND {
         const size_t n = sp[s].n;
         require(cap >= n, "output capacity below the particle count", APIC_ERR_CAPACITY);
         sync();
-        if (sp[s].alive) APIC_CUDA(cudaMemcpyAsync(alive, sp[s].alive, n, cudaMemcpyDeviceToHost, stream));
-        else std::memset(alive, 1, n);
+        if (sp[s].alive[0] && n) {  // in load order, through the other buffer (free outside a sort)
+            const int b = buf[s];
+            k_unpermute<<<(unsigned)((n + kThreads - 1) / kThreads), kThreads, 0, stream>>>(
+                sp[s].id[b], sp[s].alive[b], sp[s].alive[b ^ 1], (unsigned)n);
+            APIC_CUDA(cudaGetLastError());
+            APIC_CUDA(cudaMemcpyAsync(alive, sp[s].alive[b ^ 1], n, cudaMemcpyDeviceToHost, stream));
+        } else {
+            std::memset(alive, 1, n);
+        }
         APIC_CUDA(cudaStreamSynchronize(stream));
     }
 
@@ -2849,7 +3047,7 @@ struct SimND {
         if (cfg.dims == 2) vol *= (cfg.out_of_plane_depth == 0.0 ? 1.0 : cfg.out_of_plane_depth);
         for (int s = 0; s < cfg.nspecies; ++s) {
             if (initialized) launch_push<kPushSync>(s);
-            k_sample_nd<<<kSampleBlocks, 256, 0, stream>>>(sp[s], cfg.dims, sample_partial, sample_done, sample_out,
+            k_sample_nd<<<kSampleBlocks, 256, 0, stream>>>(sp[s], sp[s].alive[buf[s]], cfg.dims, sample_partial, sample_done, sample_out,
                                                            solver.F.E, solver.F.rho, (long long)ncells,
                                                            0.5 * p.eps * vol, vol, s, s == cfg.nspecies - 1,
                                                            p.wall[0], p.wall[1], p.wall[2], p.n[0], p.n[1], p.n[2]);

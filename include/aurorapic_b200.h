@@ -399,8 +399,8 @@ typedef struct {
        counts nodes (spacing length / (n - 1)); one wall axis solves by FFT along the periodic axis and
        a tridiagonal sweep per mode, two by a direct sine-transform solve (extents 2^k + 1).  Sides are
        left, right, bottom, top.  particle_boundary: 0 auto (periodic on a periodic axis, absorbing on
-       a wall axis), 1 absorbing, 2 reflecting, 3 periodic.  FP64 form; particles are not re-sorted;
-       absorbed particles stay in place, flagged dead (apic_simnd_read_alive). */
+       a wall axis), 1 absorbing, 2 reflecting, 3 periodic.  FP64 form; absorbed
+       particles are kept, flagged dead (apic_simnd_read_alive). */
     int wall_axis[2];
     double wall_potential[4];
     int particle_boundary[4];

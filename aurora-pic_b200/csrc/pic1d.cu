@@ -150,6 +150,7 @@ struct Params1D {
     int f32;  // FP32 velocities (both FP32 forms)
     int c32;  // FP32 cell form: int32 cell + float offset positions, FP32 arithmetic
     double L, dx, inv_dx, dt, eps, rho_scale, inv_rho_scale;
+    double rdx;  // 1 / dx (cells_of)
     unsigned mode;
     uint64_t seed;
     double phi_left, phi_right;
@@ -163,6 +164,7 @@ struct Params1D {
     double* phi;
     unsigned long long* rho_acc;
     const double* tw;       // periodic: twiddles (cos, sin)(2 pi m / n), m < n
+    int dft_n1;             // periodic: the largest divisor of nx up to its square root (dft_two_step)
     const double* thomas_r; // Dirichlet: 1/denominator of the Thomas forward sweep
     const double* thomas_a; // Dirichlet: -cp of the back substitution
     BirthRec* births;
@@ -191,8 +193,11 @@ struct Params1D {
 
 // wrap_periodic, src/FieldSolver.cpp:15-17: fmod(fmod(x, L) + L, L).  For
 // |x| < 2L every fmod is a single exact subtraction (Sterbenz), so the fast
-// branch returns the same bits as the two library fmod calls.
+// branch returns the same bits as the two library fmod calls; a position
+// already inside [0, L) stays as it is (the reference's (x + L) - L rounds its
+// last bits away).
 __device__ __forceinline__ double wrap_periodic(double x, double L) {
+    if (x >= 0.0 && x < L) return x;
     if (!(fabs(x) < 2.0 * L)) return fmod(fmod(x, L) + L, L);
     const double r = x >= L ? x - L : (x <= -L ? x + L : x);  // fmod(x, L)
     const double y = r + L;
@@ -206,37 +211,31 @@ struct Cic {
 
 // interpolate_electric / deposit_charge index + fraction, src/FieldSolver.cpp:909-924,
 // src/Species.cpp:167-183
-__device__ __forceinline__ Cic cic_periodic(double x, double L, double dx, int nx) {
-    const double xp = wrap_periodic(x, L);
-    const double g = xp / dx;
-    const double fl = floor(g);
-    const unsigned long long i = (unsigned long long)fl;
-    const double f = g - (double)i;
-    // i % nx and (i + 1) % nx; i <= nx after the wrap, so the remainders are
-    // single subtractions (the 64-bit division only for out-of-range input)
-    const unsigned long long n = (unsigned long long)nx;
-    const unsigned long long i1 = i + 1;
+__device__ __forceinline__ Cic cic_periodic(double x, const Params1D& p) {
+    const double xp = wrap_periodic(x, p.L);
+    const double g = cells_of(xp, p.dx, p.rdx);
+    const int i = (int)floor(g);
+    // i % nx and (i + 1) % nx; 0 <= i <= nx after the wrap (a NaN converts to 0)
     Cic c;
-    c.i0 = (int)(i < n ? i : (i < 2 * n ? i - n : i % n));
-    c.i1 = (int)(i1 < n ? i1 : (i1 < 2 * n ? i1 - n : i1 % n));
+    const double f = g - (double)i;
+    c.i0 = (unsigned)i < (unsigned)p.nx ? i : 0;
+    c.i1 = c.i0 + 1 == p.nx ? 0 : c.i0 + 1;
     c.w0 = 1.0 - f;
     c.w1 = f;
     return c;
 }
 
-__device__ __forceinline__ Cic cic_dirichlet(double x, double L, double dx, int nx) {
+__device__ __forceinline__ Cic cic_dirichlet(double x, const Params1D& p) {
     // std::clamp (a NaN position, already flagged as non-finite, lands on the
     // left wall so that every index stays inside the grid)
-    const double xp = !(x >= 0.0) ? 0.0 : (L < x ? L : x);
-    const double g = xp / dx;
-    double fl = floor(g);
-    const double lim = (double)(nx - 2);
-    if (lim < fl) fl = lim;  // std::min<double>(floor(g), nx - 2)
-    const unsigned long long i = (unsigned long long)fl;
+    const double xp = !(x >= 0.0) ? 0.0 : (p.L < x ? p.L : x);
+    const double g = cells_of(xp, p.dx, p.rdx);
+    int i = (int)floor(g);
+    if (i > p.nx - 2) i = p.nx - 2;  // std::min<double>(floor(g), nx - 2)
     const double f = g - (double)i;
     Cic c;
-    c.i0 = (int)i;
-    c.i1 = (int)i + 1;
+    c.i0 = i;
+    c.i1 = i + 1;
     c.w0 = 1.0 - f;
     c.w1 = f;
     return c;
@@ -244,7 +243,7 @@ __device__ __forceinline__ Cic cic_dirichlet(double x, double L, double dx, int 
 
 template <bool DIRICHLET>
 __device__ __forceinline__ Cic cic(double x, const Params1D& p) {
-    return DIRICHLET ? cic_dirichlet(x, p.L, p.dx, p.nx) : cic_periodic(x, p.L, p.dx, p.nx);
+    return DIRICHLET ? cic_dirichlet(x, p) : cic_periodic(x, p);
 }
 
 __device__ __forceinline__ double gather(const double* E, const Cic& c) {
@@ -385,8 +384,15 @@ template <int VDIM, bool DIRICHLET, bool F32, bool DIAG>
 __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sE = reinterpret_cast<double*>(smem_raw);
-    unsigned long long* sRho = reinterpret_cast<unsigned long long*>(sE + p.nx);
+    unsigned* sLo = reinterpret_cast<unsigned*>(sE + p.nx);  // the fixed-point density (shared_add64)
+    unsigned* sHi = sLo + p.nx;
     __shared__ unsigned s_cnt[32];
+    // the collision tallies of each warp, added to the run's totals once per
+    // CTA (tens of thousands of candidates a step added to the same few global
+    // counters: discharge of 512 cells x 512 particles, pass 69 -> 64 us)
+    constexpr int kWarps = kThreads / 32;
+    __shared__ unsigned s_cand[kWarps], s_null[kWarps], s_chan[kWarps][kMaxModels][kMaxChannels];
+    __shared__ double s_energy[kWarps][kMaxModels][kMaxChannels];
     __shared__ unsigned s_qlen;
     __shared__ CandidateEntry s_queue[kQueue];
 
@@ -394,8 +400,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
     const unsigned mode = p.mode;
     for (int i = tid; i < p.nx; i += kThreads) {
         sE[i] = p.E[i];
-        sRho[i] = 0ull;
+        sLo[i] = 0u;
+        sHi[i] = 0u;
     }
+    for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
+        (&s_chan[warp][0][0])[i] = 0u;
+        (&s_energy[warp][0][0])[i] = 0.0;
+    }
+    if (lane == 0) s_cand[warp] = s_null[warp] = 0u;
     if (tid == 0) s_qlen = 0;
     DevState* st = p.st;
     unsigned tiles_before[kMaxSpecies + 1];
@@ -511,11 +523,12 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
         if (mcc) {
             const unsigned qlen = min(s_qlen, (unsigned)kQueue);
             const MccModelDev& M = p.model[S.model];
-            for (unsigned q = tid; q < qlen; q += kThreads) {
-                CandidateEntry& ce = s_queue[q];
+            for (unsigned q0 = warp * 32; q0 < qlen; q0 += kThreads) {
+                CollideResult r;
+                if (q0 + lane < qlen) {
+                CandidateEntry& ce = s_queue[q0 + lane];
                 PhiloxStream rng(p.seed, ce.slot, mcc_step, (uint32_t)s);
                 rng.seek(ce.draws);
-                CollideResult r;
                 unsigned nion = 0;
                 const unsigned slot = ce.slot;
                 const double px = ce.x;
@@ -548,14 +561,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                          },
                          true, ce.first_wait);
                 if (r.error) atomicOr(&st->error, r.error);
-                atomicAdd(&st->candidates, (unsigned long long)r.candidates);
-                if (r.nulls) atomicAdd(&st->nulls, (unsigned long long)r.nulls);
-                for (int ch = 0; ch < M.nch; ++ch) {
-                    if (r.channel[ch]) {
-                        atomicAdd(&st->chan[S.model][ch], (unsigned long long)r.channel[ch]);
-                        atomicAdd(&st->chan_energy[S.model][ch], r.energy_change[ch] * S.weight);
-                    }
-                }
                 if (DIAG && p.coll_acc) {
                     // tracked_energy_change, src/Simulation.cpp:862-923: the weighted
                     // projectile change per channel, deposited at the particle (the
@@ -567,6 +572,17 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                     }
                 }
                 ce.v[0] = vel[0]; ce.v[1] = vel[1]; ce.v[2] = vel[2];
+                }
+                __syncwarp();
+                const unsigned nc = __reduce_add_sync(0xffffffffu, r.candidates);
+                const unsigned nn = __reduce_add_sync(0xffffffffu, r.nulls);
+                if (lane == 0) { s_cand[warp] += nc; s_null[warp] += nn; }
+                for (int ch = 0; ch < M.nch; ++ch) {
+                    const unsigned c = __reduce_add_sync(0xffffffffu, r.channel[ch]);
+                    if (!c) continue;
+                    const double e = warp_sum(r.energy_change[ch] * S.weight);
+                    if (lane == 0) { s_chan[warp][S.model][ch] += c; s_energy[warp][S.model][ch] += e; }
+                }
             }
             __syncthreads();
         }
@@ -616,8 +632,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                 const Cic d = cic<DIRICHLET>(x[k], p);
                 long long a0, a1;
                 deposit_contrib<DIRICHLET>(d, S, p, a0, a1);
-                atomicAdd(&sRho[d.i0], (unsigned long long)a0);
-                atomicAdd(&sRho[d.i1], (unsigned long long)a1);
+                shared_add64(sLo, sHi, d.i0, a0);
+                shared_add64(sLo, sHi, d.i1, a1);
             }
         }
         if (DIAG && p.ledger) {
@@ -670,8 +686,26 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
     }
     if (mode & kModeDeposit) {
         for (int i = tid; i < p.nx; i += kThreads) {
-            const unsigned long long a = sRho[i];
+            const unsigned long long a = join64(sLo[i], sHi[i]);
             if (a) atomicAdd(&p.rho_acc[i], a);
+        }
+    }
+    // (the tile loop ends on a barrier)
+    if ((mode & kModeSyncMcc) && tid < kMaxModels * kMaxChannels) {
+        unsigned long long c = 0ull;
+        double e = 0.0;
+        for (int w = 0; w < kWarps; ++w) {
+            c += (&s_chan[w][0][0])[tid];
+            e += (&s_energy[w][0][0])[tid];
+        }
+        if (c) {
+            atomicAdd(&st->chan[0][0] + tid, c);
+            atomicAdd(&st->chan_energy[0][0] + tid, e);
+        }
+        if (tid < 2) {
+            c = 0ull;
+            for (int w = 0; w < kWarps; ++w) c += tid ? s_null[w] : s_cand[w];
+            if (c) atomicAdd(tid ? &st->nulls : &st->candidates, c);
         }
     }
 }
@@ -734,12 +768,81 @@ __device__ __forceinline__ double electrode(double offset, const apic_voltage_dr
     return offset + d.amplitude * sin(2.0 * 3.141592653589793 * d.frequency * t + d.phase);
 }
 
+// One discrete Fourier transform of n points by one CTA in two steps of n1 and
+// n2 = n / n1 terms per point (the Cooley-Tukey split for any divisor n1),
+// n (n1 + n2) multiply-adds instead of n^2: with j = n2 j1 + j2 and
+// k = k1 + n1 k2,
+//   mid[k1][j2] = sum_j1 in(n2 j1 + j2) w^(n2 j1 k1),
+//   out(k) = sum_j2 mid[k1][j2] w^(j2 k),
+// w = exp(-+2 pi i / n) from exact twiddles (cos, sin)(2 pi m / n).  Only the
+// outputs k < kout are formed.  A prime n falls back to n1 = 1, the direct sum.
+// (Step of the 16,384-particle two-stream deck on 128 nodes: 29.1 -> 24.9 us.)
+// NA arrays are transformed together (in and out take all of them per point);
+// sign is that of the exponent.
+template <int NA, class In, class Out>
+__device__ __forceinline__ void dft_two_step(int n, int n1, int kout, double sign, const double2* tw, In in,
+                                             double2* mid, Out out) {
+    const int n2 = n / n1;
+    if (n1 > 1) {
+#pragma unroll 1
+        for (int t = threadIdx.x; t < n; t += kPostThreads) {
+            const int k1 = t / n2, j2 = t - k1 * n2;
+            double2 sum[NA] = {};
+            int m = 0;
+            const int dm = n2 * k1;  // < n
+#pragma unroll 2
+            for (int j1 = 0, j = j2; j1 < n1; ++j1, j += n2) {
+                double2 a[NA];
+                in(j, a);
+                const double2 w = tw[m];
+                const double ws = sign * w.y;
+#pragma unroll
+                for (int q = 0; q < NA; ++q) {
+                    sum[q].x = fma(a[q].x, w.x, fma(-a[q].y, ws, sum[q].x));
+                    sum[q].y = fma(a[q].x, ws, fma(a[q].y, w.x, sum[q].y));
+                }
+                m += dm;
+                if (m >= n) m -= n;
+            }
+#pragma unroll
+            for (int q = 0; q < NA; ++q) mid[q * n + t] = sum[q];
+        }
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int k = threadIdx.x; k < kout; k += kPostThreads) {
+        const int k1 = k % n1;
+        double2 sum[NA] = {};
+        int m = 0;
+#pragma unroll 2
+        for (int j2 = 0; j2 < n2; ++j2) {
+            double2 a[NA];
+            if (n1 > 1) {
+#pragma unroll
+                for (int q = 0; q < NA; ++q) a[q] = mid[q * n + k1 * n2 + j2];
+            } else {
+                in(j2, a);
+            }
+            const double2 w = tw[m];
+            const double ws = sign * w.y;
+#pragma unroll
+            for (int q = 0; q < NA; ++q) {
+                sum[q].x = fma(a[q].x, w.x, fma(-a[q].y, ws, sum[q].x));
+                sum[q].y = fma(a[q].x, ws, fma(a[q].y, w.x, sum[q].y));
+            }
+            m += k;
+            if (m >= n) m -= n;
+        }
+        out(k, sum);
+    }
+}
+
 // Shared-memory layout of the post kernel (dynamic): the fixed-point density,
 // the solver's constant coefficients and, for the periodic solve, the per-mode
 // spectra.  Everything the solve needs is loaded in one round trip at entry.
 __host__ __device__ inline size_t post_smem_bytes(int nx, bool dirichlet) {
     return (size_t)nx * 8 /* rho_i */ + (size_t)nx * 8 /* rho */ +
-           (dirichlet ? (size_t)2 * nx * 8 : (size_t)2 * nx * 8 /* twiddles */ + (size_t)4 * nx * 8 /* spectra */);
+           (dirichlet ? (size_t)2 * nx * 8 : (size_t)2 * nx * 8 /* twiddles */ + ((size_t)5 * nx + 2) * 8 /* spectra */);
 }
 
 template <int VDIM, bool DIRICHLET, bool F32, bool C32 = false>
@@ -760,7 +863,7 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
     double* s_rho = reinterpret_cast<double*>(s_rhoi + nx);
     double* s_c0 = s_rho + nx;                       // Dirichlet: 1/denominators; periodic: twiddles (2 nx)
     double* s_c1 = s_c0 + nx;                        // Dirichlet: -cp
-    double* s_spec = s_c0 + 2 * nx;                  // periodic: 4 nx spectra
+    double* s_spec = s_c0 + 2 * nx;                  // periodic: the spectrum and a transform's middle
     DevState* st = p.st;
     const int tid = threadIdx.x;
     const bool solve = (post & kPostSolve) != 0;
@@ -1017,49 +1120,35 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         __syncthreads();
         const double mean = s_mean;
         const double twopi = 2.0 * 3.141592653589793;
-        double* sp_r = s_spec;
-        double* sp_i = s_spec + nx;
-        double* se_r = s_spec + 2 * nx;
-        double* se_i = s_spec + 3 * nx;
-        // forward transform: mode k per thread, summed over j in the reference's order,
-        // then the per-mode potential and field, src/FieldSolver.cpp:418-428
-        for (int k = tid; k < nx; k += kPostThreads) {
-            if (k == 0) { sp_r[0] = sp_i[0] = se_r[0] = se_i[0] = 0.0; continue; }
-            double re = 0.0, im = 0.0;
-            unsigned m = 0;
-            for (int j = 0; j < nx; ++j) {
-                const double a = s_rho[j] - mean;
-                re += a * s_c0[2 * m];
-                im += a * (-s_c0[2 * m + 1]);
-                m += (unsigned)k;
-                if (m >= (unsigned)nx) m -= (unsigned)nx;
-            }
-            re /= (double)nx;
-            im /= (double)nx;
-            const double kk = (k <= nx / 2) ? (double)k : -(double)(nx - k);
-            const double wave = twopi * kk / p.L;
-            const double den = p.eps * wave * wave;
-            const double pr = re / den, pi = im / den;
-            sp_r[k] = pr;
-            sp_i[k] = pi;
-            se_r[k] = wave * pi;    // -(0,1) * wave * phik
-            se_i[k] = -(wave * pr);
-        }
+        const int half = nx / 2;
+        double2* const spec = reinterpret_cast<double2*>(s_spec);  // phi_k, k <= nx / 2
+        double2* const mid = spec + half + 1;                      // 2 nx values
+        const double2* const tw = reinterpret_cast<const double2*>(s_c0);
+        // forward: the modes 0 .. nx / 2 of the real density, then
+        // phi_k = rho_k / (eps k^2), src/FieldSolver.cpp:418-428
+        dft_two_step<1>(
+            nx, p.dft_n1, half + 1, -1.0, tw, [&](int j, double2* v) { v[0] = {s_rho[j] - mean, 0.0}; }, mid,
+            [&](int k, const double2* v) {
+                const double wave = twopi * (double)k / p.L;
+                const double den = p.eps * wave * wave * (double)nx;
+                spec[k] = k ? double2{v[0].x / den, v[0].y / den} : double2{0.0, 0.0};
+            });
         __syncthreads();
-        // inverse: each node j sums its modes in order k = 1 .. n-1
-        for (int j = tid; j < nx; j += kPostThreads) {
-            double ph = 0.0, ef = 0.0;
-            unsigned m = (unsigned)j;
-            for (int k = 1; k < nx; ++k) {
-                const double cs = s_c0[2 * m], sn = s_c0[2 * m + 1];
-                ph += sp_r[k] * cs - sp_i[k] * sn;
-                ef += se_r[k] * cs - se_i[k] * sn;
-                m += (unsigned)j;
-                if (m >= (unsigned)nx) m -= (unsigned)nx;
-            }
-            p.phi[j] = ph;
-            p.E[j] = ef;
-        }
+        // inverse: phi and E_k = -i k phi_k together; the modes above nx / 2
+        // are the conjugates of those below (both fields are real)
+        dft_two_step<2>(
+            nx, p.dft_n1, nx, 1.0, tw,
+            [&](int k, double2* v) {
+                const bool upper = k > half;
+                const double2 a = spec[upper ? nx - k : k];
+                const double wave = twopi * (double)(upper ? k - nx : k) / p.L;
+                v[0] = {a.x, upper ? -a.y : a.y};
+                v[1] = {wave * v[0].y, -(wave * v[0].x)};
+            },
+            mid, [&](int j, const double2* v) {
+                p.phi[j] = v[0].x;
+                p.E[j] = v[1].x;
+            });
     } else {
         __syncthreads();
         // solve_dirichlet_tridiagonal, src/FieldSolver.cpp:733-759, with the
@@ -1707,6 +1796,7 @@ struct Sim1D {
         p.L = c.length;
         p.dx = c.length / (double)(dir ? c.nx - 1 : c.nx);  // Grid::Grid, src/Grid.cpp:19-22
         p.inv_dx = 1.0 / p.dx;
+        p.rdx = reciprocal_spacing(p.dx);
         p.dt = c.dt;
         p.eps = (c.units == APIC_SI ? 8.8541878128e-12 : 1.0) * rel;  // include/pic/Types.hpp:17-27
         p.seed = c.seed;
@@ -1872,6 +1962,9 @@ struct Sim1D {
             double* d = dalloc<double>(tw.size());
             APIC_CUDA(cudaMemcpyAsync(d, tw.data(), tw.size() * sizeof(double), cudaMemcpyHostToDevice, stream));
             p.tw = d;
+            p.dft_n1 = 1;
+            for (int k = 2; k * k <= p.nx; ++k)
+                if (p.nx % k == 0) p.dft_n1 = k;
             APIC_CUDA(cudaStreamSynchronize(stream));
         } else {
             // Thomas coefficients of the constant [-1 2 -1] matrix, src/FieldSolver.cpp:745-752

@@ -122,8 +122,9 @@ __global__ void k_cell_to_x(const int* __restrict__ cell, const float* __restric
 template <int VDIM, bool DIRICHLET>
 __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D p) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned long long* sRho = reinterpret_cast<unsigned long long*>(smem_raw);
-    float* sE = reinterpret_cast<float*>(sRho + p.nx);
+    unsigned* sLo = reinterpret_cast<unsigned*>(smem_raw);  // the fixed-point density (shared_add64)
+    unsigned* sHi = sLo + p.nx;
+    float* sE = reinterpret_cast<float*>(sHi + p.nx);
     constexpr int kWarps = kThreads / 32;
     __shared__ unsigned s_mask[kWarps][kChunk32 / 32];
     // the CTA's wall-loss tallies, added to the run's totals once at the end
@@ -138,7 +139,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D 
     const int nx = p.nx;
     for (int i = tid; i < nx; i += kThreads) {
         sE[i] = (float)p.E[i];
-        sRho[i] = 0ull;
+        sLo[i] = 0u;
+        sHi[i] = 0u;
     }
     if (tid == 0) s_ncand = 0u;
     CandRec32* region = p.cands ? p.cands + (size_t)blockIdx.x * p.cand_per_region : nullptr;
@@ -320,8 +322,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D 
                     if (i0 == 0) q0 *= 2.0f;
                     if (i1 == nx - 1) q1 *= 2.0f;
                 }
-                atomicAdd(&sRho[i0], (unsigned long long)(long long)__float2int_rn(q0));
-                atomicAdd(&sRho[i1], (unsigned long long)(long long)__float2int_rn(q1));
+                shared_add64(sLo, sHi, i0, __float2int_rn(q0));
+                shared_add64(sLo, sHi, i1, __float2int_rn(q1));
             }
             __stcs(S.vh32[0] + idx, vh[k]);
             if (mode & (kModeWriteV | kModeInitHalf)) S.v[idx] = (double)vc[k];
@@ -330,7 +332,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D 
     __syncthreads();
     if (mode & kModeDeposit) {
         for (int i = tid; i < nx; i += kThreads) {
-            const unsigned long long a = sRho[i];
+            const unsigned long long a = join64(sLo[i], sHi[i]);
             if (a) atomicAdd(&p.rho_acc[i], a);
         }
     }
@@ -354,8 +356,12 @@ constexpr int kCollideThreads = 128;
 constexpr int kMaxRegions = 2048;  // regions (CTAs of the pass) the dense numbering covers
 template <int VDIM, bool DIRICHLET>
 __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
-    __shared__ unsigned long long s_cand, s_null, s_chan[kMaxModels][kMaxChannels], s_lost[kMaxSpecies][2];
-    __shared__ double s_energy[kMaxModels][kMaxChannels], s_lost_energy[kMaxSpecies][2];
+    constexpr int kWarps = kCollideThreads / 32;
+    __shared__ unsigned s_cand, s_null, s_chan[kMaxModels][kMaxChannels];
+    __shared__ unsigned long long s_lost[kMaxSpecies][2];
+    // each warp's collision energies, summed by shuffles: double adds to one
+    // shared word are a compare-and-swap loop that a warp runs lane by lane
+    __shared__ double s_energy[kWarps][kMaxModels][kMaxChannels], s_lost_energy[kMaxSpecies][2];
     __shared__ unsigned s_dead[kMaxSpecies];
     __shared__ unsigned s_start[kMaxRegions + 1];  // first dense index of each region
     const int tid = threadIdx.x;
@@ -377,16 +383,15 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         for (int k = 0; k < PER; ++k) s_start[tid * PER + k] = o[k];
         if (tid == 0) s_start[kMaxRegions] = total;
     }
-    if (tid < kMaxModels * kMaxChannels) {
-        (&s_chan[0][0])[tid] = 0ull;
-        (&s_energy[0][0])[tid] = 0.0;
-    }
+    const int lane = tid & 31, warp = tid >> 5;
+    if (tid < kMaxModels * kMaxChannels) (&s_chan[0][0])[tid] = 0u;
+    for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) (&s_energy[warp][0][0])[i] = 0.0;
     if (tid < kMaxSpecies * 2) {
         (&s_lost[0][0])[tid] = 0ull;
         (&s_lost_energy[0][0])[tid] = 0.0;
     }
     if (tid < kMaxSpecies) s_dead[tid] = 0u;
-    if (tid == 0) s_cand = s_null = 0ull;
+    if (tid == 0) s_cand = s_null = 0u;
     __syncthreads();
     DevState* st = p.st;
     const unsigned mode = p.mode;
@@ -396,7 +401,11 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
     const float dt_in = dt * (1.0f - kFltEpsilon);  // largest first wait kept inside the step
     const int nx = p.nx;
     const int ncell = DIRICHLET ? nx - 1 : nx;
-    for (unsigned d = blockIdx.x * kCollideThreads + tid; d < ntotal; d += gridDim.x * kCollideThreads) {
+    for (unsigned d0 = blockIdx.x * kCollideThreads + warp * 32; d0 < ntotal; d0 += gridDim.x * kCollideThreads) {
+        int model = -1;                  // of this lane's candidate
+        double energy[kMaxChannels] = {};  // its energy change per channel
+        const unsigned d = d0 + lane;
+        auto candidate = [&]() {
         // region holding dense index d: the last region whose start is <= d
         unsigned lo = 0, hi = regions;
         while (hi - lo > 1) {
@@ -408,6 +417,12 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         const SpeciesDev& S = p.sp[s];
         const MccModel32& M = p.model32[S.model];
         const MccModelDev& G = p.gmodel[S.model];
+        model = S.model;
+        auto tally = [&](int ch, double de) {  // (a select over the slots keeps the sums in registers)
+#pragma unroll
+            for (int i = 0; i < kMaxChannels; ++i)
+                if (i == ch) energy[i] += de;
+        };
         const unsigned slot = rec.slot;
         Philox32 rng(p.seed, slot, mcc_step, (uint32_t)s);
         // first waiting time: the exponential truncated to the step
@@ -419,8 +434,8 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         collide3f(
             M, v, dt, wait, rng, r, [&](float speed) { return frequency_bound_ok_far(G, (double)speed); },
             [&](int ch, double de) {
-                atomicAdd(&s_chan[S.model][ch], 1ull);
-                atomicAdd(&s_energy[S.model][ch], de * S.weight);
+                atomicAdd(&s_chan[S.model][ch], 1u);
+                tally(ch, de * S.weight);
             },
             [&](int ch, const float* vs, const float* vi) {
                 const unsigned bslot = atomicAdd(&st->nbirths, 2u);
@@ -440,12 +455,12 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
                 }
                 const SpeciesDev& A = p.sp[C.secondary];
                 const SpeciesDev& B = p.sp[C.ion];
-                atomicAdd(&s_energy[S.model][ch], energy64(A.mass * A.weight, vs) + energy64(B.mass * B.weight, vi));
+                tally(ch, energy64(A.mass * A.weight, vs) + energy64(B.mass * B.weight, vi));
                 ++nion;
             });
         if (r.error) atomicOr(&st->error, r.error);
-        atomicAdd(&s_cand, (unsigned long long)r.candidates);
-        if (r.nulls) atomicAdd(&s_null, (unsigned long long)r.nulls);
+        atomicAdd(&s_cand, r.candidates);
+        if (r.nulls) atomicAdd(&s_null, r.nulls);
         // the rest of the step, as in the pass
         const float E = rec.E;
         float vh = v[0] - S.hqmdt32 * E;  // src/Simulation.cpp:924-926
@@ -482,7 +497,7 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         if (!keep) {
             atomicAdd(&s_dead[s], 1u);
             S.cell[0][slot] = kDeadCell;
-            continue;
+            return;
         }
         if (mode & kModeDeposit) {
             int i0, i1;
@@ -502,12 +517,26 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         S.vy32[0][slot] = v[1];
         S.vz32[0][slot] = v[2];
         if (mode & kModeWriteV) S.v[slot] = (double)v[0];
+        };
+        if (d < ntotal) candidate();
+        __syncwarp();
+        for (int m = 0; m < kMaxModels; ++m) {
+            if (!__any_sync(0xffffffffu, model == m)) continue;
+#pragma unroll
+            for (int ch = 0; ch < kMaxChannels; ++ch) {
+                const double e = model == m ? energy[ch] : 0.0;
+                if (!__any_sync(0xffffffffu, e != 0.0)) continue;
+                const double w = warp_sum(e);
+                if (lane == 0) s_energy[warp][m][ch] += w;
+            }
+        }
     }
     __syncthreads();
     if (tid < kMaxModels * kMaxChannels) {
-        const unsigned long long c = (&s_chan[0][0])[tid];
-        if (c) atomicAdd(&st->chan[0][0] + tid, c);
-        const double e = (&s_energy[0][0])[tid];
+        const unsigned c = (&s_chan[0][0])[tid];
+        if (c) atomicAdd(&st->chan[0][0] + tid, (unsigned long long)c);
+        double e = 0.0;
+        for (int w = 0; w < kWarps; ++w) e += (&s_energy[w][0][0])[tid];
         if (e != 0.0) atomicAdd(&st->chan_energy[0][0] + tid, e);
     }
     if (tid < kMaxSpecies * 2) {
@@ -518,8 +547,8 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
     }
     if (tid < kMaxSpecies && s_dead[tid]) atomicAdd(&st->holes[tid], s_dead[tid]);
     if (tid == 0) {
-        if (s_cand) atomicAdd(&st->candidates, s_cand);
-        if (s_null) atomicAdd(&st->nulls, s_null);
+        if (s_cand) atomicAdd(&st->candidates, (unsigned long long)s_cand);
+        if (s_null) atomicAdd(&st->nulls, (unsigned long long)s_null);
     }
 }
 

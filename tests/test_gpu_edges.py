@@ -1,0 +1,101 @@
+"""Ragged sizes of the device kernels against the CPU oracle (1e-12 relative,
+max-norm): particle counts around the edges of a thread's run, a warp and a
+CTA, wall runs whose absorbed particles move to the end of the sorted order, and
+periodic 1D grids with every kind of divisor."""
+import numpy as np
+import pytest
+
+import apic
+import pyoracle as po
+from common import rel_max
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-12
+SPECIES = [(-1.0, 1.0, 0.05), (1.0, 50.0, 0.05)]
+
+
+def _particles(n, dims, length, seed):
+    rng = np.random.default_rng(seed)
+    pos = np.zeros((3, n))
+    for a in range(dims):
+        pos[a] = rng.uniform(0.0, length[a], n)
+    return pos, rng.standard_normal((3, n))
+
+
+@pytest.mark.parametrize("dims,B", [(2, (0.0, 0.0, 0.0)), (2, (0.1, 0.2, 0.3)), (3, (0.1, 0.2, 0.3))])
+@pytest.mark.parametrize("count", [1, 2, 3, 31, 33, 65, 511, 513, 1025])
+def test_push_of_ragged_counts(dims, B, count):
+    n, length = ((8, 4), (4.0, 2.0)) if dims == 2 else ((8, 4, 4), (4.0, 2.0, 3.0))
+    dev = apic.SimulationND(apic.config_nd(dims=dims, n=n, length=length, dt=0.1, magnetic_field=B, sort_interval=2,
+                                           species=[(q, m, w, count) for q, m, w in SPECIES]))
+    ora = po.SimND(dims, n, length, 0.1, 1.0, B, SPECIES)
+    for k in range(2):
+        pos, v = _particles(count, dims, length, 10 * count + k)
+        dev.load(k, pos, v)
+        ora.load(k, pos, v, v)
+    dev.initialize()
+    ora.initialize()
+    dev.step(5)
+    ora.step(5)
+    for k in range(2):
+        for x, y in zip(dev.particles(k), ora.particles(k)):
+            assert rel_max(x[:dims], y[:dims]) < TOL
+    for x, y in zip(dev.fields(), ora.fields()):
+        assert rel_max(x, y) < TOL
+
+
+@pytest.mark.parametrize("count", [1, 2, 65, 513, 1025])
+@pytest.mark.parametrize("sort", [1, 3, 1000])
+def test_walls_of_ragged_counts(count, sort):
+    """Positions, the dead flags and the loss counts in load order, however
+    often the particles are sorted."""
+    n, length, B = (8, 9), (4.0, 2.0), (0.0, 0.0, 0.2)
+    wall, pot, pb = (0, 1), (0.0, 0.0, 0.0, 1.5), (0, 0, 1, 2)
+    dev = apic.SimulationND(apic.config_nd(dims=2, n=n, length=length, dt=0.1, magnetic_field=B, sort_interval=sort,
+                                           species=[(q, m, w, count) for q, m, w in SPECIES],
+                                           walls=(wall, pot, [3 if b == 0 else b for b in pb])))
+    ora = po.SimND(2, n, length, 0.1, 1.0, B, SPECIES)
+    ora.set_walls(wall, pot, pb)
+    for k in range(2):
+        pos, v = _particles(count, 2, length, 10 * count + k)
+        dev.load(k, pos, v)
+        ora.load(k, pos, v, v)
+    dev.initialize()
+    ora.initialize()
+    dev.step(6)
+    ora.step(6)
+    for k in range(2):
+        alive, losses = ora.alive_losses(k)
+        assert np.array_equal(dev.alive(k), alive)
+        assert np.array_equal(dev.boundary_losses(k), np.asarray(losses)[:4])
+        keep = np.asarray(alive) == 1
+        if keep.any():
+            for x, y in zip(dev.particles(k)[::2], ora.particles(k)[::2]):  # positions, v_half
+                assert rel_max(x[:2][:, keep], y[:2][:, keep]) < TOL
+    for x, y in zip(dev.fields(), ora.fields()):
+        assert rel_max(x, y) < TOL
+
+
+@pytest.mark.parametrize("nx", [3, 4, 5, 12, 37, 64, 97, 100, 127, 255, 256, 1022, 1024, 1999, 2048])
+def test_periodic_1d_solve(nx):
+    """Two-step transforms (even and odd extents, squares, primes)."""
+    rng = np.random.default_rng(nx)
+    xs = [rng.uniform(0.0, 2.0, 3000), rng.uniform(0.0, 2.0, 3000)]
+    args = (nx, 2.0, 1.3, 0.0, 0.0, [-1.0, 1.5], [0.1, 0.1], xs)
+    rho, phi, E = apic.deposit_solve_gather_1d(apic.PERIODIC, *args)[:3]
+    dx = 2.0 / nx
+    want = np.zeros(nx)
+    for q, x in zip((-0.1, 0.15), xs):
+        g = x / dx
+        i = np.floor(g).astype(int)
+        f = g - i
+        want += np.bincount(i % nx, q / dx * (1 - f), nx) + np.bincount((i + 1) % nx, q / dx * f, nx)
+    assert rel_max(rho, want) < TOL
+    hat = np.fft.fft(rho - rho.mean())
+    k = 2 * np.pi * np.fft.fftfreq(nx, dx)
+    k[0] = 1.0
+    ph = hat / (1.3 * k * k)
+    ek = -1j * k * ph
+    ph[0] = ek[0] = 0.0
+    assert rel_max(phi, np.fft.ifft(ph).real) < TOL
+    assert rel_max(E, np.fft.ifft(ek).real) < TOL

@@ -76,11 +76,16 @@ __device__ inline int upper_bound_indexed(const MccChannelDev& c, double energy)
     const TableIndex& ix = c.index;
     int lo = 0, hi = c.rows;
     if (ix.nbins > 0) {
-        const double t = (log2(energy) - ix.lmin) * ix.inv_width;
+        // the single-precision log is good to 1e-5 bins' widths inside float's
+        // range; one more bin of slack on each side covers it, and the search
+        // below ends at the same row
+        const bool in_float = energy > 1e-36 && energy < 1e36;
+        const double l2 = in_float ? (double)__log2f((float)energy) : log2(energy);
+        const double t = (l2 - ix.lmin) * ix.inv_width;
         // (a NaN energy takes the whole table: the search stays inside it)
         const int b = !(t >= -1.0) ? -1 : (t > (double)ix.nbins ? ix.nbins : (int)floor(t));
-        lo = b >= 1 ? (int)__ldg(ix.first_gt + (b - 1)) : 0;
-        hi = b + 2 <= ix.nbins ? (int)__ldg(ix.first_gt + (b + 2)) : c.rows;
+        lo = b >= 2 ? (int)__ldg(ix.first_gt + (b - 2)) : 0;
+        hi = b + 3 <= ix.nbins ? (int)__ldg(ix.first_gt + (b + 3)) : c.rows;
     }
     const double* e = c.energy;
     while (lo < hi) {
@@ -125,11 +130,22 @@ __device__ inline bool rates_for_speed(const MccModelDev& m, double speed, doubl
         const int n = c0.rows;
         const bool below = energy <= __ldg(c0.energy), above = energy >= __ldg(c0.energy + n - 1);
         const int high = (below || above) ? 0 : upper_bound_indexed(c0, energy);
+        double fraction = 0.0;  // of the shared bracket (table_at)
+        if (!below && !above) {
+            const double el = __ldg(c0.energy + high - 1), eh = __ldg(c0.energy + high);
+            fraction = (energy - el) / (eh - el);
+        }
         for (int i = 0; i < m.nch; ++i) {
             const MccChannelDev& c = m.ch[i];
             double rate = 0.0;
             if (energy >= c.threshold) {
-                const double sg = below ? __ldg(c.sigma) : above ? __ldg(c.sigma + n - 1) : table_at(c, energy, high);
+                double sg;
+                if (below || above) {
+                    sg = __ldg(c.sigma + (below ? 0 : n - 1));
+                } else {
+                    const double sl = __ldg(c.sigma + high - 1), sh = __ldg(c.sigma + high);
+                    sg = sl + fraction * (sh - sl);
+                }
                 rate = m.neutral_density * sg * speed;
             }
             rates[i] = rate;
@@ -292,10 +308,10 @@ struct CollideResult {
 // receives (channel, secondary velocity[3], ion velocity[3]) per ionization.
 // When have_first is set, the caller already ran the first loop iteration's
 // bound check and waiting-time draw (the stream continues after them) and
-// passes that waiting time.
-template <class S, class OnSecondary>
+// passes that waiting time.  bound_ok(speed) runs validate_frequency_bound.
+template <class S, class OnSecondary, class BoundOk>
 __device__ inline void collide3(const MccModelDev& m, double v[3], double dt, S& s, CollideResult& r,
-                                OnSecondary&& on_secondary, bool have_first = false, double first_wait = 0.0) {
+                                OnSecondary&& on_secondary, bool have_first, double first_wait, BoundOk&& bound_ok) {
     if (!isfinite(v[0]) || !isfinite(v[1]) || !isfinite(v[2])) { r.error |= kErrNonFinite; return; }
     double elapsed = 0.0;
     for (;;) {
@@ -304,7 +320,7 @@ __device__ inline void collide3(const MccModelDev& m, double v[3], double dt, S&
             waiting = first_wait;
             have_first = false;
         } else {
-            if (!frequency_bound_ok(m, norm3(v[0], v[1], v[2]))) { r.error |= kErrMajorant; return; }
+            if (!bound_ok(norm3(v[0], v[1], v[2]))) { r.error |= kErrMajorant; return; }
             // open_unit_interval, src/Collision.cpp:46-51 (bounded for replay arrays)
             double u = uniform01(s);
             for (int guard = 0; !(u > 0.0) && guard < 64 && !s.overrun(); ++guard) u = uniform01(s);
@@ -392,15 +408,22 @@ __device__ inline void collide3(const MccModelDev& m, double v[3], double dt, S&
     if (s.overrun()) r.error |= kErrReplay;
 }
 
+template <class S, class OnSecondary>
+__device__ inline void collide3(const MccModelDev& m, double v[3], double dt, S& s, CollideResult& r,
+                                OnSecondary&& on_secondary, bool have_first = false, double first_wait = 0.0) {
+    collide3(m, v, dt, s, r, on_secondary, have_first, first_wait,
+             [&](double speed) { return frequency_bound_ok(m, speed); });
+}
+
 // NullCollisionModel::collide(double&) (1V), src/Collision.cpp:831-905, with
 // the scalar sample_neutral_velocity (:687-700) and the 1V apply_channel
 // (:717-760): the scattered speed takes a random sign, the top bit of one
 // draw (uniform_int_distribution<int>(0, 1) on a 64-bit engine).  The model
 // has no ionization and only isotropic channels (checked at create).  Same
 // first-iteration convention as collide3.
-template <class S>
+template <class S, class BoundOk>
 __device__ inline void collide1(const MccModelDev& m, double& v, double dt, S& s, CollideResult& r,
-                                bool have_first = false, double first_wait = 0.0) {
+                                bool have_first, double first_wait, BoundOk&& bound_ok) {
     if (!isfinite(v)) { r.error |= kErrNonFinite; return; }
     double elapsed = 0.0;
     for (;;) {
@@ -409,7 +432,7 @@ __device__ inline void collide1(const MccModelDev& m, double& v, double dt, S& s
             waiting = first_wait;
             have_first = false;
         } else {
-            if (!frequency_bound_ok(m, fabs(v))) { r.error |= kErrMajorant; return; }
+            if (!bound_ok(fabs(v))) { r.error |= kErrMajorant; return; }
             double u = uniform01(s);
             for (int guard = 0; !(u > 0.0) && guard < 64 && !s.overrun(); ++guard) u = uniform01(s);
             if (s.overrun()) { r.error |= kErrReplay; return; }

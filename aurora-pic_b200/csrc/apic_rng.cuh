@@ -32,26 +32,47 @@ __host__ __device__ inline void philox4x32_10(uint32_t c0, uint32_t c1, uint32_t
     out[0] = c0; out[1] = c1; out[2] = c2; out[3] = c3;
 }
 
+// One Philox block as a call: a collision loop draws at a dozen places, and
+// ten unrolled rounds at each of them make its code several times larger than
+// the instruction caches that its few resident warps keep refilling.
+static __device__ __noinline__ uint4 philox_call(uint32_t block, uint32_t slot, uint32_t step, uint32_t stream,
+                                                 uint32_t k0, uint32_t k1) {
+    uint32_t o[4];
+    philox4x32_10(block, slot, step, stream, k0, k1, o);
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
 // Raw 64-bit draws k = 0, 1, 2, ... of one particle's stream: draw k is half
-// of Philox block k/2 (low pair for even k, high pair for odd k).
-struct PhiloxStream {
+// of Philox block k/2 (low pair for even k, high pair for odd k).  CALLED takes
+// the blocks from philox_call.
+template <bool CALLED>
+struct PhiloxDraws {
     uint32_t k0, k1, slot, step, stream;
     uint32_t index = 0;
     uint32_t buf[4];
-    __device__ PhiloxStream(uint64_t seed, uint32_t slot_, uint32_t step_, uint32_t stream_)
+    __device__ PhiloxDraws(uint64_t seed, uint32_t slot_, uint32_t step_, uint32_t stream_)
         : k0((uint32_t)seed), k1((uint32_t)(seed >> 32)), slot(slot_), step(step_), stream(stream_) {}
+    __device__ void fill(uint32_t block) {
+        if (CALLED) {
+            const uint4 b = philox_call(block, slot, step, stream, k0, k1);
+            buf[0] = b.x; buf[1] = b.y; buf[2] = b.z; buf[3] = b.w;
+        } else {
+            philox4x32_10(block, slot, step, stream, k0, k1, buf);
+        }
+    }
     __device__ uint64_t next() {
         const uint32_t k = index++;
-        if ((k & 1u) == 0u) philox4x32_10(k >> 1, slot, step, stream, k0, k1, buf);
+        if ((k & 1u) == 0u) fill(k >> 1);
         return (k & 1u) ? ((uint64_t)buf[3] << 32 | buf[2]) : ((uint64_t)buf[1] << 32 | buf[0]);
     }
     __device__ bool overrun() const { return false; }
     // continue a stream that already produced k draws
     __device__ void seek(uint32_t k) {
         index = k;
-        if (k & 1u) philox4x32_10(k >> 1, slot, step, stream, k0, k1, buf);
+        if (k & 1u) fill(k >> 1);
     }
 };
+using PhiloxStream = PhiloxDraws<false>;
 
 struct ReplayStream {
     const uint64_t* draws;

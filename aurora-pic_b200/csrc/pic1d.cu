@@ -51,7 +51,10 @@ namespace apic {
 constexpr int kThreads = 256;
 constexpr int kItems = 4;
 constexpr int kTile = kThreads * kItems;
-constexpr int kMinBlocks = 2;  // resident CTAs of k_pass1d per SM (register budget)
+// resident CTAs of k_pass1d per SM (register budget): with collisions, and without
+constexpr int kMinBlocks = 2;
+template <int VDIM>
+constexpr int kPlainBlocks = VDIM == 1 ? 4 : 3;
 constexpr int kWarpCounts = kItems * (kThreads / 32);  // per-(item, warp) survivor counts of a tile
 static_assert(kWarpCounts <= 32, "the survivor scan runs in one warp");
 constexpr int kMaxSpecies = APIC_MAX_SPECIES;
@@ -282,13 +285,57 @@ __device__ __forceinline__ unsigned range_of(const unsigned* lstart, unsigned nr
 }
 
 // Physical slot of logical particle `idx`, walking forward from range r0
-// (a range at or before the one holding idx): a tile spans few ranges.
+// (a range at or before the one holding idx).
 __device__ __forceinline__ unsigned physical_slot_from(const unsigned* lstart, const unsigned* start, unsigned nr,
                                                        unsigned r0, unsigned idx) {
     unsigned r = r0;
     while (r + 1 < nr && __ldg(lstart + r + 1) <= idx) ++r;
     return __ldg(start + r) + (idx - __ldg(lstart + r));
 }
+
+// The 32 ranges a warp needs for a tile, one per lane.  A range holds at most
+// kTile particles (or is the only one), so range r starts at or before particle
+// r kTile and the tile's first range is at or after base / kTile: usually that
+// one or the next, since a step's losses are few.  One coalesced load and a
+// ballot replace the binary search's chain of dependent loads (1 M particles: ten
+// per tile); only a window that ends before the tile does falls back to it.
+struct RangeWindow {
+    unsigned start, delta;  // this lane's range: logical start, slot minus logical index
+    unsigned first, last;   // window indices of the ranges at the tile's ends
+    unsigned r0;
+    bool whole;
+    __device__ __forceinline__ RangeWindow(const unsigned* lstart, const unsigned* rstart, unsigned nr, unsigned base,
+                                           unsigned end, int lane) {
+        r0 = nr ? min(base / (unsigned)kTile, nr - 1u) : 0u;
+        load(lstart, rstart, nr, lane);
+        first = __popc(__ballot_sync(0xffffffffu, start <= base));
+        if (first == 32u && r0 + 32u < nr) {  // (uniform) heavy losses: search, and load again from there
+            r0 = range_of(lstart, nr, base);
+            load(lstart, rstart, nr, lane);
+            first = __popc(__ballot_sync(0xffffffffu, start <= base));
+        }
+        first = first ? first - 1u : 0u;
+        last = __popc(__ballot_sync(0xffffffffu, start < end));
+        last = last ? last - 1u : 0u;
+        whole = last < 31u || r0 + 32u >= nr;
+    }
+    __device__ __forceinline__ void load(const unsigned* lstart, const unsigned* rstart, unsigned nr, int lane) {
+        const bool in = r0 + lane < nr;
+        start = in ? __ldg(lstart + r0 + lane) : 0xFFFFFFFFu;
+        delta = in ? __ldg(rstart + r0 + lane) - start : 0u;
+    }
+    // slot of particle idx of the tile (all lanes call; `live`: this lane's particle exists)
+    __device__ __forceinline__ unsigned slot(const unsigned* lstart, const unsigned* rstart, unsigned nr, unsigned idx,
+                                             bool live) const {
+        if (!whole) return live ? physical_slot_from(lstart, rstart, nr, r0 + first, idx) : 0u;
+        unsigned d = __shfl_sync(0xffffffffu, delta, first);
+        for (unsigned w = first + 1; w <= last; ++w) {
+            const unsigned s = __shfl_sync(0xffffffffu, start, w), e = __shfl_sync(0xffffffffu, delta, w);
+            if (idx >= s) d = e;
+        }
+        return idx + d;
+    }
+};
 
 // ---- campaign diagnostics stencil ---------------------------------------------
 
@@ -332,9 +379,8 @@ __device__ __forceinline__ void collision_energy_deposit(const Params1D& p, doub
 struct CandidateEntry {
     double v[3];
     double x;
-    double first_wait;
+    uint64_t draw;  // the first raw draw (its waiting time falls inside the step)
     unsigned slot;
-    unsigned draws;
 };
 constexpr int kQueue = 384;
 
@@ -376,12 +422,18 @@ __device__ __noinline__ bool bgk_relax(uint64_t seed, unsigned idx, uint32_t ste
     return true;
 }
 
-// DIAG: the instantiation that also deposits the spatial collision energy,
-// keeps the electric-work ledger and applies the legacy BGK model (run only
-// inside a campaign-diagnostics window, with the ledger or with BGK, so the
-// plain pass keeps its register allocation).
-template <int VDIM, bool DIRICHLET, bool F32, bool DIAG>
-__global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
+// The pass's instantiations: without collision models (a kernel a third of the
+// size: the collision code cost a collisionless pass its registers and its
+// instruction cache; 1 M particles on 64 nodes, with the range window above, 36 -> 21 us)
+// and the one that takes them, deposits the spatial collision energy, keeps the
+// electric-work ledger and applies the legacy BGK model (start and read-back
+// passes, campaign-diagnostics windows, the ledger, BGK).
+// The steady step of runs with collision models and none of these is k_pass1d_mcc.
+enum : int { kPassPlain = 0, kPassDiag = 1 };
+
+template <int VDIM, bool DIRICHLET, bool F32, int KIND>
+__global__ void __launch_bounds__(kThreads, KIND == kPassPlain ? kPlainBlocks<VDIM> : kMinBlocks) k_pass1d(Params1D p) {
+    constexpr bool MCC = KIND != kPassPlain, DIAG = MCC;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     double* sE = reinterpret_cast<double*>(smem_raw);
     unsigned* sLo = reinterpret_cast<unsigned*>(sE + p.nx);  // the fixed-point density (shared_add64)
@@ -394,7 +446,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
     __shared__ unsigned s_cand[kWarps], s_null[kWarps], s_chan[kWarps][kMaxModels][kMaxChannels];
     __shared__ double s_energy[kWarps][kMaxModels][kMaxChannels];
     __shared__ unsigned s_qlen;
-    __shared__ CandidateEntry s_queue[kQueue];
+    __shared__ CandidateEntry s_queue[MCC ? kQueue : 1];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned mode = p.mode;
@@ -403,12 +455,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
         sLo[i] = 0u;
         sHi[i] = 0u;
     }
-    for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
-        (&s_chan[warp][0][0])[i] = 0u;
-        (&s_energy[warp][0][0])[i] = 0.0;
+    if (MCC) {
+        for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
+            (&s_chan[warp][0][0])[i] = 0u;
+            (&s_energy[warp][0][0])[i] = 0.0;
+        }
+        if (lane == 0) s_cand[warp] = s_null[warp] = 0u;
+        if (tid == 0) s_qlen = 0;
     }
-    if (lane == 0) s_cand[warp] = s_null[warp] = 0u;
-    if (tid == 0) s_qlen = 0;
     DevState* st = p.st;
     unsigned tiles_before[kMaxSpecies + 1];
     tiles_before[0] = 0;
@@ -427,12 +481,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
         const unsigned n = st->n[s];
         const unsigned nr = st->nranges[s];
         const unsigned base = tile * kTile;
-        const bool mcc = (mode & kModeSyncMcc) && S.model >= 0;
-        // one search per warp for the range of its first particle
-        const unsigned wfirst = base + (unsigned)(tid & ~31);
-        unsigned r0 = 0;
-        if (lane == 0 && wfirst < n) r0 = range_of(S.rlstart[0], nr, wfirst);
-        r0 = __shfl_sync(0xffffffffu, r0, 0);
+        const bool mcc = MCC && (mode & kModeSyncMcc) && S.model >= 0;
+        const RangeWindow rw(S.rlstart[0], S.rstart[0], nr, base, min(base + (unsigned)kTile, n), lane);
 
         double x[kItems], vh[kItems], vy[kItems], vz[kItems], vc[kItems], Ek[kItems];
         double vo[kItems];  // DIAG with the ledger: v at the end of the particle's last step
@@ -445,7 +495,8 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
             const bool live = idx < n;
             keep[k] = live;
             queued[k] = -1;
-            const unsigned ph = live ? physical_slot_from(S.rlstart[0], S.rstart[0], nr, r0, idx) : 0u;
+            const unsigned slot = rw.slot(S.rlstart[0], S.rstart[0], nr, idx, live);
+            const unsigned ph = live ? slot : 0u;
             x[k] = live ? S.x[0][ph] : 0.0;
             vh[k] = live ? ld_comp<F32>(S.vh[0], S.vh32[0], ph) : 0.0;
             vy[k] = (VDIM == 3 && live) ? ld_comp<F32>(S.vy[0], S.vy32[0], ph) : 0.0;
@@ -480,7 +531,6 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                     queued[k] = -2;  // re-initialise the half step in phase C
                 }
                 if (mcc) {
-                    const MccModelDev& M = p.model[S.model];
                     // first iteration of NullCollisionModel::collide, src/Collision.cpp:926-933
                     const double s2 = vc[k] * vc[k] + vy[k] * vy[k] + vz[k] * vz[k];
                     if (!isfinite(s2)) {  // NullCollisionModel rejects non-finite velocities, src/Collision.cpp:910-916
@@ -488,28 +538,21 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                         continue;
                     }
                     // validate_frequency_bound at |v| (1V: src/Collision.cpp:856) or at speed(v)
-                    if (!(s2 <= M.v_safe2) && !frequency_bound_ok(M, VDIM == 3 ? sqrt(s2) : fabs(vc[k])))
+                    if (!(s2 <= p.model[S.model].v_safe2) &&
+                        !frequency_bound_ok_far(p.gmodel[S.model], VDIM == 3 ? sqrt(s2) : fabs(vc[k])))
                         atomicOr(&st->error, kErrMajorant);
-                    PhiloxStream rng(p.seed, idx, mcc_step, (uint32_t)s);
+                    PhiloxDraws<true> rng(p.seed, idx, mcc_step, (uint32_t)s);
                     const uint64_t d0 = rng.next();
-                    // the raw-draw threshold decides exactly as -log(u)/nu < dt would
-                    bool cand = d0 != 0ull ? (!S.no_candidates && d0 >= S.cand_draw_min) : true;
-                    double wait = 0.0;
-                    if (cand) {
-                        double u = d0 != 0ull ? canonical_of(d0) : 0.0;
-                        for (int guard = 0; !(u > 0.0) && guard < 64; ++guard) u = uniform01(rng);
-                        wait = -log(u) / M.max_frequency;
-                        cand = isfinite(wait) && wait < p.dt;
-                    }
-                    if (cand) {
+                    // the raw-draw threshold decides exactly as -log(u)/nu < dt would (a zero
+                    // draw is redrawn: the collision loop decides)
+                    if (d0 == 0ull || (!S.no_candidates && d0 >= S.cand_draw_min)) {
                         const unsigned q = atomicAdd(&s_qlen, 1u);
                         if (q < (unsigned)kQueue) {
                             CandidateEntry& ce = s_queue[q];
                             ce.v[0] = vc[k]; ce.v[1] = vy[k]; ce.v[2] = vz[k];
-                            ce.first_wait = wait;
                             ce.x = x[k];
+                            ce.draw = d0;
                             ce.slot = idx;
-                            ce.draws = rng.index;
                             queued[k] = (int)q;
                         } else {
                             atomicOr(&st->error, kErrBirths);  // queue sized for > 30% candidates per tile
@@ -518,22 +561,27 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                 }
             }
         }
-        __syncthreads();
+        if (MCC) __syncthreads();
         // -- phase B: full collision loops of the queued candidates --
-        if (mcc) {
+        if (MCC && mcc) {
             const unsigned qlen = min(s_qlen, (unsigned)kQueue);
             const MccModelDev& M = p.model[S.model];
             for (unsigned q0 = warp * 32; q0 < qlen; q0 += kThreads) {
                 CollideResult r;
                 if (q0 + lane < qlen) {
                 CandidateEntry& ce = s_queue[q0 + lane];
-                PhiloxStream rng(p.seed, ce.slot, mcc_step, (uint32_t)s);
-                rng.seek(ce.draws);
+                PhiloxDraws<true> rng(p.seed, ce.slot, mcc_step, (uint32_t)s);
+                rng.seek(1u);
+                const MccModelDev& G = p.gmodel[S.model];
+                double u = ce.draw != 0ull ? canonical_of(ce.draw) : 0.0;
+                for (int guard = 0; !(u > 0.0) && guard < 64; ++guard) u = uniform01(rng);
+                const double first_wait = -log(u) / M.max_frequency;
+                auto bound_ok = [&](double speed) { return frequency_bound_ok_far(G, speed); };
                 unsigned nion = 0;
                 const unsigned slot = ce.slot;
                 const double px = ce.x;
                 double vel[3] = {ce.v[0], ce.v[1], ce.v[2]};
-                if (VDIM == 1) collide1(M, vel[0], p.dt, rng, r, true, ce.first_wait);
+                if (VDIM == 1) collide1(M, vel[0], p.dt, rng, r, true, first_wait, bound_ok);
                 else collide3(M, vel, p.dt, rng, r,
                          [&](int ch, const double* vs, const double* vi) {
                              const unsigned bslot = atomicAdd(&st->nbirths, 2u);
@@ -559,7 +607,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                              atomicAdd(&st->chan_energy[S.model][ch], added);
                              ++nion;
                          },
-                         true, ce.first_wait);
+                         true, first_wait, bound_ok);
                 if (r.error) atomicOr(&st->error, r.error);
                 if (DIAG && p.coll_acc) {
                     // tracked_energy_change, src/Simulation.cpp:862-923: the weighted
@@ -585,13 +633,14 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
                 }
             }
             __syncthreads();
+            if (tid == 0) s_qlen = 0;  // (every thread has read it; the next tile adds after a barrier)
         }
         // -- phase C: re-initialise, kick, drift, walls, deposit --
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             if (!keep[k]) continue;
             const double E = Ek[k];
-            if (mcc) {
+            if (MCC && mcc) {
                 if (queued[k] >= 0) {
                     const CandidateEntry& ce = s_queue[queued[k]];
                     vc[k] = ce.v[0]; vy[k] = ce.v[1]; vz[k] = ce.v[2];
@@ -640,38 +689,43 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
             const double w = warp_sum(wsum);
             if (lane == 0 && w != 0.0) atomicAdd(&st->work[s], w);
         }
-        // ---- order-preserving compaction of the survivors ----
+        // ---- order-preserving compaction of the survivors: nothing moves in a
+        // tile that lost no particle (every tile of a periodic run, most others) ----
+        bool lost_any = false;
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) lost_any = lost_any || (base + k * kThreads + tid < n && !keep[k]);
+        const bool compact = __syncthreads_or(lost_any);
         unsigned ballots[kItems];
+        if (compact) {
 #pragma unroll
-        for (int k = 0; k < kItems; ++k) {
-            ballots[k] = __ballot_sync(0xffffffffu, keep[k]);
-            if (lane == 0) s_cnt[k * (kThreads / 32) + warp] = __popc(ballots[k]);
-        }
-        __syncthreads();
-        if (warp == 0) {
-            const unsigned c = lane < kWarpCounts ? s_cnt[lane] : 0u;
-            unsigned incl = c;
+            for (int k = 0; k < kItems; ++k) {
+                ballots[k] = __ballot_sync(0xffffffffu, keep[k]);
+                if (lane == 0) s_cnt[k * (kThreads / 32) + warp] = __popc(ballots[k]);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                const unsigned c = lane < kWarpCounts ? s_cnt[lane] : 0u;
+                unsigned incl = c;
 #pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
-                if (lane >= o) incl += y;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+                    if (lane >= o) incl += y;
+                }
+                s_cnt[lane] = incl - c;
+                const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
+                if (lane == 0) S.chunk_surv[tile] = total;
             }
-            s_cnt[lane] = incl - c;
-            const unsigned total = __shfl_sync(0xffffffffu, incl, 31);
-            if (lane == 0) {
-                S.chunk_surv[tile] = total;
-                s_qlen = 0;
-            }
+            __syncthreads();
+        } else if (tid == 0) {
+            S.chunk_surv[tile] = min((unsigned)kTile, n - base);
         }
-        __syncthreads();
         // survivors of this chunk keep their order at the chunk's own slots
-        const unsigned long long out_base = base;
         const unsigned lt = (1u << lane) - 1u;
 #pragma unroll
         for (int k = 0; k < kItems; ++k) {
             if (!keep[k]) continue;
-            const unsigned long long o =
-                out_base + s_cnt[k * (kThreads / 32) + warp] + __popc(ballots[k] & lt);
+            const unsigned o = base + (compact ? s_cnt[k * (kThreads / 32) + warp] + __popc(ballots[k] & lt)
+                                               : (unsigned)(k * kThreads + tid));
             if (o >= S.capacity) { atomicOr(&st->error, kErrCapacity); continue; }
             S.x[1][o] = x[k];
             st_comp<F32>(S.vh[1], S.vh32[1], o, vh[k]);
@@ -682,16 +736,321 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks) k_pass1d(Params1D p) {
             if (mode & (kModeWriteV | kModeInitHalf)) S.v[o] = vc[k];
             if (DIAG && p.ledger) S.vold[1][o] = (mode & (kModeSyncMcc | kModeInitHalf)) ? vc[k] : vo[k];
         }
-        __syncthreads();
+        if (compact) __syncthreads();
     }
+    __syncthreads();
     if (mode & kModeDeposit) {
         for (int i = tid; i < p.nx; i += kThreads) {
             const unsigned long long a = join64(sLo[i], sHi[i]);
             if (a) atomicAdd(&p.rho_acc[i], a);
         }
     }
-    // (the tile loop ends on a barrier)
-    if ((mode & kModeSyncMcc) && tid < kMaxModels * kMaxChannels) {
+    if (MCC && (mode & kModeSyncMcc) && tid < kMaxModels * kMaxChannels) {
+        unsigned long long c = 0ull;
+        double e = 0.0;
+        for (int w = 0; w < kWarps; ++w) {
+            c += (&s_chan[w][0][0])[tid];
+            e += (&s_energy[w][0][0])[tid];
+        }
+        if (c) {
+            atomicAdd(&st->chan[0][0] + tid, c);
+            atomicAdd(&st->chan_energy[0][0] + tid, e);
+        }
+        if (tid < 2) {
+            c = 0ull;
+            for (int w = 0; w < kWarps; ++w) c += tid ? s_null[w] : s_cand[w];
+            if (c) atomicAdd(tid ? &st->nulls : &st->candidates, c);
+        }
+    }
+}
+
+// The steady step of a run with collision models: k_pass1d's phases (synchronize
+// and first draw, collision loops of the candidates, the rest of the step) with the
+// same arithmetic.  A candidate's loop is a chain of several thousand
+// dependent instructions (about 30 us), so the pass takes as long as the tiles that
+// one CTA runs after another: here the CTAs are small and keep no particle
+// state across the collision phase (each phase reads its particles again, from L2), so
+// that four fit an SM and all 512 tiles of a 524,288-particle discharge run
+// at once (pass 64 -> 47 us).  A tile's survivors are written to their own slots and
+// moved up only when the tile lost a particle.
+constexpr int kMccThreads = 128;
+constexpr int kMccBlocks = 4;                                // resident CTAs per SM
+constexpr int kMccBatches = kTile / (kMccThreads * kItems);  // batches of kItems particles per thread
+
+template <int VDIM, bool DIRICHLET, bool F32>
+__global__ void __launch_bounds__(kMccThreads, kMccBlocks) k_pass1d_mcc(Params1D p) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double* sE = reinterpret_cast<double*>(smem_raw);
+    unsigned* sLo = reinterpret_cast<unsigned*>(sE + p.nx);  // the fixed-point density (shared_add64)
+    unsigned* sHi = sLo + p.nx;
+    constexpr int kWarps = kMccThreads / 32;
+    __shared__ unsigned s_cnt[kWarps];
+    __shared__ unsigned s_cand[kWarps], s_null[kWarps], s_chan[kWarps][kMaxModels][kMaxChannels];
+    __shared__ double s_energy[kWarps][kMaxModels][kMaxChannels];
+    __shared__ unsigned s_qlen;
+    __shared__ CandidateEntry s_queue[kQueue];
+    __shared__ unsigned short s_of[kTile];  // queue entry of a candidate, by place in the tile
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (int i = tid; i < p.nx; i += kMccThreads) {
+        sE[i] = p.E[i];
+        sLo[i] = 0u;
+        sHi[i] = 0u;
+    }
+    for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
+        (&s_chan[warp][0][0])[i] = 0u;
+        (&s_energy[warp][0][0])[i] = 0.0;
+    }
+    if (lane == 0) s_cand[warp] = s_null[warp] = 0u;
+    if (tid == 0) s_qlen = 0;
+    DevState* st = p.st;
+    unsigned tiles_before[kMaxSpecies + 1];
+    tiles_before[0] = 0;
+#pragma unroll
+    for (int s = 0; s < kMaxSpecies; ++s)
+        tiles_before[s + 1] = tiles_before[s] + (s < p.nspecies ? (st->n[s] + kTile - 1) / kTile : 0);
+    const unsigned total_tiles = tiles_before[kMaxSpecies];
+    const uint32_t mcc_step = (uint32_t)(st->step - 1ull);
+    __syncthreads();
+
+    for (unsigned t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+        const int s = t < tiles_before[1] ? 0 : (t < tiles_before[2] ? 1 : (t < tiles_before[3] ? 2 : 3));
+        const unsigned tile = t - (s == 0 ? 0u : (s == 1 ? tiles_before[1] : (s == 2 ? tiles_before[2] : tiles_before[3])));
+        const SpeciesDev& S = p.sp[s];
+        const unsigned n = st->n[s];
+        const unsigned nr = st->nranges[s];
+        const unsigned base = tile * kTile;
+        const bool mcc = S.model >= 0;
+        const RangeWindow rw(S.rlstart[0], S.rstart[0], nr, base, min(base + (unsigned)kTile, n), lane);
+        if (mcc) {
+            // -- phase A: gather, synchronize, first collision draw --
+            const MccModelDev& M = p.model[S.model];
+#pragma unroll 1
+            for (int b = 0; b < kMccBatches; ++b) {
+                double x[kItems], vc[kItems], vy[kItems], vz[kItems];
+#pragma unroll
+                for (int k = 0; k < kItems; ++k) {
+                    const unsigned idx = base + (b * kItems + k) * kMccThreads + tid;
+                    const bool live = idx < n;
+                    const unsigned slot = rw.slot(S.rlstart[0], S.rstart[0], nr, idx, live);
+                    const unsigned ph = live ? slot : 0u;
+                    x[k] = live ? S.x[0][ph] : 0.0;
+                    vc[k] = live ? ld_comp<F32>(S.vh[0], S.vh32[0], ph) : 0.0;
+                    vy[k] = (VDIM == 3 && live) ? ld_comp<F32>(S.vy[0], S.vy32[0], ph) : 0.0;
+                    vz[k] = (VDIM == 3 && live) ? ld_comp<F32>(S.vz[0], S.vz32[0], ph) : 0.0;
+                }
+#pragma unroll
+                for (int k = 0; k < kItems; ++k) {
+                    const unsigned place = (b * kItems + k) * kMccThreads + tid, idx = base + place;
+                    s_of[place] = 0xFFFFu;
+                    if (idx >= n) continue;
+                    // synchronize_leapfrog, src/Pusher.cpp:78-80
+                    vc[k] = vc[k] + S.hqm * gather(sE, cic<DIRICHLET>(x[k], p)) * p.dt;
+                    const double s2 = vc[k] * vc[k] + vy[k] * vy[k] + vz[k] * vz[k];
+                    if (!isfinite(s2)) {  // src/Collision.cpp:910-916
+                        atomicOr(&st->error, kErrNonFinite);
+                        continue;
+                    }
+                    // validate_frequency_bound at |v| (1V: src/Collision.cpp:856) or at speed(v)
+                    if (!(s2 <= M.v_safe2) &&
+                        !frequency_bound_ok_far(p.gmodel[S.model], VDIM == 3 ? sqrt(s2) : fabs(vc[k])))
+                        atomicOr(&st->error, kErrMajorant);
+                    uint32_t o[4];
+                    philox4x32_10(0u, idx, mcc_step, (uint32_t)s, (uint32_t)p.seed, (uint32_t)(p.seed >> 32), o);
+                    const uint64_t d0 = (uint64_t)o[1] << 32 | o[0];  // PhiloxStream's first draw
+                    // the raw-draw threshold decides exactly as -log(u)/nu < dt would (a zero
+                    // draw is redrawn: the collision loop decides)
+                    if (d0 == 0ull || (!S.no_candidates && d0 >= S.cand_draw_min)) {
+                        const unsigned q = atomicAdd(&s_qlen, 1u);
+                        if (q < (unsigned)kQueue) {
+                            CandidateEntry& ce = s_queue[q];
+                            ce.v[0] = vc[k]; ce.v[1] = vy[k]; ce.v[2] = vz[k];
+                            ce.x = x[k];
+                            ce.draw = d0;
+                            ce.slot = idx;
+                            s_of[place] = (unsigned short)q;
+                        } else {
+                            atomicOr(&st->error, kErrBirths);  // queue sized for > 30% candidates per tile
+                        }
+                    }
+                }
+            }
+            __syncthreads();
+            // -- phase B: full collision loops of the queued candidates --
+            const unsigned qlen = min(s_qlen, (unsigned)kQueue);
+#pragma unroll 1
+            for (unsigned q0 = warp * 32; q0 < qlen; q0 += kMccThreads) {
+                CollideResult r;
+                if (q0 + lane < qlen) {
+                    CandidateEntry& ce = s_queue[q0 + lane];
+                    PhiloxDraws<true> rng(p.seed, ce.slot, mcc_step, (uint32_t)s);
+                    rng.seek(1u);
+                    const MccModelDev& G = p.gmodel[S.model];
+                    double u = ce.draw != 0ull ? canonical_of(ce.draw) : 0.0;
+                    for (int guard = 0; !(u > 0.0) && guard < 64; ++guard) u = uniform01(rng);
+                    const double first_wait = -log(u) / M.max_frequency;
+                    auto bound_ok = [&](double speed) { return frequency_bound_ok_far(G, speed); };
+                    unsigned nion = 0;
+                    double vel[3] = {ce.v[0], ce.v[1], ce.v[2]};
+                    if (VDIM == 1) collide1(M, vel[0], p.dt, rng, r, true, first_wait, bound_ok);
+                    else collide3(M, vel, p.dt, rng, r,
+                             [&](int ch, const double* vs, const double* vi) {
+                                 const unsigned bslot = atomicAdd(&st->nbirths, 2u);
+                                 const MccChannelDev& C = M.ch[ch];
+                                 if (bslot + 2u <= p.births_cap) {
+                                     const unsigned long long key =
+                                         ((unsigned long long)s << 56) | ((unsigned long long)ce.slot << 16) | (nion << 1);
+                                     BirthRec a, c;
+                                     a.key = key; a.species = C.secondary; a.pad = 0;
+                                     c.key = key | 1ull; c.species = C.ion; c.pad = 0;
+                                     a.x = c.x = ce.x;
+                                     for (int d = 0; d < 3; ++d) { a.v[d] = vs[d]; c.v[d] = vi[d]; }
+                                     p.births[bslot] = a;
+                                     p.births[bslot + 1] = c;
+                                 } else {
+                                     atomicOr(&st->error, kErrBirths);
+                                 }
+                                 const SpeciesDev& A = p.sp[C.secondary];
+                                 const SpeciesDev& B = p.sp[C.ion];
+                                 const double added =
+                                     0.5 * A.mass * A.weight * (vs[0] * vs[0] + vs[1] * vs[1] + vs[2] * vs[2]) +
+                                     0.5 * B.mass * B.weight * (vi[0] * vi[0] + vi[1] * vi[1] + vi[2] * vi[2]);
+                                 atomicAdd(&st->chan_energy[S.model][ch], added);
+                                 ++nion;
+                             },
+                             true, first_wait, bound_ok);
+                    if (r.error) atomicOr(&st->error, r.error);
+                    ce.v[0] = vel[0]; ce.v[1] = vel[1]; ce.v[2] = vel[2];
+                }
+                __syncwarp();
+                const unsigned nc = __reduce_add_sync(0xffffffffu, r.candidates);
+                const unsigned nn = __reduce_add_sync(0xffffffffu, r.nulls);
+                if (lane == 0) { s_cand[warp] += nc; s_null[warp] += nn; }
+#pragma unroll 1
+                for (int ch = 0; ch < M.nch; ++ch) {
+                    const unsigned c = __reduce_add_sync(0xffffffffu, r.channel[ch]);
+                    if (!c) continue;
+                    const double e = warp_sum(r.energy_change[ch] * S.weight);
+                    if (lane == 0) { s_chan[warp][S.model][ch] += c; s_energy[warp][S.model][ch] += e; }
+                }
+            }
+            __syncthreads();
+            if (tid == 0) s_qlen = 0;  // (every thread has read it; the next tile adds after a barrier)
+        }
+        // -- phase C: synchronize again, re-initialise, kick, drift, walls, deposit --
+        unsigned kept = 0u;  // bit b kItems + k: this thread's particle survives
+        bool lost_any = false;
+#pragma unroll 1
+        for (int b = 0; b < kMccBatches; ++b) {
+            double x[kItems], vh[kItems], vy[kItems], vz[kItems];
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const unsigned idx = base + (b * kItems + k) * kMccThreads + tid;
+                const bool live = idx < n;
+                const unsigned slot = rw.slot(S.rlstart[0], S.rstart[0], nr, idx, live);
+                const unsigned ph = live ? slot : 0u;
+                x[k] = live ? S.x[0][ph] : 0.0;
+                vh[k] = live ? ld_comp<F32>(S.vh[0], S.vh32[0], ph) : 0.0;
+                vy[k] = (VDIM == 3 && live) ? ld_comp<F32>(S.vy[0], S.vy32[0], ph) : 0.0;
+                vz[k] = (VDIM == 3 && live) ? ld_comp<F32>(S.vz[0], S.vz32[0], ph) : 0.0;
+            }
+#pragma unroll
+            for (int k = 0; k < kItems; ++k) {
+                const unsigned place = (b * kItems + k) * kMccThreads + tid, idx = base + place;
+                if (idx >= n) continue;
+                const double E = gather(sE, cic<DIRICHLET>(x[k], p));
+                if (mcc) {
+                    double vc = vh[k] + S.hqm * E * p.dt;
+                    const unsigned q = s_of[place];
+                    if (q != 0xFFFFu) {
+                        const CandidateEntry& ce = s_queue[q];
+                        vc = ce.v[0]; vy[k] = ce.v[1]; vz[k] = ce.v[2];
+                    }
+                    // initialize_leapfrog_half_step after the collision, src/Simulation.cpp:924-926
+                    vh[k] = vc - S.hqm * E * p.dt;
+                }
+                // kick_leapfrog + drift_leapfrog, src/Pusher.cpp:70-76
+                vh[k] = vh[k] + S.qm * E * p.dt;
+                x[k] = x[k] + vh[k] * p.dt;
+                bool keep = true;
+                if (!DIRICHLET) {
+                    x[k] = wrap_periodic(x[k], p.L);
+                } else if (x[k] < 0.0 || x[k] > p.L) {
+                    // absorbing walls and loss ledger, src/Simulation.cpp:1047-1077
+                    const double sp2 = vh[k] * vh[k] + vy[k] * vy[k] + vz[k] * vz[k];
+                    const int side = x[k] < 0.0 ? 0 : 1;
+                    atomicAdd(&st->lost[s][side], 1ull);
+                    atomicAdd(&st->lost_energy[s][side], 0.5 * S.mass * S.weight * sp2);
+                    keep = false;
+                }
+                if (!isfinite(x[k]) || !isfinite(vh[k])) {
+                    // flagged and dropped: a non-finite particle deposits nothing
+                    atomicOr(&st->error, kErrNonFinite);
+                    keep = false;
+                }
+                if (!keep) {
+                    lost_any = true;
+                    continue;
+                }
+                kept |= 1u << (b * kItems + k);
+                const Cic d = cic<DIRICHLET>(x[k], p);
+                long long a0, a1;
+                deposit_contrib<DIRICHLET>(d, S, p, a0, a1);
+                shared_add64(sLo, sHi, d.i0, a0);
+                shared_add64(sLo, sHi, d.i1, a1);
+                if (idx >= S.capacity) { atomicOr(&st->error, kErrCapacity); continue; }
+                S.x[1][idx] = x[k];
+                st_comp<F32>(S.vh[1], S.vh32[1], idx, vh[k]);
+                if (VDIM == 3) {
+                    st_comp<F32>(S.vy[1], S.vy32[1], idx, vy[k]);
+                    st_comp<F32>(S.vz[1], S.vz32[1], idx, vz[k]);
+                }
+            }
+        }
+        if (!__syncthreads_or(lost_any)) {
+            if (tid == 0) S.chunk_surv[tile] = min((unsigned)kTile, n - base);
+            continue;
+        }
+        // -- order-preserving compaction in place, one row of kMccThreads places after
+        // another: a row's survivors move to places of this or earlier rows, which
+        // have all been read by then --
+        unsigned out = base;
+#pragma unroll 1
+        for (int r = 0; r < kMccBatches * kItems; ++r) {
+            const unsigned idx = base + r * kMccThreads + tid;
+            const bool keep = (kept >> r) & 1u;
+            const double x = keep ? S.x[1][idx] : 0.0;
+            const double vh = keep ? ld_comp<F32>(S.vh[1], S.vh32[1], idx) : 0.0;
+            const double vy = (VDIM == 3 && keep) ? ld_comp<F32>(S.vy[1], S.vy32[1], idx) : 0.0;
+            const double vz = (VDIM == 3 && keep) ? ld_comp<F32>(S.vz[1], S.vz32[1], idx) : 0.0;
+            const unsigned bal = __ballot_sync(0xffffffffu, keep);
+            if (lane == 0) s_cnt[warp] = __popc(bal);
+            __syncthreads();
+            unsigned o = out + __popc(bal & ((1u << lane) - 1u));
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) {
+                const unsigned c = s_cnt[w];
+                if (w < warp) o += c;
+                out += c;
+            }
+            if (keep && o != idx) {
+                S.x[1][o] = x;
+                st_comp<F32>(S.vh[1], S.vh32[1], o, vh);
+                if (VDIM == 3) {
+                    st_comp<F32>(S.vy[1], S.vy32[1], o, vy);
+                    st_comp<F32>(S.vz[1], S.vz32[1], o, vz);
+                }
+            }
+            __syncthreads();
+        }
+        if (tid == 0) S.chunk_surv[tile] = out - base;
+    }
+    __syncthreads();
+    for (int i = tid; i < p.nx; i += kMccThreads) {
+        const unsigned long long a = join64(sLo[i], sHi[i]);
+        if (a) atomicAdd(&p.rho_acc[i], a);
+    }
+    if (tid < kMaxModels * kMaxChannels) {
         unsigned long long c = 0ull;
         double e = 0.0;
         for (int w = 0; w < kWarps; ++w) {
@@ -845,18 +1204,43 @@ __host__ __device__ inline size_t post_smem_bytes(int nx, bool dirichlet) {
            (dirichlet ? (size_t)2 * nx * 8 : (size_t)2 * nx * 8 /* twiddles */ + ((size_t)5 * nx + 2) * 8 /* spectra */);
 }
 
+// Exclusive sum of one value per thread over the CTA; `total` is the same in
+// every thread.  s_w holds one word per warp.
+__device__ __forceinline__ unsigned block_exclusive_sum(unsigned v, unsigned* s_w, unsigned& total) {
+    constexpr int NW = kPostThreads / 32;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += y;
+    }
+    if (lane == 31) s_w[warp] = incl;
+    __syncthreads();
+    const unsigned w = lane < NW ? s_w[lane] : 0u;
+    const unsigned before = __reduce_add_sync(0xffffffffu, lane < warp ? w : 0u);
+    total = __reduce_add_sync(0xffffffffu, w);
+    __syncthreads();
+    return before + incl - v;
+}
+
+// One CTA per step.  Its time is latency: a chain of a few loads and scans, and the
+// fetch of its own instructions, which no other CTA shares (most of
+// its stalls).  So the loops are kept rolled and a thread handles one chunk, one
+// product, one node at a time (two-stream deck on 128 nodes: 17.3 -> 13.4 us between
+// events around the launch).
 template <int VDIM, bool DIRICHLET, bool F32, bool C32 = false>
 __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned post) {
     using Sort = cub::BlockRadixSort<unsigned long long, kPostThreads, kPostItems, int>;
-    using ScanU = cub::BlockScan<unsigned, kPostThreads>;
     __shared__ union {
         typename Sort::TempStorage sort;
-        typename ScanU::TempStorage scan;
+        unsigned long long keys[kPostThreads];
     } tmp;
+    __shared__ unsigned short s_order[kMaxBirths];  // products in rank order
+    __shared__ unsigned s_scan[kPostThreads / 32];
     __shared__ unsigned s_surv[kMaxSpecies], s_kept[kMaxSpecies], s_bstart[kMaxSpecies], s_nch[kMaxSpecies];
     __shared__ double s_red[kPostThreads / 32];
-    __shared__ double s_mean;
-    __shared__ unsigned s_carry;
+    __shared__ double s_mean, s_electrode[2];
     extern __shared__ __align__(16) unsigned char post_raw[];
     const int nx = p.nx;
     unsigned long long* s_rhoi = reinterpret_cast<unsigned long long*>(post_raw);
@@ -865,22 +1249,27 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
     double* s_c1 = s_c0 + nx;                        // Dirichlet: -cp
     double* s_spec = s_c0 + 2 * nx;                  // periodic: the spectrum and a transform's middle
     DevState* st = p.st;
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool solve = (post & kPostSolve) != 0;
+    const double field_time = (post & kPostAdvance) ? st->time + p.dt : st->time;
 
     // -- one round trip: density accumulators and solver coefficients --
     if (solve) {
+#pragma unroll 1
         for (int i = tid; i < nx; i += kPostThreads) {
             s_rhoi[i] = p.rho_acc[i];
             p.rho_acc[i] = 0ull;
             if (DIRICHLET) {
                 if (i < nx - 2) { s_c0[i] = p.thomas_r[i]; s_c1[i] = p.thomas_a[i]; }
             } else {
-                s_c0[2 * i] = p.tw[2 * i];
-                s_c0[2 * i + 1] = p.tw[2 * i + 1];
+                reinterpret_cast<double2*>(s_c0)[i] = reinterpret_cast<const double2*>(p.tw)[i];
             }
         }
+        // one lane of two warps each: the sine's code is there once
+        if (DIRICHLET && lane == 0 && warp < 2)
+            s_electrode[warp] = electrode(warp ? p.phi_right : p.phi_left, warp ? p.drive_right : p.drive_left, field_time);
     }
+    unsigned nb = st->nbirths;
 
     // -- output range table: chunk c of the pass kept its survivors at slots
     //    [c * kTile, c * kTile + surv_c); logical starts are their prefix sums
@@ -892,49 +1281,37 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
             s_surv[tid] = st->n[tid];
             s_bstart[tid] = st->n[tid];
             s_nch[tid] = 0;
-            s_kept[tid] = 0;
         }
-        __syncthreads();
     }
+    if (tid < p.nspecies) s_kept[tid] = 0;
+#pragma unroll 1
     for (int s = 0; s < (C32 ? 0 : p.nspecies); ++s) {
         const SpeciesDev& S = p.sp[s];
         const unsigned nch = (st->n[s] + CHUNK - 1) / CHUNK;
-        if (tid == 0) s_carry = 0;
-        __syncthreads();
-        for (unsigned b0 = 0; b0 < nch; b0 += kPostThreads * kPostItems) {
-            unsigned cnt[kPostItems], pre[kPostItems];
-#pragma unroll
-            for (int k = 0; k < kPostItems; ++k) {
-                const unsigned c = b0 + tid * kPostItems + k;
-                cnt[k] = c < nch ? S.chunk_surv[c] : 0u;
-            }
+        unsigned carry = 0;
+#pragma unroll 1
+        for (unsigned b0 = 0; b0 < nch; b0 += kPostThreads) {
+            const unsigned c = b0 + tid;
+            const unsigned cnt = c < nch ? S.chunk_surv[c] : 0u;
             unsigned total;
-            ScanU(tmp.scan).ExclusiveSum(cnt, pre, total);
-            const unsigned carry = s_carry;
-#pragma unroll
-            for (int k = 0; k < kPostItems; ++k) {
-                const unsigned c = b0 + tid * kPostItems + k;
-                if (c < nch) {
-                    S.rstart[1][c] = c * CHUNK;
-                    S.rcount[1][c] = cnt[k];
-                    S.rlstart[1][c] = carry + pre[k];
-                }
+            const unsigned pre = block_exclusive_sum(cnt, s_scan, total);
+            if (c < nch) {
+                S.rstart[1][c] = c * CHUNK;
+                S.rcount[1][c] = cnt;
+                S.rlstart[1][c] = carry + pre;
+                if (c == nch - 1) s_bstart[s] = c * CHUNK + cnt;
             }
-            __syncthreads();
-            if (tid == 0) s_carry = carry + total;
-            __syncthreads();
+            carry += total;
         }
         if (tid == 0) {
-            s_surv[s] = s_carry;
+            s_surv[s] = carry;
             s_nch[s] = nch;
-            s_bstart[s] = nch ? (nch - 1) * CHUNK + S.chunk_surv[nch - 1] : 0u;
-            s_kept[s] = 0;
+            if (!nch) s_bstart[s] = 0u;
         }
-        __syncthreads();
     }
+    __syncthreads();
 
     // -- ionization products, in (parent species, parent slot, product) order --
-    unsigned nb = st->nbirths;
     if (nb > p.births_cap) nb = p.births_cap;
     if (nb > (unsigned)kMaxBirths) {
         if (tid == 0) atomicOr(&st->error, kErrBirths);
@@ -955,38 +1332,26 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         }
     }
     if (nb > 0) {
-        int idx[kPostItems];
-        // up to one product per thread: rank tid in item 0 (the blocked scans
-        // below then still visit the products in rank order); more: the radix
-        // sort's blocked layout, ranks tid * kPostItems + k
-        const bool one_each = nb <= (unsigned)kPostThreads;
-        auto rank_of = [&](int k) -> unsigned {
-            return one_each ? (k == 0 ? (unsigned)tid : nb) : (unsigned)(tid * kPostItems + k);
-        };
-        if (one_each) {
-            // a few products (the usual case): each finds its rank by counting
-            // the smaller keys, one key per thread
-            __shared__ unsigned long long s_keys[kPostThreads];
-            __shared__ int s_order[kPostThreads];
-            if (tid < (int)nb) s_keys[tid] = p.births[tid].key;
+        if (nb <= (unsigned)kPostThreads) {
+            // a few products (the usual case): a key's rank is the number of
+            // smaller keys, counted by one warp per key
+            if (tid < (int)nb) tmp.keys[tid] = p.births[tid].key;
             __syncthreads();
-            if (tid < (int)nb) {
-                const unsigned long long key = s_keys[tid];
+#pragma unroll 1
+            for (unsigned i = warp; i < nb; i += kPostThreads / 32) {
+                const unsigned long long key = tmp.keys[i];
                 unsigned r = 0;
-                for (unsigned q = 0; q < nb; ++q) {
-                    const unsigned long long o = s_keys[q];
-                    r += (o < key || (o == key && q < (unsigned)tid)) ? 1u : 0u;
+#pragma unroll 1
+                for (unsigned q = lane; q < nb; q += 32) {
+                    const unsigned long long o = tmp.keys[q];
+                    r += (o < key || (o == key && q < i)) ? 1u : 0u;
                 }
-                s_order[r] = tid;
-            }
-            __syncthreads();
-#pragma unroll
-            for (int k = 0; k < kPostItems; ++k) {
-                const unsigned rank = rank_of(k);
-                idx[k] = rank < nb ? s_order[rank] : 0;
+                r = __reduce_add_sync(0xffffffffu, r);
+                if (lane == 0) s_order[r] = (unsigned short)i;
             }
         } else {
             unsigned long long keys[kPostItems];
+            int idx[kPostItems];
 #pragma unroll
             for (int k = 0; k < kPostItems; ++k) {
                 const unsigned i = tid * kPostItems + k;
@@ -994,82 +1359,75 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
                 idx[k] = (int)i;
             }
             Sort(tmp.sort).Sort(keys, idx);
+#pragma unroll
+            for (int k = 0; k < kPostItems; ++k) s_order[tid * kPostItems + k] = (unsigned short)idx[k];
         }
         __syncthreads();
-        double bx[kPostItems], bvh[kPostItems], bv[kPostItems][3];
-        int bs[kPostItems];
-        bool keep[kPostItems];
-#pragma unroll
-        for (int k = 0; k < kPostItems; ++k) {
-            keep[k] = false;
-            bs[k] = -1;
-            const unsigned rank = rank_of(k);
-            if (rank >= nb) continue;
-            const BirthRec r = p.births[idx[k]];
-            const SpeciesDev& S = p.sp[r.species];
-            bs[k] = r.species;
-            bx[k] = r.x;
-            bv[k][0] = r.v[0]; bv[k][1] = r.v[1]; bv[k][2] = r.v[2];
-            const double E = gather(p.E, cic<DIRICHLET>(r.x, p));
-            // append_product: v_half = v, then initialize_leapfrog_half_step, src/Simulation.cpp:985-1004
-            bvh[k] = r.v[0] - S.hqm * E * p.dt;
-            keep[k] = true;
-            if (post & kPostPushBirths) {
-                bvh[k] = bvh[k] + S.qm * E * p.dt;
-                bx[k] = bx[k] + bvh[k] * p.dt;
-                if (!DIRICHLET) {
-                    bx[k] = wrap_periodic(bx[k], p.L);
-                } else if (bx[k] < 0.0 || bx[k] > p.L) {
-                    if (p.ledger) {  // electric work of a wall crossing, src/Simulation.cpp:1047-1056
-                        const double hmw = 0.5 * S.mass * S.weight;
-                        atomicAdd(&st->work[r.species], hmw * bvh[k] * bvh[k] - hmw * bv[k][0] * bv[k][0]);
+#pragma unroll 1
+        for (unsigned b0 = 0; b0 < nb; b0 += kPostThreads) {
+            double bx = 0.0, bvh = 0.0, bv[3] = {0.0, 0.0, 0.0};
+            int bs = -1;  // species of this thread's product (none, or lost to a wall: -1)
+            if (b0 + tid < nb) {
+                const BirthRec r = p.births[s_order[b0 + tid]];
+                const SpeciesDev& S = p.sp[r.species];
+                bs = r.species;
+                bx = r.x;
+                bv[0] = r.v[0]; bv[1] = r.v[1]; bv[2] = r.v[2];
+                const double E = gather(p.E, cic<DIRICHLET>(r.x, p));
+                // append_product: v_half = v, then initialize_leapfrog_half_step, src/Simulation.cpp:985-1004
+                bvh = r.v[0] - S.hqm * E * p.dt;
+                if (post & kPostPushBirths) {
+                    bvh = bvh + S.qm * E * p.dt;
+                    bx = bx + bvh * p.dt;
+                    if (!DIRICHLET) {
+                        bx = wrap_periodic(bx, p.L);
+                    } else if (bx < 0.0 || bx > p.L) {
+                        if (p.ledger) {  // electric work of a wall crossing, src/Simulation.cpp:1047-1056
+                            const double hmw = 0.5 * S.mass * S.weight;
+                            atomicAdd(&st->work[r.species], hmw * bvh * bvh - hmw * bv[0] * bv[0]);
+                        }
+                        const double sp2 = bvh * bvh + bv[1] * bv[1] + bv[2] * bv[2];
+                        const int side = bx < 0.0 ? 0 : 1;
+                        atomicAdd(&st->lost[r.species][side], 1ull);
+                        atomicAdd(&st->lost_energy[r.species][side], 0.5 * S.mass * S.weight * sp2);
+                        bs = -1;
                     }
-                    const double sp2 = bvh[k] * bvh[k] + bv[k][1] * bv[k][1] + bv[k][2] * bv[k][2];
-                    const int side = bx[k] < 0.0 ? 0 : 1;
-                    atomicAdd(&st->lost[r.species][side], 1ull);
-                    atomicAdd(&st->lost_energy[r.species][side], 0.5 * S.mass * S.weight * sp2);
-                    keep[k] = false;
-                }
-                if (keep[k] && solve) {
-                    const Cic d = cic<DIRICHLET>(bx[k], p);
-                    long long a0, a1;
-                    deposit_contrib<DIRICHLET>(d, S, p, a0, a1);
-                    atomicAdd(&s_rhoi[d.i0], (unsigned long long)a0);
-                    atomicAdd(&s_rhoi[d.i1], (unsigned long long)a1);
+                    if (bs >= 0 && solve) {
+                        const Cic d = cic<DIRICHLET>(bx, p);
+                        long long a0, a1;
+                        deposit_contrib<DIRICHLET>(d, S, p, a0, a1);
+                        atomicAdd(&s_rhoi[d.i0], (unsigned long long)a0);
+                        atomicAdd(&s_rhoi[d.i1], (unsigned long long)a1);
+                    }
                 }
             }
-        }
-        for (int s = 0; s < p.nspecies; ++s) {
-            unsigned flags[kPostItems], ranks[kPostItems];
-#pragma unroll
-            for (int k = 0; k < kPostItems; ++k) flags[k] = (keep[k] && bs[k] == s) ? 1u : 0u;
-            unsigned total;
-            __syncthreads();
-            ScanU(tmp.scan).ExclusiveSum(flags, ranks, total);
-            const SpeciesDev& S = p.sp[s];
-#pragma unroll
-            for (int k = 0; k < kPostItems; ++k) {
-                if (!flags[k]) continue;
-                const unsigned long long o = (unsigned long long)s_bstart[s] + ranks[k];
+#pragma unroll 1
+            for (int s = 0; s < p.nspecies; ++s) {
+                unsigned total;
+                const unsigned rank = block_exclusive_sum(bs == s ? 1u : 0u, s_scan, total);
+                const unsigned long long o = (unsigned long long)s_bstart[s] + s_kept[s] + rank;
+                __syncthreads();
+                if (tid == 0) s_kept[s] += total;
+                if (bs != s) continue;
+                const SpeciesDev& S = p.sp[s];
                 if (o >= S.capacity) { atomicOr(&st->error, kErrCapacity); continue; }
                 if (C32) {
                     int c;
                     float f;
-                    position_to_cell<DIRICHLET>(bx[k], p, c, f);
+                    position_to_cell<DIRICHLET>(bx, p, c, f);
                     S.cell[OUT][o] = c;
                     S.off[OUT][o] = f;
                 } else {
-                    S.x[OUT][o] = bx[k];
+                    S.x[OUT][o] = bx;
                 }
-                st_comp<F32>(S.vh[OUT], S.vh32[OUT], o, bvh[k]);
+                st_comp<F32>(S.vh[OUT], S.vh32[OUT], o, bvh);
                 if (VDIM == 3) {
-                    st_comp<F32>(S.vy[OUT], S.vy32[OUT], o, bv[k][1]);
-                    st_comp<F32>(S.vz[OUT], S.vz32[OUT], o, bv[k][2]);
+                    st_comp<F32>(S.vy[OUT], S.vy32[OUT], o, bv[1]);
+                    st_comp<F32>(S.vz[OUT], S.vz32[OUT], o, bv[2]);
                 }
-                S.v[o] = bv[k][0];
-                if (p.ledger) S.vold[OUT][o] = bv[k][0];
+                S.v[o] = bv[0];
+                if (p.ledger) S.vold[OUT][o] = bv[0];
             }
-            if (tid == 0) s_kept[s] = total;
         }
         __syncthreads();
     }
@@ -1100,13 +1458,13 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
 
     // -- density: fixed point -> FP64 ---------------------------------------
     double local = 0.0;
+#pragma unroll 1
     for (int i = tid; i < nx; i += kPostThreads) {
         const double r = (double)(long long)s_rhoi[i] * p.inv_rho_scale;
         s_rho[i] = r;
         p.rho[i] = r;
         local += r;
     }
-    const double field_time = (post & kPostAdvance) ? st->time + p.dt : st->time;
     if (!DIRICHLET) {
         // solve_periodic_spectral(Grid&), src/FieldSolver.cpp:407-440
         for (int o = 16; o > 0; o >>= 1) local += __shfl_down_sync(0xffffffffu, local, o);
@@ -1119,7 +1477,7 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         }
         __syncthreads();
         const double mean = s_mean;
-        const double twopi = 2.0 * 3.141592653589793;
+        const double wave1 = 2.0 * 3.141592653589793 / p.L;
         const int half = nx / 2;
         double2* const spec = reinterpret_cast<double2*>(s_spec);  // phi_k, k <= nx / 2
         double2* const mid = spec + half + 1;                      // 2 nx values
@@ -1129,7 +1487,7 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         dft_two_step<1>(
             nx, p.dft_n1, half + 1, -1.0, tw, [&](int j, double2* v) { v[0] = {s_rho[j] - mean, 0.0}; }, mid,
             [&](int k, const double2* v) {
-                const double wave = twopi * (double)k / p.L;
+                const double wave = wave1 * (double)k;
                 const double den = p.eps * wave * wave * (double)nx;
                 spec[k] = k ? double2{v[0].x / den, v[0].y / den} : double2{0.0, 0.0};
             });
@@ -1141,7 +1499,7 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
             [&](int k, double2* v) {
                 const bool upper = k > half;
                 const double2 a = spec[upper ? nx - k : k];
-                const double wave = twopi * (double)(upper ? k - nx : k) / p.L;
+                const double wave = wave1 * (double)(upper ? k - nx : k);
                 v[0] = {a.x, upper ? -a.y : a.y};
                 v[1] = {wave * v[0].y, -(wave * v[0].x)};
             },
@@ -1153,33 +1511,37 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         __syncthreads();
         // solve_dirichlet_tridiagonal, src/FieldSolver.cpp:733-759, with the
         // forward sweep and the back substitution evaluated as affine scans
-        const double phil = electrode(p.phi_left, p.drive_left, field_time);
-        const double phir = electrode(p.phi_right, p.drive_right, field_time);
+        const double phil = s_electrode[0], phir = s_electrode[1];
         const int m = nx - 2;
         const double dx2 = p.dx * p.dx;
         __shared__ Affine s_wt[kPostThreads / 32 + 1];
         double* s_dp = reinterpret_cast<double*>(s_rhoi);  // the fixed-point density is converted already
-        // forward sweep: dp_i = r_i (d_i + dp_{i-1})
-        block_affine_scan(
-            m,
-            [&](int i) {
-                double d = s_rho[i + 1] * dx2 / p.eps;
-                if (i == 0) d += phil;
-                if (i == m - 1) d += phir;
-                const double r = s_c0[i];
-                return Affine{r, r * d};
-            },
-            [&](int i, double v) { s_dp[i] = v; }, s_wt);
-        // back substitution in reverse: z_t = a[m-1-t] z_{t-1} + dp[m-1-t]
-        double* s_phi = s_c0;  // coefficients no longer needed
-        block_affine_scan(
-            m, [&](int t) { return Affine{s_c1[m - 1 - t], s_dp[m - 1 - t]}; },
-            [&](int t, double v) { s_phi[m - t] = v; }, s_wt);
+        double* s_phi = s_rho;                             // its right-hand sides are used by then
+        // the forward sweep dp_i = r_i (d_i + dp_{i-1}), then the back
+        // substitution in reverse z_t = a[m-1-t] z_{t-1} + dp[m-1-t] (one copy of the scan's code)
+#pragma unroll 1
+        for (int back = 0; back < 2; ++back)
+            block_affine_scan(
+                m,
+                [&](int i) {
+                    if (back) return Affine{s_c1[m - 1 - i], s_dp[m - 1 - i]};
+                    double d = s_rho[i + 1] * dx2 / p.eps;
+                    if (i == 0) d += phil;
+                    if (i == m - 1) d += phir;
+                    const double r = s_c0[i];
+                    return Affine{r, r * d};
+                },
+                [&](int i, double v) {
+                    if (back) s_phi[m - i] = v;
+                    else s_dp[i] = v;
+                },
+                s_wt);
         if (tid == 0) {
             s_phi[0] = phil;
             s_phi[nx - 1] = phir;
         }
         __syncthreads();
+#pragma unroll 1
         for (int i = tid; i < nx; i += kPostThreads) {
             double e;
             if (i == 0) e = -(s_phi[1] - s_phi[0]) / p.dx;
@@ -1736,7 +2098,7 @@ struct Sim1D {
 
     // graphs of two steady steps (collision part pending), one per buffer parity
     cudaGraphExec_t pair_exec[2] = {nullptr, nullptr};
-    int blocks_cache = 0;
+    int blocks_cache = 0;  // SMs of the device
 
     void drop_graphs() {
         for (auto& g : pair_exec)
@@ -1942,6 +2304,8 @@ struct Sim1D {
             p.cand_count = dalloc<unsigned>(regions);
             p.cand_regions = (unsigned)regions;
             p.cand_per_region = (unsigned)per;
+        }
+        if (c.nmodels > 0) {
             MccModelDev* g = dalloc<MccModelDev>(c.nmodels);
             APIC_CUDA(cudaMemcpyAsync(g, p.model, c.nmodels * sizeof(MccModelDev), cudaMemcpyHostToDevice, stream));
             APIC_CUDA(cudaStreamSynchronize(stream));
@@ -2030,18 +2394,21 @@ struct Sim1D {
         return q;
     }
 
-    int grid_blocks() {
-        if (blocks_cache) return blocks_cache;
-        int sms = 148;
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+    // one resident wave of the pass kernel: per_sm CTAs per SM, no more than the tiles
+    int wave(int per_sm) {
+        if (!blocks_cache) {
+            int sms = 148;
+            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+            blocks_cache = sms;
+        }
         size_t tiles = 0;
         for (int s = 0; s < cfg.nspecies; ++s) tiles += (cfg.species[s].capacity + kTile - 1) / kTile;  // 8 warp chunks of c32 per tile
-        // one resident wave of the pass kernel: kMinBlocks (kMinBlocks32) CTAs per SM
-        blocks_cache = (int)std::max<size_t>(1, std::min<size_t>(tiles, (size_t)sms * (c32 ? kMinBlocks32 : kMinBlocks)));
-#ifdef APIC_C32_GRID_DIV
-        if (c32) blocks_cache = std::max(1, blocks_cache / APIC_C32_GRID_DIV);
-#endif
-        return blocks_cache;
+        return (int)std::max<size_t>(1, std::min<size_t>(tiles, (size_t)blocks_cache * per_sm));
+    }
+    int grid_blocks() {
+        if (c32) return wave(kMinBlocks32);
+        if (cfg.nmodels || p.bgk) return wave(kMinBlocks);
+        return wave(cfg.velocity_dimensions == 1 ? kPlainBlocks<1> : kPlainBlocks<3>);
     }
 
     // Optional per-kernel timing (CUDA events on the handle's stream).
@@ -2067,10 +2434,11 @@ struct Sim1D {
     template <int VDIM, bool DIR, bool F32>
     static void set_attributes() {
         const int smem = kMaxNx1D * 16;
-        APIC_CUDA(cudaFuncSetAttribute(k_pass1d<VDIM, DIR, F32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem));
-        APIC_CUDA(cudaFuncSetAttribute(k_pass1d<VDIM, DIR, F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       smem));
+        APIC_CUDA(cudaFuncSetAttribute(k_pass1d<VDIM, DIR, F32, kPassPlain>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        APIC_CUDA(cudaFuncSetAttribute(k_pass1d_mcc<VDIM, DIR, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        APIC_CUDA(cudaFuncSetAttribute(k_pass1d<VDIM, DIR, F32, kPassDiag>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
         const int psm = (int)post_smem_bytes(DIR ? kMaxNx1D : kMaxNx1DPeriodic, DIR);
         APIC_CUDA(cudaFuncSetAttribute(k_post1d<VDIM, DIR, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize, psm));
         APIC_CUDA(cudaFuncSetAttribute(k_moments1d<VDIM, DIR, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -2114,9 +2482,13 @@ struct Sim1D {
     template <int VDIM, bool DIR, bool F32>
     void launch_kernels(const Params1D& q, int blocks, size_t smem, size_t post_smem, unsigned post, EvPair& ev) {
         if (q.coll_acc || q.ledger || q.bgk)
-            k_pass1d<VDIM, DIR, F32, true><<<blocks, kThreads, smem, stream>>>(q);
+            k_pass1d<VDIM, DIR, F32, kPassDiag><<<blocks, kThreads, smem, stream>>>(q);
+        else if (cfg.nmodels && q.mode == (kModeSyncMcc | kModeKickDrift | kModeDeposit))
+            k_pass1d_mcc<VDIM, DIR, F32><<<wave(kMccBlocks), kMccThreads, smem, stream>>>(q);
+        else if (cfg.nmodels)
+            k_pass1d<VDIM, DIR, F32, kPassDiag><<<blocks, kThreads, smem, stream>>>(q);
         else
-            k_pass1d<VDIM, DIR, F32, false><<<blocks, kThreads, smem, stream>>>(q);
+            k_pass1d<VDIM, DIR, F32, kPassPlain><<<blocks, kThreads, smem, stream>>>(q);
         if (timing) cudaEventRecord(ev.b, stream);
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(1);

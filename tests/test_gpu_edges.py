@@ -99,3 +99,44 @@ def test_periodic_1d_solve(nx):
     ph[0] = ek[0] = 0.0
     assert rel_max(phi, np.fft.ifft(ph).real) < TOL
     assert rel_max(E, np.fft.ifft(ek).real) < TOL
+
+
+@pytest.mark.parametrize("mcc", [False, True])
+@pytest.mark.parametrize("count,leaving", [(1, 0.0), (1023, 0.3), (1025, 0.3), (4097, 0.9), (100_003, 0.6), (100_003, 0.98)])
+def test_1d_heavy_wall_losses(mcc, count, leaving):
+    """Survivors keep their order through tiles that lose some, most or nearly
+    all of their particles (and so read their next tile from many short ranges)."""
+    from apic import workloads as W
+    from common import load_device, load_oracle, oracle_config
+    wl = W.ccp_helium(particles_per_cell=1, cells=32, seed=2, table_rows=256)
+    if not mcc:
+        wl.models = []
+    rng = np.random.default_rng(count)
+    for s in wl.species:
+        s.weight *= 1e-6
+        s.capacity = 2 * count + 4096
+        s.x = rng.uniform(0.0, wl.length, count)
+        s.v, s.vy, s.vz = (s.thermal * rng.standard_normal(count) for _ in range(3))
+        go = rng.random(count) < leaving  # these cross the gap in one of the first three steps
+        s.v[go] = rng.choice([-1.0, 1.0], go.sum()) * wl.length / wl.dt / rng.integers(1, 4, go.sum())
+        if mcc:  # fast enough to leave, slow enough for the models' frequency bound: move them to the walls instead
+            s.v[go] = s.thermal * np.abs(rng.standard_normal(go.sum())) * -1.0
+            s.x[go] = np.abs(s.v[go]) * wl.dt * rng.uniform(0.2, 2.5, go.sum())
+    cfg, tabs = W.to_device_config(wl, seed=77)
+    dev = apic.Simulation1D(cfg, tabs)
+    load_device(dev, wl)
+    dev.initialize()
+    T = po.TableSet()
+    ora = po.Sim1D(oracle_config(wl, T), 1, 77)
+    load_oracle(ora, wl)
+    ora.initialize()
+    for steps in (1, 2, 3):
+        dev.step(steps)
+        ora.step(steps)
+        for k in range(2):
+            a, b = dev.particles(k), ora.particles(k)
+            assert len(a["x"]) == len(b["x"])
+            for c in ("x", "vh", "v", "vy", "vz"):
+                assert rel_max(a[c], b[c]) < 1e-11
+        for x, y in zip(dev.fields(), ora.fields()):
+            assert rel_max(x, y) < 1e-11

@@ -140,3 +140,50 @@ def test_1d_heavy_wall_losses(mcc, count, leaving):
                 assert rel_max(a[c], b[c]) < 1e-11
         for x, y in zip(dev.fields(), ora.fields()):
             assert rel_max(x, y) < 1e-11
+
+
+@pytest.mark.parametrize("n,axis", [((4, 3), 0), ((3, 4), 1), ((8, 34), 0), ((35, 16), 1), ((1024, 40), 0),
+                                    ((4, 4002), 0), ((4, 4003), 0), ((4100, 8), 1)])
+def test_mixed_solve_sizes(n, axis):
+    """Odd row counts (a pair with one row), one interior row, the longest
+    column kept in shared memory and longer ones."""
+    rng = np.random.default_rng(sum(n))
+    rho = rng.standard_normal((n[1], n[0]))
+    phi, E = apic.field_solve_mixed_2d(n, (2.0, 3.0), axis, 1.3, 0.7, -1.1, rho)
+    pr, Er = po.solve_mixed_2d(rho, n, (2.0, 3.0), axis, 1.3, 0.7, -1.1)
+    # the oracle's own column solve has a condition number of about (rows / pi)^2
+    rows = n[1] if axis == 0 else n[0]
+    tol = max(TOL, 2.2e-16 * (rows / np.pi) ** 2)
+    assert rel_max(phi, pr) < tol
+    assert rel_max(E, Er) < 10 * tol
+
+
+@pytest.mark.parametrize("n", [(3, 3), (5, 3), (3, 513), (513, 9), (3, 5, 9), (17, 3, 3), (33, 65, 17)])
+def test_dirichlet_solve_sizes(n):
+    """The discrete equation at every interior node: eps Laplacian(phi) = -rho."""
+    rng = np.random.default_rng(sum(n))
+    dims = len(n)
+    length = (2.0, 3.0, 1.5)[:dims]
+    shape = tuple(reversed(n))
+    rho = rng.standard_normal(shape)
+    sides = (0.3, -0.2, 1.0, 0.5) if dims == 2 else None
+    phi, E = apic.field_solve_dirichlet_nd(n, length, 1.3, rho, sides)
+    p = phi.reshape(shape)
+    lap, scale = 0.0, 0.0
+    inner = tuple(slice(1, -1) for _ in range(dims))
+    for a in range(dims):
+        ax, h = dims - 1 - a, length[a] / (n[a] - 1)
+        up = tuple(slice(2, None) if b == ax else slice(1, -1) for b in range(dims))
+        dn = tuple(slice(0, -2) if b == ax else slice(1, -1) for b in range(dims))
+        lap = lap + (p[up] - 2 * p[inner] + p[dn]) / h ** 2
+        scale += 4.0 / h ** 2
+        e = E[a].reshape(shape)
+        assert rel_max(e[inner], -(p[up] - p[dn]) / (2 * h)) < TOL
+    # the residual's rounding is that of the largest term of the Laplacian
+    assert np.max(np.abs(1.3 * lap + rho[inner])) < 1e-13 * scale * 1.3 * np.max(np.abs(p))
+    if dims == 2:
+        assert np.all(p[1:-1, 0] == 0.3) and np.all(p[1:-1, -1] == -0.2)
+        assert np.all(p[0, 1:-1] == 1.0) and np.all(p[-1, 1:-1] == 0.5)
+        assert p[0, 0] == 0.65 and p[-1, -1] == 0.15
+    else:
+        assert np.all(p[0] == 0.0) and np.all(p[:, :, -1] == 0.0)

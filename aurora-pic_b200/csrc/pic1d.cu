@@ -1835,7 +1835,9 @@ cudaError_t bounded_wait(cudaStream_t stream, double seconds) {
         if (e != cudaErrorNotReady) break;
         const double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > seconds) { e = cudaErrorNotReady; break; }
-        std::this_thread::sleep_for(std::chrono::microseconds(el < 0.01 ? 2 : 200));
+        // a sleep takes at least the timer slack (about 55 us): short waits poll
+        if (el > 0.002) std::this_thread::sleep_for(std::chrono::microseconds(el < 0.05 ? 20 : 200));
+        else std::this_thread::yield();
     }
     cudaEventDestroy(ev);
     return e;
@@ -2109,8 +2111,17 @@ struct Sim1D {
         if (stream) cudaStreamSynchronize(stream);
         drop_graphs();
         for (void* a : allocations) cudaFree(a);
+        if (host) cudaFreeHost(host);
         if (stream) cudaStreamDestroy(stream);
     }
+
+    // pinned read-back block: the run's state, then room for the three fields
+    struct HostBlock {
+        DevState state;
+        double* fields() { return reinterpret_cast<double*>(this + 1); }
+    };
+    static_assert(sizeof(HostBlock) % alignof(double) == 0, "the fields follow the state");
+    HostBlock* host = nullptr;
 
     void create(const apic_config1d& c) {
         cfg = c;
@@ -2311,9 +2322,10 @@ struct Sim1D {
             APIC_CUDA(cudaStreamSynchronize(stream));
             p.gmodel = g;
         }
-        p.E = dalloc<double>(c.nx);
-        p.rho = dalloc<double>(c.nx);
-        p.phi = dalloc<double>(c.nx);
+        p.rho = dalloc<double>(3 * c.nx);
+        p.phi = p.rho + c.nx;
+        p.E = p.phi + c.nx;
+        APIC_CUDA(cudaHostAlloc(&host, sizeof(HostBlock) + 3 * c.nx * sizeof(double), cudaHostAllocDefault));
         p.rho_acc = dalloc<unsigned long long>(c.nx);
         if (!dir) {
             std::vector<double> tw(2 * c.nx);
@@ -2773,12 +2785,12 @@ struct Sim1D {
     }
 
     int sync_status() {
+        // the run's state comes back with the wait itself, into pinned memory
+        APIC_CUDA(cudaMemcpyAsync(&host->state, st, sizeof(DevState), cudaMemcpyDeviceToHost, stream));
         const cudaError_t e = bounded_wait(stream, wait_limit_s);
         if (e == cudaErrorNotReady) throw Error(APIC_ERR_TIMEOUT, "device work did not complete in time");
         APIC_CUDA(e);
-        unsigned word = 0;
-        APIC_CUDA(cudaMemcpyAsync(&word, &st->error, sizeof word, cudaMemcpyDeviceToHost, stream));
-        APIC_CUDA(cudaStreamSynchronize(stream));
+        const unsigned word = host->state.error;
         if (word) {
             const int s = status_from_device(word);
             APIC_CUDA(cudaMemsetAsync(&st->error, 0, sizeof(unsigned), stream));
@@ -2790,10 +2802,7 @@ struct Sim1D {
 
     DevState read_state() {
         sync_status();
-        DevState h;
-        APIC_CUDA(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, stream));
-        APIC_CUDA(cudaStreamSynchronize(stream));
-        return h;
+        return host->state;
     }
 
     size_t count(int s) {
@@ -2978,12 +2987,14 @@ struct Sim1D {
     }
 
     void read_fields(double* rho, double* phi, double* E) {
+        // rho, phi and E are one block on the device: one copy, one wait
+        double* h = host->fields();
+        const size_t n = cfg.nx;
+        APIC_CUDA(cudaMemcpyAsync(h, p.rho, 3 * n * sizeof(double), cudaMemcpyDeviceToHost, stream));
         sync_status();
-        const size_t bytes = cfg.nx * sizeof(double);
-        if (rho) APIC_CUDA(cudaMemcpyAsync(rho, p.rho, bytes, cudaMemcpyDeviceToHost, stream));
-        if (phi) APIC_CUDA(cudaMemcpyAsync(phi, p.phi, bytes, cudaMemcpyDeviceToHost, stream));
-        if (E) APIC_CUDA(cudaMemcpyAsync(E, p.E, bytes, cudaMemcpyDeviceToHost, stream));
-        APIC_CUDA(cudaStreamSynchronize(stream));
+        if (rho) std::memcpy(rho, h, n * sizeof(double));
+        if (phi) std::memcpy(phi, h + n, n * sizeof(double));
+        if (E) std::memcpy(E, h + 2 * n, n * sizeof(double));
     }
 };
 

@@ -19,12 +19,15 @@
 // local.  Compiled with --fmad=false: particle arithmetic follows the
 // reference operation by operation.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstring>
 #include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "apic_common.cuh"
@@ -2735,6 +2738,110 @@ void ensure_solver_attributes() {
     g_attr_done[dev] = true;
 }
 
+// the interleaved field as planes
+template <int DIM>
+__global__ void k_split_field(const double* __restrict__ E, double* __restrict__ ex, double* __restrict__ ey,
+                              double* __restrict__ ez, size_t N) {
+    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < N; i += (size_t)gridDim.x * blockDim.x) {
+        if (DIM == 2) {
+            const double2 e = reinterpret_cast<const double2*>(E)[i];
+            ex[i] = e.x;
+            ey[i] = e.y;
+        } else {
+            const double4 e = reinterpret_cast<const double4*>(E)[i];
+            ex[i] = e.x;
+            ey[i] = e.y;
+            ez[i] = e.z;
+        }
+    }
+}
+
+// Device to pageable host copies of a few hundred megabytes: kWorkers threads
+// take 1 MB pieces in turn, each with two pinned buffers and a stream of its own, so
+// the transfers overlap the host copies and the page faults of fresh
+// destinations, which one thread would take one after another.  Small reads take the driver's
+// own path.  The buffers (16 MB pinned) belong to the run and are made at its
+// first large read.
+struct HostCopier {
+    static constexpr int kWorkers = 8;
+    static constexpr size_t kPiece = 1 << 20, kLarge = 16 << 20;
+    struct Job {
+        double* dst;
+        const double* src;
+        size_t bytes;
+    };
+    unsigned char* pinned = nullptr;
+    cudaStream_t streams[kWorkers] = {};
+
+    ~HostCopier() {
+        for (auto& s : streams)
+            if (s) cudaStreamDestroy(s);
+        if (pinned) cudaFreeHost(pinned);
+    }
+
+    // the sources must be complete: the workers' streams do not wait for `stream`
+    void run(const std::vector<Job>& jobs, cudaStream_t stream) {
+        size_t total = 0;
+        for (const Job& j : jobs) total += j.bytes;
+        if (total < kLarge) {
+            for (const Job& j : jobs) APIC_CUDA(cudaMemcpyAsync(j.dst, j.src, j.bytes, cudaMemcpyDeviceToHost, stream));
+            APIC_CUDA(cudaStreamSynchronize(stream));
+            return;
+        }
+        if (!pinned) APIC_CUDA(cudaHostAlloc(&pinned, 2 * kWorkers * kPiece, cudaHostAllocDefault));
+        for (auto& s : streams)
+            if (!s) APIC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+        struct Piece {
+            unsigned char* dst;
+            const unsigned char* src;
+            size_t bytes;
+        };
+        std::vector<Piece> pieces;
+        for (const Job& j : jobs)
+            for (size_t o = 0; o < j.bytes; o += kPiece)
+                pieces.push_back({reinterpret_cast<unsigned char*>(j.dst) + o,
+                                  reinterpret_cast<const unsigned char*>(j.src) + o, std::min(kPiece, j.bytes - o)});
+        int device = 0;
+        APIC_CUDA(cudaGetDevice(&device));
+        std::atomic<size_t> next{0};
+        std::atomic<int> failed{0};
+        auto work = [&](int t) {
+            unsigned char* buf[2] = {pinned + 2 * t * kPiece, pinned + (2 * t + 1) * kPiece};
+            cudaError_t e = cudaSetDevice(device);
+            const Piece* held = nullptr;  // copied into buf[which ^ 1], not yet handed over
+            int which = 0;
+            while (e == cudaSuccess) {
+                const size_t k = next.fetch_add(1);
+                const Piece* p = k < pieces.size() ? &pieces[k] : nullptr;
+                if (held) e = cudaStreamSynchronize(streams[t]);
+                if (e == cudaSuccess && p)
+                    e = cudaMemcpyAsync(buf[which], p->src, p->bytes, cudaMemcpyDeviceToHost, streams[t]);
+                if (e != cudaSuccess) break;
+                if (held) std::memcpy(held->dst, buf[which ^ 1], held->bytes);
+                held = p;
+                which ^= 1;
+                if (!p) break;
+            }
+            if (e != cudaSuccess) failed.store((int)e);
+        };
+        std::vector<std::thread> threads;
+        for (int t = 1; t < kWorkers; ++t) {
+            try {
+                threads.emplace_back(work, t);
+            } catch (const std::system_error&) {
+                break;  // fewer workers: those that run take every piece
+            }
+        }
+        work(0);
+        for (auto& t : threads) t.join();
+        // (a worker that failed leaves with its copy possibly in flight)
+        if (failed.load()) {
+            for (auto& s : streams) cudaStreamSynchronize(s);
+            APIC_CUDA((cudaError_t)failed.load());
+        }
+    }
+};
+
 struct SimND {
     apic_config_nd cfg{};
     std::string last_error;
@@ -3147,6 +3254,8 @@ struct SimND {
     // ---- walls: persistent solve scratch on the run's stream ----
     bool walls = false;
     WallSolver wall_solver;
+    double* wall_planes = nullptr;  // read_fields: Ex | Ey (| Ez)
+    HostCopier copier;
 
     void setup_walls(const apic_config_nd& c) {
         const int dims = c.dims;
@@ -3175,6 +3284,7 @@ struct SimND {
         wall_solver.alloc = [this](size_t bytes) -> void* { return dalloc<unsigned char>(bytes); };
         wall_solver.setup(dims, p.n, p.d, p.wall, p.eps, c.wall_potential);
         wall_solver.set_sides(solver.F.phi);
+        wall_planes = dalloc<double>(dims * N);
         APIC_CUDA(cudaStreamSynchronize(stream));
     }
 
@@ -3379,20 +3489,27 @@ struct SimND {
         for (int k = 0; k < 2 * cfg.dims; ++k) out[k] = h[k];
     }
 
+    // The components are separated on the device (a strided loop over the interleaved
+    // field on the host took longer than 48 steps of the 256^3 deck) into
+    // the work arrays of the solve, which are free between steps.
     void read_fields(double* rho, double* phi, double* E) {
-        sync();
         const size_t N = ncells;
-        if (rho) APIC_CUDA(cudaMemcpyAsync(rho, solver.F.rho, N * 8, cudaMemcpyDeviceToHost, stream));
-        if (phi) APIC_CUDA(cudaMemcpyAsync(phi, solver.F.phi, N * 8, cudaMemcpyDeviceToHost, stream));
+        std::vector<HostCopier::Job> jobs;
+        if (rho) jobs.push_back({rho, solver.F.rho, N * sizeof(double)});
+        if (phi) jobs.push_back({phi, solver.F.phi, N * sizeof(double)});
         if (E) {
-            const int st = cfg.dims == 2 ? 2 : 4;
-            std::vector<double> h(N * st);
-            APIC_CUDA(cudaMemcpyAsync(h.data(), solver.F.E, N * st * 8, cudaMemcpyDeviceToHost, stream));
-            APIC_CUDA(cudaStreamSynchronize(stream));
+            double* plane[3];
             for (int c = 0; c < cfg.dims; ++c)
-                for (size_t g = 0; g < N; ++g) E[c * N + g] = h[g * st + c];
+                plane[c] = walls ? wall_planes + c * N
+                                 : reinterpret_cast<double*>(c < 2 ? solver.F.A : solver.F.B) + (c & 1) * N;
+            const unsigned g = (unsigned)std::min<size_t>((N + 255) / 256, 4096);
+            if (cfg.dims == 2) k_split_field<2><<<g, 256, 0, stream>>>(solver.F.E, plane[0], plane[1], nullptr, N);
+            else k_split_field<3><<<g, 256, 0, stream>>>(solver.F.E, plane[0], plane[1], plane[2], N);
+            APIC_CUDA(cudaGetLastError());
+            for (int c = 0; c < cfg.dims; ++c) jobs.push_back({E + c * N, plane[c], N * sizeof(double)});
         }
-        APIC_CUDA(cudaStreamSynchronize(stream));
+        sync();
+        copier.run(jobs, stream);
     }
 
     void sample(apic_sample_nd* out) {

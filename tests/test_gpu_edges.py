@@ -187,3 +187,24 @@ def test_dirichlet_solve_sizes(n):
         assert p[0, 0] == 0.65 and p[-1, -1] == 0.15
     else:
         assert np.all(p[0] == 0.0) and np.all(p[:, :, -1] == 0.0)
+
+
+@pytest.mark.parametrize("n", [(64, 32), (1024, 1024), (64, 128, 128)])
+def test_fields_read_back(n):
+    """Small reads (one copy after another) and large ones (threads): every
+    component in its place."""
+    dims = len(n)
+    length = tuple(float(k) for k in n)
+    count = 20011
+    dev = apic.SimulationND(apic.config_nd(dims=dims, n=n, length=length, dt=0.1,
+                                           species=[(q, m, w, count) for q, m, w in SPECIES]))
+    for k in range(2):
+        pos, v = _particles(count, dims, length, 5 + k)
+        dev.load(k, pos, v)
+    dev.initialize()
+    for _ in range(2):
+        dev.step(1)
+        rho, phi, E = dev.fields()
+        p2, E2 = apic.field_solve_periodic_nd(dims, n, length, 1.0, rho)
+        assert rel_max(phi, p2) < TOL
+        assert rel_max(E, E2) < TOL

@@ -464,6 +464,288 @@ __global__ void __launch_bounds__(kThreads, 4) k_swarm_collide(Batch b) {
     }
 }
 
+// ---- fixed populations: many steps of a chunk in one launch -----------------------
+//
+// Without branching, electrons only meet in the step's sums, so a CTA runs
+// all steps of a launch on one chunk with the velocities and displacements
+// in shared memory: no state crosses memory between steps, and the collision loops
+// of one chunk overlap the streaming part of the other chunks on the SM.
+// Each step: the streaming part as in k_swarm_push, the candidates queued in shared
+// memory; then their collision loops, one per thread.  A step's sums go to the
+// run's totals of that step (integers and maxima: any order gives the same bits),
+// which k_swarm_reduce_steps folds into the run, step by step, at the end.
+// 12 runs of 100,000 electrons (FP32), per step: 63 us as three kernels, now 32.
+struct StepTotals {
+    unsigned long long vsum, esum, emax_bits, cand, nulls;
+    unsigned counts[kMaxChannels];
+    unsigned err, pad;
+};
+
+constexpr int kStepThreads = 128;
+static_assert(kStepThreads >= 96, "three warps add and reset a step's sums");
+constexpr int kStepBlocks = 4;  // per SM (5: 13.2 against 12.9 ms for 400 steps; 256 threads x 2: 19.2)
+constexpr size_t kStepsPerKernel = 128;  // bounds the totals (10 KB a run slot)
+template <class T>
+constexpr size_t steps_smem() { return kChunk * (6 * sizeof(T) + sizeof(uint16_t)); }
+
+// One candidate's collision loop and second half kick (finish_candidate without
+// births); v is the stored velocity, in and out.
+template <class T>
+struct ElectronSums {
+    unsigned long long vsum = 0, esum = 0, emax = 0;
+    unsigned err = 0;
+};
+
+template <class T>
+__device__ __forceinline__ void collide_electron(const MccModelDev& M, const MccModel32& M32, const RunCfg& R,
+                                                 uint32_t step, uint32_t i, T (&v)[3], ElectronSums<T>& t,
+                                                 unsigned* cand, unsigned* nulls, unsigned* counts) {
+    if constexpr (sizeof(T) == 4) {
+        const float hk = (float)R.half_kick;
+        v[0] += hk;
+        Philox32 rng(R.seed, i, step, 0u);
+        const uint32_t w0 = rng.next(), w1 = rng.next();
+        const uint64_t d0 = (uint64_t)w1 << 32 | w0;
+        const float dt = (float)R.dt;
+        const float u0 = ((float)(d0 >> 41) + 0.5f) * 1.1920928955078125e-7f;
+        const float first_wait = fminf(-__logf(u0) * M32.inv_max_frequency, dt * (1.0f - kFltEpsilon));
+        CollideResult32 r;
+        collide3f(
+            M32, v, dt, first_wait, rng, r, [&](float speed) { return frequency_bound_ok_far(M, (double)speed); },
+            [&](int ch, double) { atomicAdd(counts + ch, 1u); }, [](int, const float*, const float*) {});
+        t.err |= r.error;
+        v[0] += hk;
+        atomicAdd(cand, r.candidates);
+        if (r.nulls) atomicAdd(nulls, r.nulls);
+    } else {
+        double w[3] = {v[0] + R.half_kick, v[1], v[2]};
+        PhiloxDraws<true> rng(R.seed, i, step, 0u);
+        double u = uniform01(rng);
+        for (int guard = 0; !(u > 0.0) && guard < 64; ++guard) u = uniform01(rng);
+        const double first_wait = -log(u) / M.max_frequency;
+        CollideResult r;
+        collide3(M, w, R.dt, rng, r, [](int, const double*, const double*) {}, true, first_wait,
+                 [&](double speed) { return frequency_bound_ok_far(M, speed); });
+        t.err |= r.error;
+        v[0] = w[0] + R.half_kick;
+        v[1] = w[1];
+        v[2] = w[2];
+        atomicAdd(cand, r.candidates);
+        if (r.nulls) atomicAdd(nulls, r.nulls);
+        for (int ch = 0; ch < M.nch; ++ch)
+            if (r.channel[ch]) atomicAdd(counts + ch, r.channel[ch]);
+    }
+    const double s2 = sq3((double)v[0], (double)v[1], (double)v[2]);
+    if (s2 > R.s2_max) t.err |= kErrMaxEnergy;
+    t.emax = max(t.emax, (unsigned long long)__double_as_longlong(s2));
+    t.vsum += to_fixed((double)v[0], R.vscale);
+    t.esum += to_fixed(s2, R.escale);
+}
+
+template <class T>
+__global__ void __launch_bounds__(kStepThreads, kStepBlocks) k_swarm_steps(Batch b, uint32_t nsteps, StepTotals* totals) {
+    extern __shared__ __align__(16) unsigned char step_raw[];
+    T* sv = reinterpret_cast<T*>(step_raw);  // [3][kChunk] velocities, then displacements
+    T* sd = sv + 3 * kChunk;
+    uint16_t* queue = reinterpret_cast<uint16_t*>(sd + 3 * kChunk);
+    constexpr int kWarps = kStepThreads / 32;
+    __shared__ unsigned long long s_sum[2][kWarps][3];  // by step parity: v, energy, maximum
+    __shared__ unsigned s_tally[2][2 + kMaxChannels];   // candidates, nulls, channels
+    __shared__ unsigned s_ncand[2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t nch_total = *b.nchunks;
+    const MccModelDev& M = *b.model;
+    const MccModel32& M32 = *b.model32;
+    for (uint32_t c = blockIdx.x; c < nch_total; c += gridDim.x) {
+        const uint32_t slot = b.chunk_run[c];
+        const RunCfg& R = b.cfg[slot];
+        if (!b.st[slot].active) continue;  // uniform over the CTA
+        const uint32_t first = b.chunk_first[c];
+        const uint32_t cnt = min((uint32_t)kChunk, R.n - first);
+        const uint32_t step0 = b.st[slot].step;
+        const uint32_t steps = min(nsteps, R.steps - step0);
+        const bool samples = step0 + steps > R.burn_in;
+        const double half_kick = R.half_kick, dt = R.dt, s2_max = R.s2_max, vscale = R.vscale, escale = R.escale;
+        const uint64_t draw_min = R.cand_draw_min;
+        const bool no_candidates = R.no_candidates != 0;
+        const uint32_t key0 = (uint32_t)R.seed, key1 = (uint32_t)(R.seed >> 32);
+        const double v_safe2 = M.v_safe2;
+        for (uint32_t li = tid; li < cnt; li += kStepThreads)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                sv[a * kChunk + li] = arr<T>(R.v[a])[first + li];
+                if (samples) sd[a * kChunk + li] = arr<T>(R.d[a])[first + li];
+            }
+        if (tid < 2) s_ncand[tid] = 0u;
+        for (int i = tid; i < 2 * (2 + kMaxChannels); i += kStepThreads) (&s_tally[0][0])[i] = 0u;
+        __syncthreads();
+        for (uint32_t k = 0; k < steps; ++k) {
+            const uint32_t step = step0 + k;
+            const bool sampling = step >= R.burn_in;
+            const int par = k & 1;
+            ElectronSums<T> t;
+            // -- streaming part (k_swarm_push); every warp takes whole rows of the chunk --
+#pragma unroll 2
+            for (uint32_t row = warp * 32; row < cnt; row += kStepThreads) {
+                const uint32_t li = row + lane;
+                bool candidate = false;
+                if (li < cnt) {
+                    uint32_t o[4];
+                    philox4x32_10(0u, first + li, step, 0u, key0, key1, o);
+                    const uint64_t d0 = (uint64_t)o[1] << 32 | o[0];  // PhiloxStream's first draw
+                    double v[3];
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) v[a] = (double)sv[a * kChunk + li];
+                    v[0] += half_kick;
+                    const double pre = sq3(v[0], v[1], v[2]);
+                    t.emax = max(t.emax, (unsigned long long)__double_as_longlong(pre));
+                    if (pre > s2_max) t.err |= kErrMaxEnergyPre;
+                    if (sampling)
+#pragma unroll
+                        for (int a = 0; a < 3; ++a)
+                            sd[a * kChunk + li] = store_as<T>((double)sd[a * kChunk + li] + v[a] * dt);
+                    // first iteration of NullCollisionModel::collide, src/Collision.cpp:926-933
+                    if (!(pre <= v_safe2) && !frequency_bound_ok_far(M, sqrt(pre))) t.err |= kErrMajorant;
+                    if (d0 != 0ull) {
+                        candidate = !no_candidates && d0 >= draw_min;
+                    } else {  // open_unit_interval draws again
+                        PhiloxDraws<true> rng(R.seed, first + li, step, 0u);
+                        double u = 0.0;
+                        for (int guard = 0; !(u > 0.0) && guard < 64; ++guard) u = uniform01(rng);
+                        const double wait = -log(u) / M.max_frequency;
+                        candidate = isfinite(wait) && wait < dt;
+                    }
+                    if (!candidate) {  // second half kick, check, store, sums
+                        v[0] += half_kick;
+                        const double en = sq3(v[0], v[1], v[2]);
+                        t.emax = max(t.emax, (unsigned long long)__double_as_longlong(en));
+                        if (en > s2_max) t.err |= kErrMaxEnergy;
+                        const T v0 = store_as<T>(v[0]);
+                        sv[li] = v0;
+                        t.vsum += to_fixed((double)v0, vscale);
+                        t.esum += to_fixed(sizeof(T) == sizeof(double) ? en : sq3((double)v0, v[1], v[2]), escale);
+                    }
+                }
+                const unsigned bal = __ballot_sync(0xffffffffu, candidate);
+                if (bal) {
+                    unsigned q0 = 0;
+                    if (lane == 0) q0 = atomicAdd(&s_ncand[par], (unsigned)__popc(bal));
+                    q0 = __shfl_sync(0xffffffffu, q0, 0);
+                    if (candidate) queue[q0 + __popc(bal & ((1u << lane) - 1u))] = (uint16_t)li;
+                }
+            }
+            __syncthreads();
+            // -- collision loops of the candidates --
+            const unsigned nc = s_ncand[par];
+            for (unsigned q = tid; q < nc; q += kStepThreads) {
+                const uint32_t li = queue[q];
+                T v[3];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) v[a] = sv[a * kChunk + li];
+                collide_electron<T>(M, M32, R, step, first + li, v, t, &s_tally[par][0], &s_tally[par][1],
+                                    &s_tally[par][2]);
+#pragma unroll
+                for (int a = 0; a < 3; ++a) sv[a * kChunk + li] = v[a];
+            }
+            __syncwarp();
+            const unsigned long long vs = warp_sum_u64(t.vsum), es = warp_sum_u64(t.esum), em = warp_max_u64(t.emax);
+            if (lane == 0) {
+                s_sum[par][warp][0] = vs;
+                s_sum[par][warp][1] = es;
+                s_sum[par][warp][2] = em;
+            }
+            StepTotals* tot = totals + (size_t)slot * nsteps + k;
+            if (t.err) atomicOr(&tot->err, t.err);
+            __syncthreads();
+            // the step's sums to the run's totals; the parity buffers are not
+            // written again before every thread has passed the next step's barriers
+            if (tid < 3) {
+                unsigned long long x = s_sum[par][0][tid];
+#pragma unroll
+                for (int w = 1; w < kWarps; ++w) {
+                    const unsigned long long y = s_sum[par][w][tid];
+                    x = tid == 2 ? max(x, y) : x + y;
+                }
+                if (tid == 0) atomicAdd(&tot->vsum, x);
+                else if (tid == 1) atomicAdd(&tot->esum, x);
+                else atomicMax(&tot->emax_bits, x);
+            } else if (tid >= 32 && tid < 32 + 2 + kMaxChannels) {
+                const unsigned x = s_tally[par][tid - 32];
+                s_tally[par][tid - 32] = 0u;
+                if (x) {
+                    if (tid < 34) atomicAdd(tid == 32 ? &tot->cand : &tot->nulls, (unsigned long long)x);
+                    else atomicAdd(tot->counts + (tid - 34), x);
+                }
+            } else if (tid == 64) {
+                s_ncand[par] = 0u;
+            }
+        }
+        __syncthreads();
+        for (uint32_t li = tid; li < cnt; li += kStepThreads)
+#pragma unroll
+            for (int a = 0; a < 3; ++a) {
+                arr<T>(R.v[a])[first + li] = sv[a * kChunk + li];
+                if (samples) arr<T>(R.d[a])[first + li] = sd[a * kChunk + li];
+            }
+        __syncthreads();
+    }
+}
+
+// Folds the steps' totals into each run in step order, as k_swarm_reduce does
+// after every step, up to and with the first step that met an error; clears them.
+__global__ void __launch_bounds__(kThreads) k_swarm_reduce_steps(Batch b, uint32_t nsteps, StepTotals* totals) {
+    __shared__ unsigned s_done;
+    const int slot = blockIdx.x, tid = threadIdx.x;
+    const RunCfg& R = b.cfg[slot];
+    RunState& S = b.st[slot];
+    if (!S.active) return;  // (its chunks were skipped: the totals are still clear)
+    StepTotals* tot = totals + (size_t)slot * nsteps;
+    const uint32_t step0 = S.step;
+    const uint32_t steps = min(nsteps, R.steps - step0);
+    if (tid == 0) s_done = steps;
+    __syncthreads();
+    for (uint32_t k = tid; k < steps; k += kThreads)
+        if (tot[k].err) atomicMin(&s_done, k + 1);
+    __syncthreads();
+    const uint32_t done = s_done;
+    const uint32_t skip = R.burn_in > step0 ? min(R.burn_in - step0, done) : 0u;  // steps before the sampling starts
+    const double w = S.weight;
+    const size_t ns = R.steps - R.burn_in;
+    for (uint32_t k = skip + tid; k < done; k += kThreads) {
+        const size_t at = step0 + k - R.burn_in;
+        R.samples[at] = (double)(long long)tot[k].vsum / R.vscale / (double)R.n;
+        R.samples[ns + at] = 0.5 * kElectronMass * ((double)(long long)tot[k].esum / R.escale) / kEvToJ / (double)R.n;
+        R.samples[2 * ns + at] = log((double)R.n * w);
+    }
+    if (tid < kMaxChannels) {
+        if (tid < b.model->nch)
+            for (uint32_t k = skip; k < done; ++k) {
+                const unsigned n = tot[k].counts[tid];
+                S.counts[tid] += n;
+                S.wcoll[tid] += w * (double)n;
+                S.wcoll2[tid] += w * w * (double)n;
+            }
+    } else if (tid == 32) {
+        for (uint32_t k = skip; k < done; ++k) S.exposure += (double)R.n * w * R.dt;
+    } else if (tid == 64) {
+        for (uint32_t k = skip; k < done; ++k) {
+            S.candidates += tot[k].cand;
+            S.nulls += tot[k].nulls;
+        }
+    } else if (tid == 96) {
+        for (uint32_t k = 0; k < done; ++k)
+            S.max_ev = fmax(S.max_ev, 0.5 * kElectronMass * __longlong_as_double((long long)tot[k].emax_bits) / kEvToJ);
+    }
+    __syncthreads();
+    if (tid == 0) {
+        if (done) S.error |= tot[done - 1].err;
+        S.step = step0 + done;
+        if (S.step >= R.steps || S.error) S.active = 0;
+    }
+    __syncthreads();
+    for (uint32_t k = tid; k < steps; k += kThreads) tot[k] = StepTotals{};
+}
+
 // ---- branching: scan of survivors and secondaries per run ------------------------
 
 __global__ void __launch_bounds__(kThreads) k_swarm_branch_scan(Batch b) {
@@ -923,8 +1205,6 @@ struct Server {
         if (h_st_pinned) cudaFreeHost(h_st_pinned);
         if (graph_exec) cudaGraphExecDestroy(graph_exec);
         if (graph) cudaGraphDestroy(graph);
-        if (graph_exec_fixed) cudaGraphExecDestroy(graph_exec_fixed);
-        if (graph_fixed) cudaGraphDestroy(graph_fixed);
         for (void* a : allocations) cudaFree(a);
         if (stream) cudaStreamDestroy(stream);
     }
@@ -1002,6 +1282,11 @@ struct Server {
         d_chunk_first = arena.alloc<uint32_t>(max_chunks);
         d_nchunks = arena.alloc<uint32_t>(1);
         d_part = arena.alloc<ChunkPartial>(max_chunks);
+        d_totals = arena.alloc<StepTotals>((size_t)c.max_runs * kStepsPerKernel);
+        APIC_CUDA(cudaFuncSetAttribute(k_swarm_steps<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)steps_smem<float>()));
+        APIC_CUDA(cudaFuncSetAttribute(k_swarm_steps<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       (int)steps_smem<double>()));
         runs.resize(c.max_runs);
         h_st.resize(c.max_runs);
         int sms = 148;
@@ -1206,35 +1491,44 @@ struct Server {
     uint32_t nchunks_host_ = 0;
 
     template <class T>
-    void enqueue_step(const Batch& b, bool branching) {
+    void enqueue_step(const Batch& b) {
         k_swarm_push<T><<<push_grid, kThreads, 0, stream>>>(b);
         k_swarm_collide<T><<<push_grid, kThreads, 0, stream>>>(b);
-        if (branching) {
-            k_swarm_branch_scan<<<conf.max_runs, kThreads, 0, stream>>>(b);
-            k_swarm_branch_compact<T><<<push_grid, kThreads, 0, stream>>>(b);
-            k_swarm_branch_resample<T><<<push_grid, kThreads, 0, stream>>>(b);
-        }
+        k_swarm_branch_scan<<<conf.max_runs, kThreads, 0, stream>>>(b);
+        k_swarm_branch_compact<T><<<push_grid, kThreads, 0, stream>>>(b);
+        k_swarm_branch_resample<T><<<push_grid, kThreads, 0, stream>>>(b);
         k_swarm_reduce<<<conf.max_runs, kThreads, 0, stream>>>(b);
     }
 
-    // Two step graphs: with the branching kernels, for batches holding a
-    // branching run, and without them.
-    cudaGraph_t graph_fixed = nullptr;
-    cudaGraphExec_t graph_exec_fixed = nullptr;
-
-    cudaGraphExec_t ensure_graph(bool branching) {
-        cudaGraph_t& g = branching ? graph : graph_fixed;
-        cudaGraphExec_t& ge = branching ? graph_exec : graph_exec_fixed;
-        if (ge) return ge;
-        const Batch b = batch();
-        APIC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
-        for (size_t k = 0; k < conf.steps_per_launch; ++k) {
-            if (fp32) enqueue_step<float>(b, branching);
-            else enqueue_step<double>(b, branching);
+    // Batches holding a branching run: the launch's steps as one graph.
+    void launch_branching() {
+        if (!graph_exec) {
+            const Batch b = batch();
+            APIC_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
+            for (size_t k = 0; k < conf.steps_per_launch; ++k) {
+                if (fp32) enqueue_step<float>(b);
+                else enqueue_step<double>(b);
+            }
+            APIC_CUDA(cudaStreamEndCapture(stream, &graph));
+            APIC_CUDA(cudaGraphInstantiate(&graph_exec, graph, 0));
         }
-        APIC_CUDA(cudaStreamEndCapture(stream, &g));
-        APIC_CUDA(cudaGraphInstantiate(&ge, g, 0));
-        return ge;
+        APIC_CUDA(cudaGraphLaunch(graph_exec, stream));
+    }
+
+    // Batches of fixed populations: all steps of each chunk in one kernel.
+    StepTotals* d_totals = nullptr;
+    template <class T>
+    void launch_fixed() {
+        const Batch b = batch();
+        for (size_t left = conf.steps_per_launch; left;) {
+            const uint32_t n = (uint32_t)std::min<size_t>(left, kStepsPerKernel);
+            k_swarm_steps<T><<<std::min<uint32_t>(push_grid / 4 * kStepBlocks, std::max(nchunks_host_, 1u)),
+                               kStepThreads, steps_smem<T>(), stream>>>(b, n, d_totals);
+            k_swarm_reduce_steps<<<conf.max_runs, kThreads, 0, stream>>>(b, n, d_totals);
+            left -= n;
+            kernel_launches += 2;
+        }
+        APIC_CUDA(cudaGetLastError());
     }
 
     // Finishes a run whose device state says it stopped (steps done, converged
@@ -1446,8 +1740,10 @@ struct Server {
             bool branching = false;
             for (int s = 0; s < conf.max_runs; ++s)
                 branching = branching || (runs[s].used && runs[s].cfg.branching);
-            if (!timing) APIC_CUDA(cudaGraphLaunch(ensure_graph(branching), stream));
-            kernel_launches += conf.steps_per_launch * (timing || branching ? 6 : 3);
+            if (!timing && branching) launch_branching();
+            else if (!timing && fp32) launch_fixed<float>();
+            else if (!timing) launch_fixed<double>();
+            if (timing || branching) kernel_launches += conf.steps_per_launch * 6;
             ++launches;
             if (!h_st_pinned) APIC_CUDA(cudaMallocHost(&h_st_pinned, h_st.size() * sizeof(RunState)));
             copy_d2h(h_st_pinned, d_st, h_st.size() * sizeof(RunState));

@@ -208,3 +208,87 @@ def test_fields_read_back(n):
         p2, E2 = apic.field_solve_periodic_nd(dims, n, length, 1.0, rho)
         assert rel_max(phi, p2) < TOL
         assert rel_max(E, E2) < TOL
+
+
+@pytest.mark.parametrize("precision", [apic.FP64, apic.FP32])
+@pytest.mark.parametrize("particles,steps_per_launch", [(1, 7), (1023, 1), (1025, 60), (2500, 129), (2500, 300)])
+def test_fixed_swarm_alone_and_beside_a_branching_run(precision, particles, steps_per_launch):
+    """Alone, a fixed population's steps run inside one kernel; beside a branching
+    run, step by step.  Both give the same bits."""
+    from apic import workloads as W
+    spec = W.swarm_c5(particles=particles, steps=260, burn_in_steps=100, seed=7)
+    branch = W.swarm_c5(particles=500, steps=260, burn_in_steps=100, seed=8, branching=True)
+    _, gas, keep = W.to_device_swarm(spec, precision=precision)
+    got = []
+    for beside in (False, True):
+        srv = apic.SwarmServer(gas, 64 << 20, max_runs=4, precision=precision, steps_per_launch=steps_per_launch)
+        rid = srv.submit(W.swarm_request(spec, 300.0, seed=5))
+        if beside:
+            srv.submit(W.swarm_request(branch, 50.0, seed=6))
+        r = None
+        while r is None:
+            srv.advance()
+            r = srv.poll(rid)
+        got.append([getattr(r, k) for k in ("status", "steps_done", "mean_velocity_x", "mean_energy_ev",
+                                            "diffusion_longitudinal", "diffusion_transverse", "max_observed_energy_ev",
+                                            "ionization_rate", "net_rate", "candidates", "null_collisions")]
+                   + list(r.channel_collisions) + list(r.channel_rate) + list(r.channel_rate_se))
+        srv.close()
+    assert got[0][0] == 0 and got[0][1] == 260
+    assert got[0] == got[1]
+
+
+def _plasma3d_run(n, count, pos, v, split, B=(0.005, 0.1, 0.2), steps=1, sort=2):
+    """One electron species (tiled push), or the same particles as `split` species of
+    fewer than two a cell each (the untiled push)."""
+    length = tuple(float(k) for k in n)
+    parts = np.array_split(np.arange(count), split)
+    dev = apic.SimulationND(apic.config_nd(dims=3, n=n, length=length, dt=0.2, magnetic_field=B, precision=apic.FP32,
+                                           sort_interval=sort, species=[(-1.0, 1.0, 0.01, len(i)) for i in parts]))
+    for k, i in enumerate(parts):
+        dev.load(k, pos[:, i], v[:, i])
+    dev.initialize()
+    dev.step(steps)
+    out = [dev.particles(k) for k in range(split)]
+    return [np.concatenate([o[c] for o in out], axis=1) for c in range(3)], dev.fields()[0]
+
+
+@pytest.mark.parametrize("steps", [1, 5])
+@pytest.mark.parametrize("n,ppc,spread", [((8, 8, 8), 4.1, 1.0), ((16, 8, 32), 7.3, 1.0), ((32, 16, 8), 5.9, 4.0),
+                                          ((8, 16, 8), 6.0, 30.0)])
+def test_tiled_push_gives_the_untiled_bits(n, ppc, spread, steps):
+    """Gather, push and deposit through a tile's shared memory against the kernels
+    without it, from thermal particles to ones that cross several tiles a step."""
+    rng = np.random.default_rng(int(10 * ppc))
+    count = int(ppc * np.prod(n)) | 1
+    pos = np.stack([rng.uniform(0.0, k, count) for k in n])
+    v = spread * rng.standard_normal((3, count))
+    (pa, va, ha), ra = _plasma3d_run(n, count, pos, v, 1, steps=steps)
+    (pb, vb, hb), rb = _plasma3d_run(n, count, pos, v, 4, steps=steps)
+    # both start from the same positions; the field differs by the rounding of the
+    # density sum (1 against 4 accumulators), which seldom moves its float; five steps
+    # sort twice more (ranks within tiles)
+    assert np.mean(pa == pb) > (0.999 if steps == 1 else 0.99) and np.mean(ha == hb) > (0.999 if steps == 1 else 0.99)
+    assert rel_max(ha, hb) < 1e-6 * steps
+    assert rel_max(ra, rb) < 1e-6 * steps
+
+
+def test_tiled_push_with_crowded_nodes():
+    """More weight on a node than one 32-bit word of a tile's box holds (and several work items
+    of one tile): the charge stays exact."""
+    n, count = (16, 8, 8), 40000
+    rng = np.random.default_rng(3)
+    pos = np.stack([rng.uniform(0.0, k, count) for k in n])
+    crowd = rng.random(count) < 0.8
+    pos[:, crowd] = np.array([[5.25], [3.5], [2.125]])
+    (px, _, _), rho = _plasma3d_run(n, count, pos, np.zeros((3, count)), 1, steps=2, sort=1)
+    i = np.floor(px).astype(int)
+    f = px - i
+    want = np.zeros(int(np.prod(n)))
+    for c in range(8):
+        o = np.array([[c & 1], [c >> 1 & 1], [c >> 2]])
+        g = (i + o) % np.array(n)[:, None]
+        w = np.prod(np.where(o == 1, f, 1.0 - f), axis=0)
+        want += np.bincount((g[2] * n[1] + g[1]) * n[0] + g[0], -0.01 * w, want.size)
+    # weights are multiples of 2^-23, offsets 24-bit floats
+    assert rel_max(rho, want) < 1e-6

@@ -904,65 +904,76 @@ __global__ void __launch_bounds__(kThreads) k_push32_step(ParamsND p, SpeciesND 
 // positions).  A run that ends inside the thread is committed with one 64-bit
 // atomic per node; each lane's last run joins a warp-segmented sum over the
 // lanes holding the same cell, whose last lane commits it.
+// One buffer of the FP32 state, by kernel argument (an index into the species'
+// arrays costs every access its pointer's load).
+struct State32 {
+    unsigned* cell;
+    float* off[3];
+    float* vel[3];
+};
+
 // 2D: the CTA's deposit into a box of nodes in shared memory (kDBoxX cells
 // along x from x0 and the cell rows y0 .. y0 + 2 around the CTA's middle
 // particle), flushed with one 64-bit global atomic per touched node: a
 // particle that left its sorted neighbours then adds into shared memory
 // instead of committing its own global atomics (which, on the few nodes a CTA
-// touches, serialise in L2).  Each node's weight sum is kept as two 32-bit
-// halves (native shared atomics; the low half adds at most 2^16 per commit and
-// the high half 2^14, so neither overflows for the CTA's particles) and
-// reassembled exactly.  Commits outside the box go to global memory as before.
+// touches, serialise in L2).  Each node's weight sum is one 32-bit word (native
+// shared atomics); an add that wraps it carries 2^32 into the global sum at once, so
+// the sums are exact.  Commits outside the box go to global memory as before.
+// (512^2, 2 x 16.8 M particles, per step: 368 us with two 16-bit halves and the box's place
+// broadcast by one thread, 336 now.)
 // (In 3D the box around a CTA's 64 cells needs 1552 nodes; zeroing and
 // flushing them and the kernel's extra registers cost more than the atomics
 // saved, so 3D commits straight to global memory.)
 constexpr int kDBoxX = 48;
 constexpr int kDBoxNodes = (kDBoxX + 1) * 4;
 struct DepositBox {
-    unsigned* lo;
-    unsigned* hi;
+    unsigned* sum;
     int x0, y0;
 };
 
 template <int DIM, bool BORIS, int ITEMS, bool PROF>
-__device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, int buf, unsigned long long* acc,
-                                         const DepositBox& box) {
+__device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, const State32& A,
+                                         unsigned long long* acc, const DepositBox& box) {
     constexpr int NN = DIM == 2 ? 4 : 8;  // nodes of a cell
     const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * ITEMS;
     const int lane = threadIdx.x & 31;
-    if ((blockIdx.x * kThreads + (threadIdx.x & ~31u)) * ITEMS >= S.n) return;  // whole warp past the end
+    if ((blockIdx.x * kThreads + (threadIdx.x & ~31u)) * ITEMS >= S.n) {  // whole warp past the end
+        if (DIM == 2) __syncthreads();
+        return;
+    }
     const int nx = p.n[0], ny = p.n[1], nz = DIM == 3 ? p.n[2] : 1;
     unsigned cl[ITEMS];
     float fo[ITEMS][3], vv[ITEMS][3];
     const bool full = first + ITEMS <= S.n;
     if (full) {
         if (ITEMS == 4) {
-            const uint4 c = __ldcs(reinterpret_cast<const uint4*>(S.cell[buf] + first));
+            const uint4 c = __ldcs(reinterpret_cast<const uint4*>(A.cell + first));
             cl[0] = c.x; cl[1] = c.y; cl[2 % ITEMS] = c.z; cl[3 % ITEMS] = c.w;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM) {
-                    const float4 f = __ldcs(reinterpret_cast<const float4*>(S.off[buf][a] + first));
+                    const float4 f = __ldcs(reinterpret_cast<const float4*>(A.off[a] + first));
                     fo[0][a] = f.x; fo[1][a] = f.y; fo[2 % ITEMS][a] = f.z; fo[3 % ITEMS][a] = f.w;
                 } else {
 #pragma unroll
                     for (int k = 0; k < ITEMS; ++k) fo[k][a] = 0.0f;
                 }
-                const float4 v = __ldcs(reinterpret_cast<const float4*>(S.vel[buf][a] + first));
+                const float4 v = __ldcs(reinterpret_cast<const float4*>(A.vel[a] + first));
                 vv[0][a] = v.x; vv[1][a] = v.y; vv[2 % ITEMS][a] = v.z; vv[3 % ITEMS][a] = v.w;
             }
         } else {
-            const uint2 c = __ldcs(reinterpret_cast<const uint2*>(S.cell[buf] + first));
+            const uint2 c = __ldcs(reinterpret_cast<const uint2*>(A.cell + first));
             cl[0] = c.x; cl[1 % ITEMS] = c.y;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM) {
-                    const float2 f = __ldcs(reinterpret_cast<const float2*>(S.off[buf][a] + first));
+                    const float2 f = __ldcs(reinterpret_cast<const float2*>(A.off[a] + first));
                     fo[0][a] = f.x; fo[1 % ITEMS][a] = f.y;
                 } else {
                     fo[0][a] = 0.0f; fo[1 % ITEMS][a] = 0.0f;
                 }
-                const float2 v = __ldcs(reinterpret_cast<const float2*>(S.vel[buf][a] + first));
+                const float2 v = __ldcs(reinterpret_cast<const float2*>(A.vel[a] + first));
                 vv[0][a] = v.x; vv[1 % ITEMS][a] = v.y;
             }
         }
@@ -971,14 +982,16 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         for (int k = 0; k < ITEMS; ++k) {
             const unsigned i = first + k;
             const bool ok = i < S.n;
-            cl[k] = ok ? S.cell[buf][i] : 0u;
+            cl[k] = ok ? A.cell[i] : 0u;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                fo[k][a] = (ok && a < DIM) ? S.off[buf][a][i] : 0.0f;
-                vv[k][a] = ok ? S.vel[buf][a][i] : 0.0f;
+                fo[k][a] = (ok && a < DIM) ? A.off[a][i] : 0.0f;
+                vv[k][a] = ok ? A.vel[a][i] : 0.0f;
             }
         }
     }
+    // 2D: the box is clear and its place read in every thread; the state's loads are under way
+    if (DIM == 2) __syncthreads();
     const unsigned kNoCell = 0xFFFFFFFFu;
     // 3D: the field lines of each later new cell in the thread's run are
     // prefetched into L1 before the first push: a cell change inside the run
@@ -1013,13 +1026,15 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
             const int bx = (ix - box.x0) & (nx - 1), by = (iy - box.y0) & (ny - 1);
             if (bx < kDBoxX && by < 3) {
                 const int b = by * (kDBoxX + 1) + bx;
+                unsigned old[NN], high = 0u;
 #pragma unroll
-                for (int j = 0; j < NN; ++j) {
-                    if (!w[j]) continue;
-                    const int q = b + (j & 1) + ((j >> 1) & 1) * (kDBoxX + 1);
-                    atomicAdd(box.lo + q, w[j] & 0xFFFFu);
-                    atomicAdd(box.hi + q, w[j] >> 16);
-                }
+                for (int j = 0; j < NN; ++j) old[j] = atomicAdd(box.sum + b + (j & 1) + (j >> 1) * (kDBoxX + 1), w[j]);
+#pragma unroll
+                for (int j = 0; j < NN; ++j) high |= old[j];
+                if (high >> 31)  // an add (at most 2^28) can only wrap a word that is past its half
+                    for (int j = 0; j < NN; ++j)
+                        if (old[j] + w[j] < old[j])
+                            atomicAdd(acc + (size_t)((iy + (j >> 1)) & (ny - 1)) * nx + ((ix + (j & 1)) & (nx - 1)), 1ull << 32);
                 return;
             }
         }
@@ -1101,31 +1116,35 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
 #pragma unroll
             for (int j = 0; j < NN; ++j) racc[j] = 0u;
         }
-        const float ux[2] = {1.0f - f[0], f[0]}, uy[2] = {1.0f - f[1], f[1]};
+        // (units of 2^-23 to nearest even: adding 2^23 leaves the integer in the low
+        // bits of the float; the scale, a power of two, is exact on any factor)
+        const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale}, uy[2] = {1.0f - f[1], f[1]};
         const float uz[2] = {DIM == 3 ? 1.0f - f[2] : 1.0f, DIM == 3 ? f[2] : 0.0f};
 #pragma unroll
-        for (int j = 0; j < NN; ++j)
-            racc[j] += (unsigned)__float2int_rn(ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1] * kWeightScale);
+        for (int j = 0; j < NN; ++j) {
+            const float w = DIM == 3 ? ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1] : ux[j & 1] * uy[(j >> 1) & 1];
+            racc[j] += __float_as_uint(w + kWeightScale) - 0x4B000000u;
+        }
     }
     // the state back, in place
     if (full) {
         if (ITEMS == 4) {
-            __stcs(reinterpret_cast<uint4*>(S.cell[buf] + first), make_uint4(cl[0], cl[1], cl[2 % ITEMS], cl[3 % ITEMS]));
+            __stcs(reinterpret_cast<uint4*>(A.cell + first), make_uint4(cl[0], cl[1], cl[2 % ITEMS], cl[3 % ITEMS]));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM)
-                    __stcs(reinterpret_cast<float4*>(S.off[buf][a] + first),
+                    __stcs(reinterpret_cast<float4*>(A.off[a] + first),
                            make_float4(fo[0][a], fo[1][a], fo[2 % ITEMS][a], fo[3 % ITEMS][a]));
-                __stcs(reinterpret_cast<float4*>(S.vel[buf][a] + first),
+                __stcs(reinterpret_cast<float4*>(A.vel[a] + first),
                        make_float4(vv[0][a], vv[1][a], vv[2 % ITEMS][a], vv[3 % ITEMS][a]));
             }
         } else {
-            __stcs(reinterpret_cast<uint2*>(S.cell[buf] + first), make_uint2(cl[0], cl[1 % ITEMS]));
+            __stcs(reinterpret_cast<uint2*>(A.cell + first), make_uint2(cl[0], cl[1 % ITEMS]));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM)
-                    __stcs(reinterpret_cast<float2*>(S.off[buf][a] + first), make_float2(fo[0][a], fo[1 % ITEMS][a]));
-                __stcs(reinterpret_cast<float2*>(S.vel[buf][a] + first), make_float2(vv[0][a], vv[1 % ITEMS][a]));
+                    __stcs(reinterpret_cast<float2*>(A.off[a] + first), make_float2(fo[0][a], fo[1 % ITEMS][a]));
+                __stcs(reinterpret_cast<float2*>(A.vel[a] + first), make_float2(vv[0][a], vv[1 % ITEMS][a]));
             }
         }
     } else {
@@ -1133,11 +1152,11 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         for (int k = 0; k < ITEMS; ++k) {
             const unsigned i = first + k;
             if (i >= S.n) continue;
-            S.cell[buf][i] = cl[k];
+            A.cell[i] = cl[k];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                if (a < DIM) S.off[buf][a][i] = fo[k][a];
-                S.vel[buf][a][i] = vv[k][a];
+                if (a < DIM) A.off[a][i] = fo[k][a];
+                A.vel[a][i] = vv[k][a];
             }
         }
     }
@@ -1167,31 +1186,28 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
 }
 
 template <int DIM, bool BORIS, int ITEMS, bool PROF>
-__global__ void __launch_bounds__(kThreads) k_push32_run(ParamsND p, SpeciesND S, int buf, unsigned long long* acc) {
+__global__ void __launch_bounds__(kThreads, 4) k_push32_run(ParamsND p, SpeciesND S, State32 A,
+                                                         unsigned long long* acc) {
     if constexpr (DIM == 2) {
-        __shared__ unsigned s_lo[kDBoxNodes], s_hi[kDBoxNodes];
-        __shared__ int s_anchor[2];
+        __shared__ unsigned s_sum[kDBoxNodes];
         const int nx = p.n[0], ny = p.n[1];
-        if (threadIdx.x == 0) {  // the box around the CTA's middle particle, before the push
-            const unsigned mid = min(blockIdx.x * kThreads * ITEMS + (unsigned)(kThreads * ITEMS / 2), S.n - 1u);
-            int ix, iy, iz;
-            unpack_cell(S.cell[buf][mid], ix, iy, iz);
-            s_anchor[0] = (ix - kDBoxX / 2) & (nx - 1);
-            s_anchor[1] = (iy - 1) & (ny - 1);
-        }
-        for (int q = threadIdx.x; q < kDBoxNodes; q += kThreads) { s_lo[q] = 0u; s_hi[q] = 0u; }
-        __syncthreads();
-        const DepositBox box{s_lo, s_hi, s_anchor[0], s_anchor[1]};
-        push_run<DIM, BORIS, ITEMS, PROF>(p, S, buf, acc, box);
+        // the box around the CTA's middle particle, read by every thread before the
+        // barrier in push_run (no particle is stored before it)
+        const unsigned mid = min(blockIdx.x * kThreads * ITEMS + (unsigned)(kThreads * ITEMS / 2), S.n - 1u);
+        int ix, iy, iz;
+        unpack_cell(A.cell[mid], ix, iy, iz);
+        for (int q = threadIdx.x; q < kDBoxNodes; q += kThreads) s_sum[q] = 0u;
+        const DepositBox box{s_sum, (ix - kDBoxX / 2) & (nx - 1), (iy - 1) & (ny - 1)};
+        push_run<DIM, BORIS, ITEMS, PROF>(p, S, A, acc, box);
         __syncthreads();
         for (int q = threadIdx.x; q < kDBoxNodes; q += kThreads) {
-            const unsigned long long v = ((unsigned long long)s_hi[q] << 16) + s_lo[q];
+            const unsigned long long v = s_sum[q];
             if (!v) continue;
             const int qx = q % (kDBoxX + 1), qy = q / (kDBoxX + 1);
             atomicAdd(acc + (size_t)((box.y0 + qy) & (ny - 1)) * nx + ((box.x0 + qx) & (nx - 1)), v);
         }
     } else {
-        push_run<DIM, BORIS, ITEMS, PROF>(p, S, buf, acc, DepositBox{nullptr, nullptr, 0, 0});
+        push_run<DIM, BORIS, ITEMS, PROF>(p, S, A, acc, DepositBox{nullptr, 0, 0});
     }
 }
 
@@ -1228,14 +1244,6 @@ template <int MARGIN>
 constexpr int kBoxNodes = kBoxSide<MARGIN> * kBoxSide<MARGIN> * kBoxSide<MARGIN>;
 template <int MARGIN>
 constexpr size_t tile32_smem() { return kBoxNodes<MARGIN> * (sizeof(float4) + sizeof(unsigned)); }
-
-// One buffer of the FP32 state, by kernel argument (an index into the species'
-// arrays costs every access its pointer's load).
-struct State32 {
-    unsigned* cell;
-    float* off[3];
-    float* vel[3];
-};
 
 // G consecutive 32-bit values as one vector (2 or 4, aligned), streamed
 template <int G, class V>
@@ -3430,6 +3438,12 @@ struct SimND {
         tiles_ready[s] = false;
     }
 
+    static State32 state32(const SpeciesND& S, int b) {
+        State32 A{S.cell[b], {}, {}};
+        for (int a = 0; a < 3; ++a) { A.off[a] = S.off[b][a]; A.vel[a] = S.vel[b][a]; }
+        return A;
+    }
+
     template <int DIM, bool BORIS>
     void launch_step32(int items, const SpeciesND& S, int b, int s) {
         const unsigned g = (unsigned)((S.n + (unsigned)items * kThreads - 1) / ((unsigned)items * kThreads));
@@ -3445,8 +3459,8 @@ struct SimND {
         }
         switch (items) {
             case 1: k_push32_step<DIM, BORIS, 1, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
-            case 2: k_push32_run<DIM, BORIS, 2, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
-            case 4: k_push32_run<DIM, BORIS, 4, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
+            case 2: k_push32_run<DIM, BORIS, 2, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), acc); break;
+            case 4: k_push32_run<DIM, BORIS, 4, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), acc); break;
             default: k_push32_step<DIM, BORIS, 8, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
         }
     }
@@ -3459,8 +3473,7 @@ struct SimND {
         const int b = buf[s];
         if (fp32 && MODE == kPushStep && S.tiled) {
             const unsigned g = ntiles + tile_extra_max(s);
-            State32 A{S.cell[b], {}, {}};
-            for (int a = 0; a < 3; ++a) { A.off[a] = S.off[b][a]; A.vel[a] = S.vel[b][a]; }
+            const State32 A = state32(S, b);
             // one cell around the tile when few particles leave it between sorts, else two
             // (a thermal electron moves about 0.1 cell a step, a heavier species at the same
             // temperature less; 256^3, electrons sorted every 3 steps: one 4.6, two 4.8 ms)

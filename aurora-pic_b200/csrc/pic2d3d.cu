@@ -2121,45 +2121,47 @@ __global__ void __launch_bounds__(kFftThreads) k_fft(FieldsND F, FftPass f) {
     }
 }
 
-// ---- 256-point lines: a four-step FFT in registers ---------------------------------
+// ---- lines of 32 .. 256 points: a four-step FFT in registers -----------------------
 //
-// Lines of 256 = 16 x 16 points, eight lines per CTA and 16 threads per line.
-// Thread slot s of a line holds the points s + 16 j (j < 16) in registers:
-// a 16-point DFT over j, the twiddles W256^(s k1), one exchange through shared
-// memory (thread s then holds column k1 = s), a second 16-point DFT, and the
-// thread holds the transform at s + 16 k2, the same positions it loaded, so a
-// pass reads and writes each element once and in place.  Lanes run along the
-// line on the x pass (16 consecutive points per half warp) and across the
+// Lines of R1 x R2 points (R1 >= R2, both powers of two), eight lines per CTA
+// and R2 threads per line.  Thread slot s of a line holds the points s + R2 j
+// (j < R1) in registers: an R1-point DFT over j, the twiddles w^(s k1), one exchange
+// through shared memory (thread s then holds the rows k1 = s + R2 q), R2-point
+// DFTs, and the thread holds the transform at s + R2 j again, the same positions
+// it loaded, so a pass reads and writes each element once and in place.  Lanes run
+// along the line on the x pass (R2 consecutive points) and across the
 // tile's lines on the strided y / z passes (8 consecutive lines, 128 B), so
-// every global access moves whole 128-256 B segments; the registers hold the
-// loads in flight (16 or 32 per thread) instead of a shared-memory tile.
-constexpr int kF256Lines = 8;
-constexpr int kF256Threads = kF256Lines * 16;
+// global accesses move whole segments; the registers hold the
+// loads in flight (R1 or 2 R1 per thread) instead of a shared-memory tile.
+// Against the shared-memory tiles of k_fft: 256^3 solve 2.77 -> 1.15 ms; 64^3
+// 78 -> 39 us, 256 x 128 (few lines) 31.7 -> 29.8 us.
+constexpr int kRegLines = 8;
 
-template <bool XP>
-__device__ __forceinline__ void f256_map(int tid, int& l, int& s) {
-    if (XP) { s = tid & 15; l = tid >> 4; }
-    else { l = tid & (kF256Lines - 1); s = tid >> 3; }
+template <int R2, bool XP>
+__device__ __forceinline__ void reg_map(int tid, int& l, int& s) {
+    if (XP) { s = tid & (R2 - 1); l = tid / R2; }
+    else { l = tid & (kRegLines - 1); s = tid / kRegLines; }
 }
 
 // exchange slot of (line l, row r, column c): written by slot c as row r,
-// read by slot r as column c; conflict-free for both lane layouts
-template <bool XP>
-__device__ __forceinline__ int f256_xi(int l, int r, int c) {
-    return XP ? (l * 16 + r) * 17 + c : (r * 16 + c) * kF256Lines + l;
+// read by column; spread over the banks for both lane layouts
+template <int R1, int R2, bool XP>
+__device__ __forceinline__ int reg_xi(int l, int r, int c) {
+    return XP ? (l * R1 + r) * (R2 + 1) + c : (r * R2 + c) * kRegLines + l;
 }
-template <bool XP>
-constexpr int f256_xsize() { return XP ? kF256Lines * 16 * 17 : kF256Lines * 256; }
+template <int R1, int R2, bool XP>
+constexpr int reg_xsize() { return XP ? kRegLines * R1 * (R2 + 1) : kRegLines * R1 * R2; }
 
-// forward (inv = false) or inverse transforms of NA lines held as a[k][16]
-template <bool XP, int NA>
-__device__ __forceinline__ void fft256(Cplx (&a)[NA][16], Cplx* xb, const Cplx* tws, int l, int s, bool inv) {
+// forward (inv = false) or inverse transforms of NA lines held as a[k][R1]
+template <int R1, int R2, bool XP, int NA>
+__device__ __forceinline__ void fft_reg(Cplx (&a)[NA][R1], Cplx* xb, const Cplx* tws, int l, int s, bool inv) {
+    constexpr int N = R1 * R2, Q = R1 / R2;
 #pragma unroll
     for (int k = 0; k < NA; ++k) {
-        dft_small<16>(a[k], inv);
+        dft_small<R1>(a[k], inv);
 #pragma unroll
-        for (int k1 = 1; k1 < 16; ++k1) {
-            Cplx w = tws[(s * k1) & 255];
+        for (int k1 = 1; k1 < R1; ++k1) {
+            Cplx w = tws[(s * k1) & (N - 1)];
             if (inv) w.im = -w.im;
             const Cplx x = a[k][k1];
             a[k][k1] = {x.re * w.re - x.im * w.im, x.re * w.im + x.im * w.re};
@@ -2169,74 +2171,78 @@ __device__ __forceinline__ void fft256(Cplx (&a)[NA][16], Cplx* xb, const Cplx* 
 #pragma unroll
     for (int k = 0; k < NA; ++k)
 #pragma unroll
-        for (int k1 = 0; k1 < 16; ++k1) xb[k * f256_xsize<XP>() + f256_xi<XP>(l, k1, s)] = a[k][k1];
+        for (int k1 = 0; k1 < R1; ++k1) xb[k * reg_xsize<R1, R2, XP>() + reg_xi<R1, R2, XP>(l, k1, s)] = a[k][k1];
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < NA; ++k) {
+    for (int k = 0; k < NA; ++k)
 #pragma unroll
-        for (int t = 0; t < 16; ++t) a[k][t] = xb[k * f256_xsize<XP>() + f256_xi<XP>(l, s, t)];
-        dft_small<16>(a[k], inv);
-        if (inv) {
+        for (int q = 0; q < Q; ++q) {
+            Cplx t[R2];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                a[k][j].re *= 1.0 / 256.0;
-                a[k][j].im *= 1.0 / 256.0;
+            for (int c = 0; c < R2; ++c) t[c] = xb[k * reg_xsize<R1, R2, XP>() + reg_xi<R1, R2, XP>(l, s + R2 * q, c)];
+            dft_small<R2>(t, inv);
+#pragma unroll
+            for (int c = 0; c < R2; ++c) {
+                if (inv) {
+                    t[c].re *= 1.0 / N;
+                    t[c].im *= 1.0 / N;
+                }
+                a[k][q + Q * c] = t[c];
             }
         }
-    }
 }
 
-template <int MODE, bool XP>
-__global__ void __launch_bounds__(kF256Threads, 3) k_fft256(FieldsND F, FftPass f) {
-    extern __shared__ __align__(16) unsigned char f256_sm[];
-    Cplx* tws = reinterpret_cast<Cplx*>(f256_sm);
-    Cplx* xb = tws + 256;
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) tws[k] = f.tw[k];
+template <int MODE, bool XP, int R1, int R2>
+__global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_fft_reg(FieldsND F, FftPass f) {
+    extern __shared__ __align__(16) unsigned char reg_sm[];
+    Cplx* tws = reinterpret_cast<Cplx*>(reg_sm);
+    Cplx* xb = tws + R1 * R2;
+    for (int k = threadIdx.x; k < R1 * R2; k += blockDim.x) tws[k] = f.tw[k];
     int l, s;
-    f256_map<XP>(threadIdx.x, l, s);
+    reg_map<R2, XP>(threadIdx.x, l, s);
     const long long base = tile_base(f, blockIdx.x) + l * f.ls + s * f.es;
-    const long long step = 16 * f.es;  // between a thread's points
+    const long long step = R2 * f.es;  // between a thread's points
     constexpr bool PAIR = MODE == kInvInPlace || MODE == kInvToFields;
-    Cplx a[PAIR ? 2 : 1][16];
+    Cplx a[PAIR ? 2 : 1][R1];
     // ---- load ----
     if constexpr (MODE == kFwdFromRho) {
         // density_at with every load issued before the stores (the arrays may
         // alias as far as the compiler knows); the same sums in species order
-        double r[16];
+        double r[R1];
         if (F.rho_in) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = F.rho_in[base + j * step];
+            for (int j = 0; j < R1; ++j) r[j] = F.rho_in[base + j * step];
         } else if (F.nacc) {
 #pragma unroll
-            for (int j = 0; j < 16; ++j) r[j] = 0.0;
+            for (int j = 0; j < R1; ++j) r[j] = 0.0;
             for (int k = 0; k < F.nacc; ++k) {
-                unsigned long long q[16];
+                unsigned long long q[R1];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) q[j] = F.acc[k][base + j * step];
+                for (int j = 0; j < R1; ++j) q[j] = F.acc[k][base + j * step];
 #pragma unroll
-                for (int j = 0; j < 16; ++j) r[j] += (double)(long long)q[j] * F.acc_scale[k];
+                for (int j = 0; j < R1; ++j) r[j] += (double)(long long)q[j] * F.acc_scale[k];
             }
             for (int k = 0; k < F.nacc; ++k)
 #pragma unroll
-                for (int j = 0; j < 16; ++j) F.acc[k][base + j * step] = 0ull;
+                for (int j = 0; j < R1; ++j) F.acc[k][base + j * step] = 0ull;
         } else {
-            unsigned long long q[16];
+            unsigned long long q[R1];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) q[j] = F.rho_acc[base + j * step];
+            for (int j = 0; j < R1; ++j) q[j] = F.rho_acc[base + j * step];
 #pragma unroll
-            for (int j = 0; j < 16; ++j) {
+            for (int j = 0; j < R1; ++j) {
                 r[j] = (double)(long long)q[j] * F.inv_scale;
                 F.rho_acc[base + j * step] = 0ull;
             }
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < R1; ++j) {
             F.rho[base + j * step] = r[j];
             a[0][j] = {r[j], 0.0};
         }
     } else {
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < R1; ++j) {
             const long long g = base + j * step;
             if (MODE == kFwdInPlace || MODE == kFwdMulInv) a[0][j] = F.W[g];
             else {
@@ -2247,22 +2253,22 @@ __global__ void __launch_bounds__(kF256Threads, 3) k_fft256(FieldsND F, FftPass 
     }
     __syncthreads();  // the twiddles are staged
     if constexpr (MODE == kFwdMulInv) {
-        fft256<XP, 1>(a, xb, tws, l, s, false);
-        Cplx ab[2][16];
+        fft_reg<R1, R2, XP, 1>(a, xb, tws, l, s, false);
+        Cplx ab[2][R1];
 #pragma unroll
-        for (int j = 0; j < 16; ++j) kspace_tab(F, base + j * step, a[0][j], ab[0][j], ab[1][j]);
-        fft256<XP, 2>(ab, xb, tws, l, s, true);
+        for (int j = 0; j < R1; ++j) kspace_tab(F, base + j * step, a[0][j], ab[0][j], ab[1][j]);
+        fft_reg<R1, R2, XP, 2>(ab, xb, tws, l, s, true);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
+        for (int j = 0; j < R1; ++j) {
             const long long g = base + j * step;
             F.A[g] = ab[0][j];
             F.B[g] = ab[1][j];
         }
     } else {
-        fft256<XP, PAIR ? 2 : 1>(a, xb, tws, l, s, PAIR);
+        fft_reg<R1, R2, XP, PAIR ? 2 : 1>(a, xb, tws, l, s, PAIR);
     // ---- store ----
 #pragma unroll
-    for (int j = 0; j < 16; ++j) {
+    for (int j = 0; j < R1; ++j) {
         const long long g = base + j * step;
         if (MODE == kFwdFromRho || MODE == kFwdInPlace) F.W[g] = a[0][j];
         else if (MODE == kInvInPlace) {
@@ -2275,11 +2281,11 @@ __global__ void __launch_bounds__(kF256Threads, 3) k_fft256(FieldsND F, FftPass 
     }
 }
 
-// shared memory of a 256-point pass: the twiddles and one exchange buffer per line set
-template <bool XP>
-constexpr size_t f256_smem(int mode) {
-    return (256 + (size_t)((mode == kFwdMulInv || mode == kInvInPlace || mode == kInvToFields) ? 2 : 1) *
-                      f256_xsize<XP>()) * sizeof(Cplx);
+// shared memory of a register pass: the twiddles and one exchange buffer per line set
+template <int R1, int R2, bool XP>
+constexpr size_t reg_smem(int mode) {
+    return (R1 * R2 + (size_t)((mode == kFwdMulInv || mode == kInvInPlace || mode == kInvToFields) ? 2 : 1) *
+                          reg_xsize<R1, R2, XP>()) * sizeof(Cplx);
 }
 
 // Simulation2D/3D sample reductions (src/Diagnostics.cpp:111-137, :205-232):
@@ -2364,8 +2370,8 @@ struct Solver {
     FieldsND F{};
     FftPass px{}, py{}, pz{};    // paired passes (four line buffers)
     FftPass pxs{}, pys{};        // single-array forward passes (two line buffers)
-    bool use256[3] = {false, false, false};  // axis a runs the 256-point register kernels
-    FftPass q256[3]{};
+    bool in_regs[3] = {false, false, false};  // axis a runs the register kernels
+    FftPass reg[3]{};
     size_t smem_fwd = 0, smem_pair = 0;
     std::vector<void*>* allocs = nullptr;
     cudaStream_t stream = nullptr;
@@ -2466,10 +2472,10 @@ struct Solver {
         }
         for (int a = 0; a < dims; ++a) {
             const long long lines = a == 0 ? (long long)F.ny * F.nz : F.nx;
-            use256[a] = n[a] == 256 && lines % kF256Lines == 0;
-            if (use256[a]) {
-                q256[a] = pass(a, kF256Lines);
-                q256[a].tw = a == 0 ? px.tw : (a == 1 ? py.tw : pz.tw);
+            in_regs[a] = n[a] >= 32 && n[a] <= 256 && lines % kRegLines == 0;
+            if (in_regs[a]) {
+                reg[a] = pass(a, kRegLines);
+                reg[a].tw = a == 0 ? px.tw : (a == 1 ? py.tw : pz.tw);
             }
         }
         smem_pair = std::max(smem_of(px, kFwdMulInv), smem_of(py, kFwdMulInv));
@@ -2484,19 +2490,24 @@ struct Solver {
         return (mode == kFwdFromRho || mode == kFwdInPlace) ? 2 * line + tw : 4 * line + tw;
     }
 
-    // one pass along `axis`: the 256-point register kernel where the extent
+    // one pass along `axis`: the register kernel where the extent
     // allows it, else the shared-memory tile kernel with pass `tile`
+    template <int MODE, int R1, int R2>
+    void reg_pass(int axis) {
+        const FftPass& q = reg[axis];
+        const unsigned g = (unsigned)tiles(q);
+        if (axis == 0)
+            k_fft_reg<MODE, true, R1, R2><<<g, kRegLines * R2, reg_smem<R1, R2, true>(MODE), stream>>>(F, q);
+        else
+            k_fft_reg<MODE, false, R1, R2><<<g, kRegLines * R2, reg_smem<R1, R2, false>(MODE), stream>>>(F, q);
+    }
     template <int MODE>
     void fft_pass(int axis, const FftPass& tile) {
-        if (use256[axis]) {
-            const FftPass& q = q256[axis];
-            if (axis == 0)
-                k_fft256<MODE, true><<<(unsigned)tiles(q), kF256Threads, f256_smem<true>(MODE), stream>>>(F, q);
-            else
-                k_fft256<MODE, false><<<(unsigned)tiles(q), kF256Threads, f256_smem<false>(MODE), stream>>>(F, q);
-        } else {
-            k_fft<MODE><<<(unsigned)tiles(tile), kFftThreads, smem_of(tile, MODE), stream>>>(F, tile);
-        }
+        if (!in_regs[axis]) k_fft<MODE><<<(unsigned)tiles(tile), kFftThreads, smem_of(tile, MODE), stream>>>(F, tile);
+        else if (reg[axis].n == 256) reg_pass<MODE, 16, 16>(axis);
+        else if (reg[axis].n == 128) reg_pass<MODE, 16, 8>(axis);
+        else if (reg[axis].n == 64) reg_pass<MODE, 8, 8>(axis);
+        else reg_pass<MODE, 8, 4>(axis);
     }
 
     // rho_acc -> rho, phi, E (the fixed-point accumulator is cleared)
@@ -2540,7 +2551,7 @@ void ensure_solver_attributes();
 //
 // Solve per step on the B200, before (one real line per CTA and transform, a
 // serial sweep per mode, separate passes for every elementwise stage) -> now:
-// 512 x 513 (mixed) 87 -> 41 us, 129^3 949 -> 304 us.
+// 512 x 513 (mixed) 87 -> 39 us, 129^3 949 -> 304 us, with the register transforms 133 us.
 constexpr size_t kWallTileBytes = 72 * 1024;  // shared memory of a tile: three CTAs per SM
 constexpr size_t kWallSmemMax = (2 * ((size_t)kMaxLine + 1) + kMaxLine) * sizeof(Cplx) > kWallTileBytes
                                     ? (2 * ((size_t)kMaxLine + 1) + kMaxLine) * sizeof(Cplx) : kWallTileBytes;
@@ -2572,6 +2583,8 @@ struct WallMesh {
     double d[3], eps;
     double side[4];                // 2D potentials: left, right, bottom, top
     int wall[3];
+    double rd[2][3], reps;         // reciprocals of d and of 2 d, and of eps
+    double ih2[2];                 // 1 / d^2 of x and y
 };
 
 // Lines of M values in place (or from rho, or into phi): X_m = sum_k x_k
@@ -2615,13 +2628,12 @@ __global__ void __launch_bounds__(kFftThreads) k_dst_pass(double* __restrict__ u
             const int la = line % f.lines_a, lb = line / f.lines_a;
             if (MODE == kDstFromRho) {  // axis 0: line (j, k) = (la, lb), right-hand side at node e
                 const size_t node = ((size_t)(w.dims == 3 ? lb + 1 : 0) * w.n[1] + (la + 1)) * w.n[0] + (e + 1);
-                v = rho[node] / w.eps;
+                v = cells_of(rho[node], w.eps, w.reps);
                 if (w.dims == 2) {  // 2D walls at their potentials; 3D walls are grounded
-                    const double idx2 = 1.0 / (w.d[0] * w.d[0]), idy2 = 1.0 / (w.d[1] * w.d[1]);
-                    if (e == 0) v += w.side[0] * idx2;
-                    if (e == M - 1) v += w.side[1] * idx2;
-                    if (la == 0) v += w.side[2] * idy2;
-                    if (la == w.n[1] - 3) v += w.side[3] * idy2;
+                    if (e == 0) v += w.side[0] * w.ih2[0];
+                    if (e == M - 1) v += w.side[1] * w.ih2[0];
+                    if (la == 0) v += w.side[2] * w.ih2[1];
+                    if (la == w.n[1] - 3) v += w.side[3] * w.ih2[1];
                 }
             } else {
                 v = u[la * f.stride_a + lb * f.stride_b + e * f.stride];
@@ -2666,6 +2678,108 @@ __global__ void __launch_bounds__(kFftThreads) k_dst_pass(double* __restrict__ u
             phi[((size_t)(w.dims == 3 ? lb + 1 : 0) * w.n[1] + (la + 1)) * w.n[0] + (e + 1)] = v;
         else
             u[la * f.stride_a + lb * f.stride_b + e * f.stride] = v;
+    }
+}
+
+// The same passes for N = R1 R2 = 64 .. 256 (33 to 129 nodes) in registers: eight
+// line pairs per CTA, laid out as in k_fft_reg.  Both halves of the odd extension are read
+// from the interior values, and the transform of an odd sequence is odd, so
+// the second transform of kDstSolve starts from the first one's own positions.
+template <int MODE, bool XP, int R1, int R2>
+__global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_dst_reg(double* __restrict__ u, WallMesh w, DstPass f,
+                                                                      const double* __restrict__ rho,
+                                                                      double* __restrict__ phi) {
+    extern __shared__ __align__(16) unsigned char reg_sm[];
+    constexpr int N = R1 * R2, M = N / 2 - 1;
+    Cplx* tws = reinterpret_cast<Cplx*>(reg_sm);
+    Cplx* xb = tws + N;
+    for (int k = threadIdx.x; k < N; k += blockDim.x) tws[k] = f.tw[k];
+    int l, s;
+    reg_map<R2, XP>(threadIdx.x, l, s);
+    int la[2], lb[2];  // the pair's two real lines
+    bool in[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        // strided passes: lane l takes lines l and l + 8 of the tile, so both loads are contiguous
+        const int line = blockIdx.x * (2 * kRegLines) + (XP ? 2 * l + c : l + kRegLines * c);
+        in[c] = line < f.lines;
+        la[c] = in[c] ? line % f.lines_a : 0;
+        lb[c] = in[c] ? line / f.lines_a : 0;
+    }
+    // every load first (no branch between them), then the right-hand side and the extension
+    const double* src[2];
+    long long stride = 1;
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (MODE == kDstFromRho) {
+            src[c] = rho + ((size_t)(w.dims == 3 ? lb[c] + 1 : 0) * w.n[1] + (la[c] + 1)) * w.n[0] + 1;
+        } else {
+            src[c] = u + la[c] * f.stride_a + lb[c] * f.stride_b;
+            stride = f.stride;
+        }
+    }
+    Cplx a[1][R1];
+#pragma unroll
+    for (int j = 0; j < R1; ++j) {
+        const int k = s + R2 * j;
+        // (k = 0 and k = M + 1, the extension's zeros, load a neighbour)
+        const int e = k <= M ? max(k - 1, 0) : min(N - k - 1, M - 1);
+        a[0][j] = {src[0][e * stride], src[1][e * stride]};
+    }
+#pragma unroll
+    for (int j = 0; j < R1; ++j) {
+        const int k = s + R2 * j;
+        const bool zero = k == 0 || k == M + 1;
+        double x[2] = {a[0][j].re, a[0][j].im};
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (MODE == kDstFromRho) {
+                x[c] = cells_of(x[c], w.eps, w.reps);
+                if (w.dims == 2) {  // 2D walls at their potentials; 3D walls are grounded
+                    const int e = k <= M ? k - 1 : N - k - 1;
+                    if (e == 0) x[c] += w.side[0] * w.ih2[0];
+                    if (e == M - 1) x[c] += w.side[1] * w.ih2[0];
+                    if (la[c] == 0) x[c] += w.side[2] * w.ih2[1];
+                    if (la[c] == w.n[1] - 3) x[c] += w.side[3] * w.ih2[1];
+                }
+            }
+            x[c] = zero || !in[c] ? 0.0 : (k <= M ? x[c] : -x[c]);
+        }
+        a[0][j] = {x[0], x[1]};
+    }
+    __syncthreads();  // the twiddles are staged
+    fft_reg<R1, R2, XP, 1>(a, xb, tws, l, s, false);
+    if (MODE == kDstSolve) {
+#pragma unroll
+        for (int j = 0; j < R1; ++j) {
+            const int k = s + R2 * j;
+            const bool zero = k == 0 || k == M + 1;
+            const int e = zero ? 0 : (k <= M ? k - 1 : N - k - 1);
+            double g[2];
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                // (the last axis: la is the x index, lb the y index in 3D)
+                const double lam = __ldg(f.eig[0] + la[c]) + (w.dims == 3 ? __ldg(f.eig[1] + lb[c]) + __ldg(f.eig[2] + e)
+                                                                         : __ldg(f.eig[1] + e));
+                g[c] = zero ? 0.0 : f.scale * __drcp_rn(lam);
+            }
+            a[0][j] = {-0.5 * a[0][j].im * g[0], 0.5 * a[0][j].re * g[1]};
+        }
+        fft_reg<R1, R2, XP, 1>(a, xb, tws, l, s, false);
+    }
+#pragma unroll
+    for (int j = 0; j < R1; ++j) {
+        const int k = s + R2 * j;
+        if (k == 0 || k > M) continue;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            if (!in[c]) continue;
+            const double v = c ? 0.5 * a[0][j].re : -0.5 * a[0][j].im;
+            if (MODE == kDstToPhi)
+                phi[((size_t)(w.dims == 3 ? lb[c] + 1 : 0) * w.n[1] + (la[c] + 1)) * w.n[0] + k] = v;
+            else
+                u[la[c] * f.stride_a + lb[c] * f.stride_b + (k - 1) * f.stride] = v;
+        }
     }
 }
 
@@ -2860,34 +2974,34 @@ __global__ void k_wall_sides(double* __restrict__ phi, WallMesh w) {
 
 // compute_electric_field(Mesh2D&) and the 3D differences, src/FieldSolver.cpp:298-346,
 // :872-904: central, one-sided at the walls, into the push's interleaved
-// layout or into planes (Ex | Ey (| Ez)).  One row of x per block row.
+// layout or into planes (Ex | Ey (| Ez)).  The differences are divided through
+// reciprocals (cells_of); rd holds 1 / d, then 1 / (2 d).
 template <int DIM>
-__global__ void k_wall_efield(const double* __restrict__ phi, double* __restrict__ E, double* __restrict__ planes,
-                              WallMesh w) {
-    const int nx = w.n[0], ny = w.n[1], nz = DIM == 3 ? w.n[2] : 1;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nx) return;
-    const size_t N = (size_t)nx * ny * nz;
-    auto slope = [&](const double* p, int c, int n, long long s, int wall, double d) {
-        if (!wall) return -(p[c + 1 == n ? -(long long)c * s : s] - p[c == 0 ? (long long)(n - 1) * s : -s]) / (2.0 * d);
-        if (c == 0) return -(p[s] - p[0]) / d;
-        if (c + 1 == n) return -(p[0] - p[-s]) / d;
-        return -(p[s] - p[-s]) / (2.0 * d);
-    };
-    for (int r = blockIdx.y * blockDim.y + threadIdx.y; r < ny * nz; r += gridDim.y * blockDim.y) {
-        const int j = DIM == 3 ? r % ny : r, k = DIM == 3 ? r / ny : 0;
-        const size_t q = (size_t)r * nx + i;
-        const double ex = slope(phi + q, i, nx, 1, w.wall[0], w.d[0]);
-        const double ey = slope(phi + q, j, ny, nx, w.wall[1], w.d[1]);
-        const double ez = DIM == 3 ? slope(phi + q, k, nz, (long long)nx * ny, w.wall[2], w.d[2]) : 0.0;
+__global__ void __launch_bounds__(256) k_wall_efield(const double* __restrict__ phi, double* __restrict__ E,
+                                                     double* __restrict__ planes, WallMesh w) {
+    const unsigned nx = w.n[0], ny = w.n[1], nz = DIM == 3 ? w.n[2] : 1, N = nx * ny * nz;
+    for (unsigned q = blockIdx.x * blockDim.x + threadIdx.x; q < N; q += gridDim.x * blockDim.x) {
+        const unsigned row = q / nx;
+        const unsigned c[3] = {q - row * nx, DIM == 3 ? row % ny : row, DIM == 3 ? row / ny : 0u};
+        const unsigned n[3] = {nx, ny, nz}, stride[3] = {1u, nx, nx * ny};
+        double e[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+            const bool low = c[a] == 0u, high = c[a] + 1u == n[a];
+            // the neighbours: wrapped on a periodic axis, the node itself past a wall
+            const unsigned up = high ? (w.wall[a] ? q : q - c[a] * stride[a]) : q + stride[a];
+            const unsigned dn = low ? (w.wall[a] ? q : q + (n[a] - 1u) * stride[a]) : q - stride[a];
+            const bool one = w.wall[a] && (low || high);
+            const double d = one ? w.d[a] : 2.0 * w.d[a];
+            e[a] = -cells_of(__ldg(phi + up) - __ldg(phi + dn), d, one ? w.rd[0][a] : w.rd[1][a]);
+        }
         if (planes) {
-            planes[q] = ex;
-            planes[N + q] = ey;
-            if (DIM == 3) planes[2 * N + q] = ez;
+#pragma unroll
+            for (int a = 0; a < DIM; ++a) planes[a * (size_t)N + q] = e[a];
         } else if (DIM == 3) {
-            reinterpret_cast<double4*>(E)[q] = make_double4(ex, ey, ez, 0.0);
+            reinterpret_cast<double4*>(E)[q] = make_double4(e[0], e[1], e[2], 0.0);
         } else {
-            reinterpret_cast<double2*>(E)[q] = make_double2(ex, ey);
+            reinterpret_cast<double2*>(E)[q] = make_double2(e[0], e[1]);
         }
     }
 }
@@ -2923,10 +3037,14 @@ struct WallSolver {
     void setup(int dims, const int* n, const double* d, const int* wall, double eps, const double* pot) {
         w.dims = dims;
         w.eps = eps;
+        w.reps = reciprocal_spacing(eps);
+        for (int a = 0; a < 2; ++a) w.ih2[a] = 1.0 / (d[a] * d[a]);
         for (int a = 0; a < 3; ++a) {
             w.n[a] = a < dims ? n[a] : 1;
             w.d[a] = a < dims ? d[a] : 1.0;
             w.wall[a] = a < dims ? wall[a] : 0;
+            w.rd[0][a] = reciprocal_spacing(w.d[a]);
+            w.rd[1][a] = reciprocal_spacing(2.0 * w.d[a]);
         }
         for (int k = 0; k < 4; ++k) w.side[k] = dims == 2 ? pot[k] : 0.0;
         ensure_solver_attributes();
@@ -2989,6 +3107,22 @@ struct WallSolver {
     template <int MODE>
     void dst(int a, const double* rho, double* phi) {
         const DstPass& f = pass[a];
+        auto in_regs = [&](auto r1, auto r2) {
+            constexpr int R1 = decltype(r1)::value, R2 = decltype(r2)::value;
+            const unsigned g = (unsigned)((f.lines + 2 * kRegLines - 1) / (2 * kRegLines));
+            if (a == 0)
+                k_dst_reg<MODE, true, R1, R2><<<g, kRegLines * R2, reg_smem<R1, R2, true>(kFwdInPlace), stream>>>(u, w, f, rho, phi);
+            else
+                k_dst_reg<MODE, false, R1, R2><<<g, kRegLines * R2, reg_smem<R1, R2, false>(kFwdInPlace), stream>>>(u, w, f, rho, phi);
+        };
+        using I8 = std::integral_constant<int, 8>;
+        using I16 = std::integral_constant<int, 16>;
+        switch (f.log2N) {
+            case 6: in_regs(I8{}, I8{}); return;
+            case 7: in_regs(I16{}, I8{}); return;
+            case 8: in_regs(I16{}, I16{}); return;
+            default: break;
+        }
         const unsigned g = (unsigned)((f.lines + 2 * f.T - 1) / (2 * f.T));
         k_dst_pass<MODE><<<g, kFftThreads, wall_smem(2 * (f.M + 1), f.T), stream>>>(u, w, f, rho, phi);
     }
@@ -3018,9 +3152,9 @@ struct WallSolver {
             dst<kDstInPlace>(1, rho, phi);
             dst<kDstToPhi>(0, rho, phi);
         }
-        const dim3 block(64, 4), grid((w.n[0] + 63) / 64, (unsigned)std::min<long long>(((long long)w.n[1] * w.n[2] + 3) / 4, 65535));
-        if (w.dims == 2) k_wall_efield<2><<<grid, block, 0, stream>>>(phi, E, planes, w);
-        else k_wall_efield<3><<<grid, block, 0, stream>>>(phi, E, planes, w);
+        const unsigned grid = (unsigned)(((size_t)w.n[0] * w.n[1] * w.n[2] + 255) / 256);
+        if (w.dims == 2) k_wall_efield<2><<<grid, 256, 0, stream>>>(phi, E, planes, w);
+        else k_wall_efield<3><<<grid, 256, 0, stream>>>(phi, E, planes, w);
         APIC_CUDA(cudaGetLastError());
     }
 };
@@ -3029,6 +3163,22 @@ namespace {
 std::mutex g_attr_mu;
 bool g_attr_done[64] = {};
 }  // namespace
+
+template <int MODE, int R1, int R2>
+static void set_reg_mode() {
+    APIC_CUDA(cudaFuncSetAttribute(k_fft_reg<MODE, true, R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)reg_smem<R1, R2, true>(MODE)));
+    APIC_CUDA(cudaFuncSetAttribute(k_fft_reg<MODE, false, R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)reg_smem<R1, R2, false>(MODE)));
+}
+template <int R1, int R2>
+static void set_reg_attributes() {
+    set_reg_mode<kFwdFromRho, R1, R2>();
+    set_reg_mode<kFwdInPlace, R1, R2>();
+    set_reg_mode<kFwdMulInv, R1, R2>();
+    set_reg_mode<kInvInPlace, R1, R2>();
+    set_reg_mode<kInvToFields, R1, R2>();
+}
 
 void ensure_solver_attributes() {
     int dev = 0;
@@ -3042,17 +3192,10 @@ void ensure_solver_attributes() {
     APIC_CUDA(cudaFuncSetAttribute(k_fft<kFwdMulInv>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
     APIC_CUDA(cudaFuncSetAttribute(k_fft<kInvInPlace>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
     APIC_CUDA(cudaFuncSetAttribute(k_fft<kInvToFields>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    const int f256x = (int)f256_smem<true>(kInvToFields), f256s = (int)f256_smem<false>(kInvToFields);
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdFromRho, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256x));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdInPlace, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256x));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdMulInv, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256x));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kInvInPlace, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256x));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kInvToFields, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256x));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdFromRho, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256s));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdInPlace, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256s));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kFwdMulInv, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256s));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kInvInPlace, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256s));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft256<kInvToFields, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, f256s));
+    set_reg_attributes<16, 16>();
+    set_reg_attributes<16, 8>();
+    set_reg_attributes<8, 8>();
+    set_reg_attributes<8, 4>();
     auto set_box = [](auto kernel, size_t bytes) {
         APIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     };

@@ -158,7 +158,7 @@ def test_mixed_solve_sizes(n, axis):
     assert rel_max(E, Er) < 10 * tol
 
 
-@pytest.mark.parametrize("n", [(3, 3), (5, 3), (3, 513), (513, 9), (3, 5, 9), (17, 3, 3), (33, 65, 17)])
+@pytest.mark.parametrize("n", [(3, 3), (5, 3), (3, 513), (513, 9), (3, 5, 9), (17, 3, 3), (33, 65, 17), (129, 33), (9, 129, 65)])
 def test_dirichlet_solve_sizes(n):
     """The discrete equation at every interior node: eps Laplacian(phi) = -rho."""
     rng = np.random.default_rng(sum(n))
@@ -292,3 +292,25 @@ def test_tiled_push_with_crowded_nodes():
         want += np.bincount((g[2] * n[1] + g[1]) * n[0] + g[0], -0.01 * w, want.size)
     # weights are multiples of 2^-23, offsets 24-bit floats
     assert rel_max(rho, want) < 1e-6
+
+
+@pytest.mark.parametrize("n", [(128, 64), (64, 128), (32, 128), (512, 32), (16, 128), (64, 64, 64), (128, 32, 16), (32, 64, 128)])
+def test_periodic_solve_of_every_line_length(n):
+    """Register transforms of 32 to 256 points along contiguous and strided axes, mixed
+    with the shared-memory tiles."""
+    rng = np.random.default_rng(sum(n))
+    dims = len(n)
+    length = (2.0, 3.0, 1.5)[:dims]
+    shape = tuple(reversed(n))
+    rho = rng.standard_normal(shape)
+    phi, E = apic.field_solve_periodic_nd(dims, n, length, 1.3, rho)
+    hat = np.fft.fftn(rho)
+    k = [2 * np.pi * np.fft.fftfreq(n[a], length[a] / n[a]).reshape([-1 if dims - 1 - b == a else 1 for b in range(dims)])
+         for a in range(dims)]
+    k2 = sum(q * q for q in k) * np.ones(shape)
+    k2.flat[0] = 1.0
+    ph = hat / (1.3 * k2)
+    ph.flat[0] = 0.0
+    assert rel_max(phi.reshape(shape), np.fft.ifftn(ph).real) < TOL
+    for a in range(dims):
+        assert rel_max(E[a].reshape(shape), np.fft.ifftn(-1j * k[a] * ph).real) < TOL

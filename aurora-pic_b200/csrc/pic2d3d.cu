@@ -450,21 +450,30 @@ enum : int { kNoField = 0, kUniformField = 1, kProfileField = 2 };
 
 // The FP64 step push: kick, drift, particle boundaries and CIC deposit of
 // kRunItems consecutive particles per thread.  Particles are sorted by cell,
-// so the field at a cell's nodes is fetched once per run of equal cells, the
-// fixed-point contributions of a run are summed in registers, a run that ends
-// inside the thread is committed with one atomic per node, and each lane's
-// last run joins a segmented sum over the lanes that end in the same cell.
+// so the fixed-point contributions of a run of equal cells are summed in registers,
+// a run that ends inside the thread is committed with one atomic per node, and each lane's
+// last run joins a segmented sum over the lanes that end in the same cell.  The
+// field is read from L1 for each particle: keeping a cell's nodes for the next particle
+// took 48 registers and a third of the warps (64^3: 436 us a step against 384).
 // The state moves as 16-byte vectors.  Contributions are integers, so the
 // density does not depend on how particles are grouped.
 // Against one particle per thread with 64-bit index remainders (both species, per
-// step): 2 x 1 M particles on 256 x 128, 81 -> 70 us; 2 x 4.2 M on 64^3,
-// 483 -> 437 us (bound by load latency at 2 CTAs an SM and, between sorts, by the
-// deposit's global atomics); walls, 2 x 2 M on 512 x 513, 161 -> 129 us and
-// 2 x 4.2 M on 129^3, 680 -> 545 us (these also sorted by cell now).
+// step): 2 x 1 M particles on 256 x 128, 81 -> 63 us; 2 x 4.2 M on 64^3,
+// 483 -> 384 us (bound by load latency and, between sorts, by the
+// deposit's global atomics); walls, 2 x 2 M on 512 x 513, 161 -> 113 us and
+// 2 x 4.2 M on 129^3, 680 -> 490 us (these also sorted by cell now).
 constexpr int kRunItems = 2;
 
+// One buffer of the FP64 state, by kernel argument (an index into the species'
+// arrays costs every access its pointer's load).
+struct State64 {
+    double* pos[3];
+    double* vh[3];
+    uint8_t* alive;
+};
+
 template <int DIM, int BKIND, bool WALLS>
-__global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, int buf) {
+__global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsND p, SpeciesND S, State64 A) {
     constexpr int NN = DIM == 2 ? 4 : 8;
     const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * kRunItems;
     const int lane = threadIdx.x & 31;
@@ -477,21 +486,20 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
     for (int a = 0; a < 3; ++a) {
         double2 q{0.0, 0.0}, w{0.0, 0.0};
         if (full) {
-            if (a < DIM) q = __ldcs(reinterpret_cast<const double2*>(S.pos[buf][a] + first));
-            w = __ldcs(reinterpret_cast<const double2*>(S.vh[buf][a] + first));
+            if (a < DIM) q = __ldcs(reinterpret_cast<const double2*>(A.pos[a] + first));
+            w = __ldcs(reinterpret_cast<const double2*>(A.vh[a] + first));
         } else if (first < S.n) {
-            if (a < DIM) q.x = S.pos[buf][a][first];
-            w.x = S.vh[buf][a][first];
+            if (a < DIM) q.x = A.pos[a][first];
+            w.x = A.vh[a][first];
         }
         x[0][a] = q.x; x[1][a] = q.y;
         v[0][a] = w.x; v[1][a] = w.y;
     }
 #pragma unroll
     for (int k = 0; k < kRunItems; ++k)
-        live[k] = first + k < S.n && (!WALLS || !S.alive[buf] || S.alive[buf][first + k]);
+        live[k] = first + k < S.n && (!WALLS || !A.alive || A.alive[first + k]);
     const unsigned kNoCell = 0xFFFFFFFFu;
-    unsigned gcell = kNoCell, rcell = kNoCell;  // cells of the cached field and of the current deposit run
-    double en[NN][DIM];
+    unsigned rcell = kNoCell;  // cell of the current deposit run
     long long racc[NN];
     unsigned rnode[3] = {0u, 0u, 0u};  // steps from the run's first node to its upper x, y, z neighbours
 #pragma unroll
@@ -508,26 +516,25 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
         if (!live[k]) continue;
         const Axis gx = axis2<WALLS>(p, 0, x[k][0]), gy = axis2<WALLS>(p, 1, x[k][1]);
         const Axis gz = DIM == 3 ? axis2<WALLS>(p, 2, x[k][DIM - 1]) : Axis{0, 0, 0.0};
-        const unsigned c0 = ((unsigned)gz.i0 * ny + gy.i0) * nx + gx.i0;
-        if (c0 != gcell) {
-            gcell = c0;
-#pragma unroll
-            for (int j = 0; j < NN; ++j) {
-                const unsigned g = ((unsigned)((j & 4) ? gz.i1 : gz.i0) * ny + ((j & 2) ? gy.i1 : gy.i0)) * nx +
-                                   ((j & 1) ? gx.i1 : gx.i0);
-                if (DIM == 2) {
-                    const double2 q = __ldg(reinterpret_cast<const double2*>(p.E) + g);
-                    en[j][0] = q.x; en[j][1] = q.y;
-                } else {
-                    const double2* E = reinterpret_cast<const double2*>(p.E) + 2 * (size_t)g;
-                    const double2 q = __ldg(E);
-                    en[j][0] = q.x; en[j][1] = q.y;
-                    en[j][DIM - 1] = __ldg(reinterpret_cast<const double*>(E + 1));
-                }
+        // field at node j of the cell
+        auto node_field = [&](int j, double* out) {
+            const unsigned g = ((unsigned)((j & 4) ? gz.i1 : gz.i0) * ny + ((j & 2) ? gy.i1 : gy.i0)) * nx +
+                               ((j & 1) ? gx.i1 : gx.i0);
+            if (DIM == 2) {
+                const double2 q = __ldg(reinterpret_cast<const double2*>(p.E) + g);
+                out[0] = q.x; out[1] = q.y;
+            } else {
+                const double2* E = reinterpret_cast<const double2*>(p.E) + 2 * (size_t)g;
+                const double2 q = __ldg(E);
+                out[0] = q.x; out[1] = q.y;
+                out[DIM - 1] = __ldg(reinterpret_cast<const double*>(E + 1));
             }
-        }
+        };
         double e[3] = {0.0, 0.0, 0.0};
         if (DIM == 2) {
+            double en[NN][DIM];
+#pragma unroll
+            for (int j = 0; j < NN; ++j) node_field(j, en[j]);
             const double fx = gx.f, fy = gy.f;
             const double w00 = (1.0 - fx) * (1.0 - fy), w10 = fx * (1.0 - fy), w01 = (1.0 - fx) * fy, w11 = fx * fy;
             e[0] = en[0][0] * w00 + en[1][0] * w10 + en[2][0] * w01 + en[3][0] * w11;
@@ -538,8 +545,10 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
 #pragma unroll
             for (int j = 0; j < NN; ++j) {
                 const double shape = wx[j & 1] * wy[(j >> 1) & 1] * wz[(j >> 2) & 1];
+                double q[3];
+                node_field(j, q);
 #pragma unroll
-                for (int a = 0; a < DIM; ++a) e[a] += en[j][a] * shape;
+                for (int a = 0; a < DIM; ++a) e[a] += q[a] * shape;
             }
         }
         // kick_boris / kick_leapfrog + drift_leapfrog, src/Pusher.cpp:109-128, :162-174
@@ -558,7 +567,7 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
             for (int a = 0; a < DIM; ++a) x[k][a] = x[k][a] + v[k][a] * p.dt;
             const int side = apply_walls<DIM>(p, x[k], v[k]);
             if (side >= 0) {
-                S.alive[buf][first + k] = 0;
+                A.alive[first + k] = 0;
                 atomicAdd(p.losses + 6 * S.index + side, 1ull);
                 continue;
             }
@@ -584,11 +593,14 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
             for (int j = 0; j < NN; ++j) racc[j] = 0;
         }
         const double ux[2] = {1.0 - ax.f, ax.f}, uy[2] = {1.0 - ay.f, ay.f}, uz[2] = {1.0 - az.f, az.f};
+        // a cell on a wall (the volume factors are 1 elsewhere)
+        const bool edge = WALLS && (ax.i0 == 0 || ax.i1 == nx - 1 || ay.i0 == 0 || ay.i1 == ny - 1 ||
+                                    (DIM == 3 && (az.i0 == 0 || az.i1 == p.n[2] - 1)));
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
             double c = DIM == 2 ? S.dep * ux[j & 1] * uy[(j >> 1) & 1]
                                 : S.dep * (ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1]);
-            if (WALLS) {  // q shape / node volume over the wall nodes' half cells
+            if (WALLS && edge) {  // q shape / node volume over the wall nodes' half cells
                 double f = area_factor<WALLS>(p, 0, (j & 1) ? ax.i1 : ax.i0) *
                            area_factor<WALLS>(p, 1, (j & 2) ? ay.i1 : ay.i0);
                 if (DIM == 3) f *= area_factor<WALLS>(p, 2, (j & 4) ? az.i1 : az.i0);
@@ -601,11 +613,11 @@ __global__ void __launch_bounds__(kThreads) k_push_run(ParamsND p, SpeciesND S, 
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         if (full) {
-            if (a < DIM) __stcs(reinterpret_cast<double2*>(S.pos[buf][a] + first), make_double2(x[0][a], x[1][a]));
-            __stcs(reinterpret_cast<double2*>(S.vh[buf][a] + first), make_double2(v[0][a], v[1][a]));
+            if (a < DIM) __stcs(reinterpret_cast<double2*>(A.pos[a] + first), make_double2(x[0][a], x[1][a]));
+            __stcs(reinterpret_cast<double2*>(A.vh[a] + first), make_double2(v[0][a], v[1][a]));
         } else if (first < S.n) {
-            if (a < DIM) S.pos[buf][a][first] = x[0][a];
-            S.vh[buf][a][first] = v[0][a];
+            if (a < DIM) A.pos[a][first] = x[0][a];
+            A.vh[a][first] = v[0][a];
         }
     }
     // each lane's last run, summed over segments of at most RSEG lanes that end in the same cell
@@ -3663,12 +3675,14 @@ struct SimND {
         if (MODE == kPushStep) {
             const unsigned g = (S.n + kRunItems * kThreads - 1) / (kRunItems * kThreads);
             const int kind = !boris ? kNoField : (p.prof_rows ? kProfileField : kUniformField);
+            State64 A{{}, {}, S.alive[b]};
+            for (int a = 0; a < 3; ++a) { A.pos[a] = S.pos[b][a]; A.vh[a] = S.vh[b][a]; }
             auto run = [&](auto dim, auto wall) {
                 constexpr int D = decltype(dim)::value;
                 constexpr bool Wl = decltype(wall)::value;
-                if (kind == kNoField) k_push_run<D, kNoField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
-                else if (kind == kUniformField) k_push_run<D, kUniformField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
-                else k_push_run<D, kProfileField, Wl><<<g, kThreads, 0, stream>>>(p, S, b);
+                if (kind == kNoField) k_push_run<D, kNoField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
+                else if (kind == kUniformField) k_push_run<D, kUniformField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
+                else k_push_run<D, kProfileField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
             };
             using D2 = std::integral_constant<int, 2>;
             using D3 = std::integral_constant<int, 3>;

@@ -192,6 +192,13 @@ struct Params1D {
     unsigned cand_regions, cand_per_region;
 };
 
+// Programmatic launches: a step's kernels are launched while the one before them
+// is finishing (grid_release, at its tail), set up what does not depend on it, and wait
+// for its completion and its writes (grid_wait) before they read anything
+// of the run.
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // ---- field gather / deposit (reference arithmetic) ----------------------
 
 // wrap_periodic, src/FieldSolver.cpp:15-17: fmod(fmod(x, L) + L, L).  For
@@ -451,10 +458,11 @@ __global__ void __launch_bounds__(kThreads, KIND == kPassPlain ? kPlainBlocks<VD
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const unsigned mode = p.mode;
     for (int i = tid; i < p.nx; i += kThreads) {
-        sE[i] = p.E[i];
         sLo[i] = 0u;
         sHi[i] = 0u;
     }
+    grid_wait();
+    for (int i = tid; i < p.nx; i += kThreads) sE[i] = p.E[i];
     if (MCC) {
         for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
             (&s_chan[warp][0][0])[i] = 0u;
@@ -739,6 +747,7 @@ __global__ void __launch_bounds__(kThreads, KIND == kPassPlain ? kPlainBlocks<VD
         if (compact) __syncthreads();
     }
     __syncthreads();
+    grid_release();
     if (mode & kModeDeposit) {
         for (int i = tid; i < p.nx; i += kThreads) {
             const unsigned long long a = join64(sLo[i], sHi[i]);
@@ -793,10 +802,11 @@ __global__ void __launch_bounds__(kMccThreads, kMccBlocks) k_pass1d_mcc(Params1D
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     for (int i = tid; i < p.nx; i += kMccThreads) {
-        sE[i] = p.E[i];
         sLo[i] = 0u;
         sHi[i] = 0u;
     }
+    grid_wait();
+    for (int i = tid; i < p.nx; i += kMccThreads) sE[i] = p.E[i];
     for (int i = lane; i < kMaxModels * kMaxChannels; i += 32) {
         (&s_chan[warp][0][0])[i] = 0u;
         (&s_energy[warp][0][0])[i] = 0.0;
@@ -1046,6 +1056,7 @@ __global__ void __launch_bounds__(kMccThreads, kMccBlocks) k_pass1d_mcc(Params1D
         if (tid == 0) S.chunk_surv[tile] = out - base;
     }
     __syncthreads();
+    grid_release();
     for (int i = tid; i < p.nx; i += kMccThreads) {
         const unsigned long long a = join64(sLo[i], sHi[i]);
         if (a) atomicAdd(&p.rho_acc[i], a);
@@ -1251,19 +1262,25 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
     DevState* st = p.st;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const bool solve = (post & kPostSolve) != 0;
-    const double field_time = (post & kPostAdvance) ? st->time + p.dt : st->time;
 
-    // -- one round trip: density accumulators and solver coefficients --
+    // -- the solver's coefficients (constant), then the density accumulators --
     if (solve) {
 #pragma unroll 1
         for (int i = tid; i < nx; i += kPostThreads) {
-            s_rhoi[i] = p.rho_acc[i];
-            p.rho_acc[i] = 0ull;
             if (DIRICHLET) {
                 if (i < nx - 2) { s_c0[i] = p.thomas_r[i]; s_c1[i] = p.thomas_a[i]; }
             } else {
                 reinterpret_cast<double2*>(s_c0)[i] = reinterpret_cast<const double2*>(p.tw)[i];
             }
+        }
+    }
+    grid_wait();
+    const double field_time = (post & kPostAdvance) ? st->time + p.dt : st->time;
+    if (solve) {
+#pragma unroll 1
+        for (int i = tid; i < nx; i += kPostThreads) {
+            s_rhoi[i] = p.rho_acc[i];
+            p.rho_acc[i] = 0ull;
         }
         // one lane of two warps each: the sine's code is there once
         if (DIRICHLET && lane == 0 && warp < 2)
@@ -1453,6 +1470,7 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         st->n[tid] = s_surv[tid] + kept;
     }
     if (tid == 0) st->nbirths = 0;
+    grid_release();
     if (!solve) return;
     __syncthreads();
 
@@ -2466,22 +2484,39 @@ struct Sim1D {
                                        psm));
     }
 
+    // a kernel of a step, launched while the one before it finishes (it calls grid_wait)
+    void launch_dependent(void (*kernel)(Params1D), int grid, int block, size_t smem, const Params1D& q) {
+        cudaLaunchConfig_t lc = {};
+        lc.gridDim = dim3((unsigned)grid);
+        lc.blockDim = dim3((unsigned)block);
+        lc.dynamicSmemBytes = smem;
+        lc.stream = stream;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        lc.attrs = attr;
+        lc.numAttrs = 1;
+        APIC_CUDA(cudaLaunchKernelEx(&lc, kernel, q));
+    }
+
     template <int VDIM, bool DIR>
     void launch_kernels_c32(const Params1D& q, int blocks, size_t post_smem, unsigned post, EvPair& ev) {
-        k_pass1d_c32<VDIM, DIR><<<blocks, kThreads, (size_t)cfg.nx * 12, stream>>>(q);
+        launch_dependent(k_pass1d_c32<VDIM, DIR>, blocks, kThreads, (size_t)cfg.nx * 12, q);
         if (VDIM == 3 && cfg.nmodels > 0 && (q.mode & kModeSyncMcc))
-            k_collide1d_c32<VDIM, DIR><<<148 * 4, kCollideThreads, 0, stream>>>(q);
+            launch_dependent(k_collide1d_c32<VDIM, DIR>, 148 * 4, kCollideThreads, 0, q);
         if (timing) cudaEventRecord(ev.b, stream);
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(1);
         lc.blockDim = dim3(kPostThreads);
         lc.dynamicSmemBytes = post_smem;
         lc.stream = stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributePriority;
         attr[0].val.priority = post_priority;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         lc.attrs = attr;
-        lc.numAttrs = 1;
+        lc.numAttrs = 2;
         APIC_CUDA(cudaLaunchKernelEx(&lc, k_post1d<VDIM, DIR, true, true>, q, post));
     }
 
@@ -2494,24 +2529,26 @@ struct Sim1D {
     template <int VDIM, bool DIR, bool F32>
     void launch_kernels(const Params1D& q, int blocks, size_t smem, size_t post_smem, unsigned post, EvPair& ev) {
         if (q.coll_acc || q.ledger || q.bgk)
-            k_pass1d<VDIM, DIR, F32, kPassDiag><<<blocks, kThreads, smem, stream>>>(q);
+            launch_dependent(k_pass1d<VDIM, DIR, F32, kPassDiag>, blocks, kThreads, smem, q);
         else if (cfg.nmodels && q.mode == (kModeSyncMcc | kModeKickDrift | kModeDeposit))
-            k_pass1d_mcc<VDIM, DIR, F32><<<wave(kMccBlocks), kMccThreads, smem, stream>>>(q);
+            launch_dependent(k_pass1d_mcc<VDIM, DIR, F32>, wave(kMccBlocks), kMccThreads, smem, q);
         else if (cfg.nmodels)
-            k_pass1d<VDIM, DIR, F32, kPassDiag><<<blocks, kThreads, smem, stream>>>(q);
+            launch_dependent(k_pass1d<VDIM, DIR, F32, kPassDiag>, blocks, kThreads, smem, q);
         else
-            k_pass1d<VDIM, DIR, F32, kPassPlain><<<blocks, kThreads, smem, stream>>>(q);
+            launch_dependent(k_pass1d<VDIM, DIR, F32, kPassPlain>, blocks, kThreads, smem, q);
         if (timing) cudaEventRecord(ev.b, stream);
         cudaLaunchConfig_t lc = {};
         lc.gridDim = dim3(1);
         lc.blockDim = dim3(kPostThreads);
         lc.dynamicSmemBytes = post_smem;
         lc.stream = stream;
-        cudaLaunchAttribute attr[1];
+        cudaLaunchAttribute attr[2];
         attr[0].id = cudaLaunchAttributePriority;
         attr[0].val.priority = post_priority;
+        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[1].val.programmaticStreamSerializationAllowed = 1;
         lc.attrs = attr;
-        lc.numAttrs = 1;
+        lc.numAttrs = 2;
         APIC_CUDA(cudaLaunchKernelEx(&lc, k_post1d<VDIM, DIR, F32>, q, post));
     }
 

@@ -138,10 +138,11 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D 
     const unsigned mode = p.mode;
     const int nx = p.nx;
     for (int i = tid; i < nx; i += kThreads) {
-        sE[i] = (float)p.E[i];
         sLo[i] = 0u;
         sHi[i] = 0u;
     }
+    grid_wait();
+    for (int i = tid; i < nx; i += kThreads) sE[i] = (float)p.E[i];
     if (tid == 0) s_ncand = 0u;
     CandRec32* region = p.cands ? p.cands + (size_t)blockIdx.x * p.cand_per_region : nullptr;
     if (lane < kChunk32 / 32) s_mask[warp][lane] = 0u;
@@ -330,6 +331,7 @@ __global__ void __launch_bounds__(kThreads, kMinBlocks32) k_pass1d_c32(Params1D 
         }
     }
     __syncthreads();
+    grid_release();
     if (mode & kModeDeposit) {
         for (int i = tid; i < nx; i += kThreads) {
             const unsigned long long a = join64(sLo[i], sHi[i]);
@@ -366,6 +368,7 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
     __shared__ unsigned s_start[kMaxRegions + 1];  // first dense index of each region
     const int tid = threadIdx.x;
     const unsigned regions = min(p.cand_regions, (unsigned)kMaxRegions);
+    grid_wait();
     {
         // exclusive prefix sums of the region counts, 16 per thread
         using Scan = cub::BlockScan<unsigned, kCollideThreads>;
@@ -532,6 +535,7 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
         }
     }
     __syncthreads();
+    grid_release();
     if (tid < kMaxModels * kMaxChannels) {
         const unsigned c = (&s_chan[0][0])[tid];
         if (c) atomicAdd(&st->chan[0][0] + tid, (unsigned long long)c);

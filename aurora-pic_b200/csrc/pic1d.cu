@@ -1275,6 +1275,15 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
         }
     }
     grid_wait();
+    // the first survivors' counts and the particle counts of every species: one round
+    // trip for what the range tables below would load species after species
+    static_assert(kMaxSpecies == 4, "the range tables pick a species' counts by hand");
+    unsigned surv0[kMaxSpecies], count[kMaxSpecies];
+#pragma unroll
+    for (int s = 0; s < kMaxSpecies; ++s) {
+        surv0[s] = !C32 && s < p.nspecies && tid < (int)p.sp[s].nscratch ? p.sp[s].chunk_surv[tid] : 0u;
+        count[s] = s < p.nspecies ? st->n[s] : 0u;
+    }
     const double field_time = (post & kPostAdvance) ? st->time + p.dt : st->time;
     if (solve) {
 #pragma unroll 1
@@ -1304,12 +1313,14 @@ __global__ void __launch_bounds__(kPostThreads) k_post1d(Params1D p, unsigned po
 #pragma unroll 1
     for (int s = 0; s < (C32 ? 0 : p.nspecies); ++s) {
         const SpeciesDev& S = p.sp[s];
-        const unsigned nch = (st->n[s] + CHUNK - 1) / CHUNK;
+        const unsigned n = s == 0 ? count[0] : s == 1 ? count[1] : s == 2 ? count[2] : count[3];
+        const unsigned first = s == 0 ? surv0[0] : s == 1 ? surv0[1] : s == 2 ? surv0[2] : surv0[3];
+        const unsigned nch = (n + CHUNK - 1) / CHUNK;
         unsigned carry = 0;
 #pragma unroll 1
         for (unsigned b0 = 0; b0 < nch; b0 += kPostThreads) {
             const unsigned c = b0 + tid;
-            const unsigned cnt = c < nch ? S.chunk_surv[c] : 0u;
+            const unsigned cnt = c < nch ? (b0 ? S.chunk_surv[c] : first) : 0u;
             unsigned total;
             const unsigned pre = block_exclusive_sum(cnt, s_scan, total);
             if (c < nch) {

@@ -3942,12 +3942,13 @@ struct SimND {
             for (int s = 0; s < cfg.nspecies; ++s) {
                 if (since_sort[s] < species_interval[s]) continue;
                 since_sort[s] = 0;
-                if (sp[s].n) launches += fp32 ? 6 : 5;  // histogram, three scan passes, scatter (FP32: rank + gather)
+                // histogram, three scan passes, scatter (FP32: rank + gather; tiles: their items)
+                if (sp[s].n) launches += (fp32 ? 6 : 5) + (sp[s].tiled ? 1 : 0);
             }
             if (sort_mask) steps_since_sort = 0;
             for (int s = 0; s < cfg.nspecies; ++s)
                 if (sp[s].n) ++launches;
-            launches += cfg.dims == 2 ? 3 : 5;  // FFT passes
+            launches += (cfg.dims == 2 ? 3 : 5) + (walls ? 2 : 0);  // transform passes (walls: density and field too)
             if (!timing) {
                 launch_step_graph(sort_mask);
             } else {

@@ -433,7 +433,7 @@ def bench_ccp1d(args, rank, dist):
     bytes_per_pstep = 64 if prec == apic.FP64 else 40
     per_pass_ms = pass_ms / max(passes, 1)
     achieved = bytes_per_pstep * mean_n / (per_pass_ms * 1e-3) / 1e9
-    traffic = _profiled_traffic("k_pass1d_ccp1d_fp64.md" if prec == apic.FP64 else "k_pass1d_c32_ccp1d_fp32.md")
+    traffic = _profiled_traffic("k_pass1d_mcc_ccp1d_fp64.md" if prec == apic.FP64 else "k_pass1d_c32_ccp1d_fp32.md")
     sim.close()
     # the other storage form of the same discharge, device-timed the same way
     other = apic.FP32 if prec == apic.FP64 else apic.FP64
@@ -457,7 +457,7 @@ def bench_ccp1d(args, rank, dist):
                 "d2h_bytes_per_step": d2h},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
                      "frac": achieved / hbm, "traffic": traffic, "peak_kind": peak_kind,
-                     "kernel": "k_pass1d<3,true,false,false>" if prec == apic.FP64 else "k_pass1d_c32<3,true>",
+                     "kernel": "k_pass1d_mcc<3,true,false>" if prec == apic.FP64 else "k_pass1d_c32<3,true>",
                      "bytes_per_particle_step": bytes_per_pstep,
                      "pass_ms": per_pass_ms, "post_ms": post_ms / max(passes, 1)},
         "gpu_launches": 2 * args.steps,
@@ -666,10 +666,12 @@ def bench_plasma(args, rank, dist):
     # streamed once per launch, so traffic grows in proportion)
     traffic, traffic_note = None, None
     items = push_items or (4 if dims == 2 else 2)
-    run_kernel = prec == apic.FP32 and items in (2, 4)  # consecutive particles per thread (k_push32_run)
+    # consecutive particles per thread (2D, k_push32_run) or whole tiles (3D, k_push32_tile)
+    run_kernel = prec == apic.FP32 and (dims == 3 or items in (2, 4))
     if prec == apic.FP32:
         captured = {2: 4194304, 3: 16777216}[dims]
-        name = f"k_push32_run_plasma{dims}d_fp32.md" if run_kernel else f"k_push32_plasma{dims}d_fp32.md"
+        name = ("k_push32_tile_plasma3d_fp32.md" if dims == 3 else
+                "k_push32_run_plasma2d_fp32.md" if run_kernel else "k_push32_plasma2d_fp32.md")
         t = _profiled_traffic(name)
         if t:
             traffic = t * (P / 2) / captured
@@ -689,7 +691,8 @@ def bench_plasma(args, rank, dist):
                 "d2h_bytes_per_step": d2h},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": traffic, "traffic_note": traffic_note, "peak_kind": peak_kind,
-                     "kernel": (("k_push32_run" if run_kernel else "k_push32_step") if prec == apic.FP32 else "k_push")
+                     "kernel": (("k_push32_tile" if dims == 3 else "k_push32_run" if run_kernel else "k_push32_step")
+                                if prec == apic.FP32 else "k_push_run")
                      + f"<{dims}, boris, items={items}>",
                      "bytes_per_particle_step": bpp, "push_ms": per_step_push,
                      "solve_ms": solve_ms / max(nsteps, 1), "sort_ms_per_step": sort_ms / max(nsteps, 1)},

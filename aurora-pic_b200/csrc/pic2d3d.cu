@@ -64,6 +64,7 @@ struct SpeciesND {
     float dep_fixed;   // dep * rho_scale
     // runs with walls and an absorbing side: Particle::alive (null: all alive)
     uint8_t* alive[2];
+    unsigned* live_end;  // particles alive at the last sort, which moved the others behind them (null: none absorb)
     // FP64 form: Boris h = 0.5 qm dt, t = h B and s = 2 t / (1 + t^2) of a full step in the uniform B
     double bh, bt[3], bs[3];
     int index;         // species index (loss ledger row)
@@ -470,6 +471,7 @@ struct State64 {
     double* pos[3];
     double* vh[3];
     uint8_t* alive;
+    const unsigned* live_end;
 };
 
 template <int DIM, int BKIND, bool WALLS>
@@ -477,7 +479,9 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsN
     constexpr int NN = DIM == 2 ? 4 : 8;
     const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * kRunItems;
     const int lane = threadIdx.x & 31;
-    if ((blockIdx.x * kThreads + (threadIdx.x & ~31u)) * kRunItems >= S.n) return;  // whole warp past the end
+    // whole warp past the end, or past the particles that were alive at the last sort
+    const unsigned warp_first = (blockIdx.x * kThreads + (threadIdx.x & ~31u)) * kRunItems;
+    if (warp_first >= (WALLS && A.live_end ? min(S.n, *A.live_end) : S.n)) return;
     const int nx = p.n[0], ny = p.n[1];
     double x[kRunItems][3], v[kRunItems][3];
     bool live[kRunItems];
@@ -612,6 +616,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsN
     // the state back, in place
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
+        if (WALLS && !live[0] && !live[1]) break;  // nothing of an absorbed pair changed
         if (full) {
             if (a < DIM) __stcs(reinterpret_cast<double2*>(A.pos[a] + first), make_double2(x[0][a], x[1][a]));
             __stcs(reinterpret_cast<double2*>(A.vh[a] + first), make_double2(v[0][a], v[1][a]));
@@ -1634,12 +1639,19 @@ __device__ __forceinline__ unsigned bin_of(const ParamsND& p, const SpeciesND& S
     return cell_of<DIM, WALLS>(p, pos);
 }
 
+// One atomic for all lanes of a warp with the same bin: after the first sort a
+// warp holds one or two cells, and the absorbed of a run with walls are one bin,
+// whose count would otherwise take one atomic after another.
 template <int DIM, bool WALLS>
 __global__ void k_cell_hist(ParamsND p, SpeciesND S, int buf, unsigned* count) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= S.n) return;
-    const double pos[3] = {S.pos[buf][0][i], S.pos[buf][1][i], DIM == 3 ? S.pos[buf][2][i] : 0.0};
-    atomicAdd(count + bin_of<DIM, WALLS>(p, S, buf, i, pos), 1u);
+    unsigned bin = ~0u;  // no particle
+    if (i < S.n) {
+        const double pos[3] = {S.pos[buf][0][i], S.pos[buf][1][i], DIM == 3 ? S.pos[buf][2][i] : 0.0};
+        bin = bin_of<DIM, WALLS>(p, S, buf, i, pos);
+    }
+    const unsigned same = __match_any_sync(0xFFFFFFFFu, bin);
+    if (bin != ~0u && (threadIdx.x & 31) == (unsigned)__ffs(same) - 1) atomicAdd(count + bin, (unsigned)__popc(same));
 }
 
 // exclusive scan of `count` (n entries) into `offset`, three launches
@@ -1696,25 +1708,36 @@ __global__ void k_scan_blocks(unsigned* block_sums, unsigned nblocks) {
     }
 }
 
-__global__ void k_scan_add(unsigned* offset, const unsigned* block_sums, unsigned n) {
+// (last, when given, receives the offset of the last bin)
+__global__ void k_scan_add(unsigned* offset, const unsigned* block_sums, unsigned n, unsigned* last) {
     const unsigned base = blockIdx.x * kScanBlock;
     const unsigned add = block_sums[blockIdx.x];
     for (unsigned k = threadIdx.x; k < (unsigned)kScanBlock; k += kThreads)
-        if (base + k < n) offset[base + k] += add;
+        if (base + k < n) {
+            const unsigned v = offset[base + k] + add;
+            offset[base + k] = v;
+            if (last && base + k + 1 == n) *last = v;
+        }
 }
 
 template <int DIM, bool WALLS>
 __global__ void k_cell_scatter(ParamsND p, SpeciesND S, int from, unsigned* cursor) {
     const unsigned i = blockIdx.x * kThreads + threadIdx.x;
-    if (i >= S.n) return;
     const int to = from ^ 1;
+    const bool valid = i < S.n;
+    const unsigned j = valid ? i : 0;
     // loads first, stores after: the buffers may alias as far as the compiler
     // knows, so loads placed after stores would each wait for the previous store
-    const double pos[3] = {S.pos[from][0][i], S.pos[from][1][i], DIM == 3 ? S.pos[from][2][i] : 0.0};
-    const double vh[3] = {S.vh[from][0][i], S.vh[from][1][i], S.vh[from][2][i]};
-    const unsigned id = S.id[from][i];
-    const uint8_t alive = WALLS && S.alive[from] ? S.alive[from][i] : 1;
-    const unsigned o = atomicAdd(cursor + bin_of<DIM, WALLS>(p, S, from, i, pos), 1u);
+    const double pos[3] = {S.pos[from][0][j], S.pos[from][1][j], DIM == 3 ? S.pos[from][2][j] : 0.0};
+    const double vh[3] = {S.vh[from][0][j], S.vh[from][1][j], S.vh[from][2][j]};
+    const unsigned id = S.id[from][j];
+    const uint8_t alive = WALLS && S.alive[from] ? S.alive[from][j] : 1;
+    const unsigned bin = valid ? bin_of<DIM, WALLS>(p, S, from, i, pos) : ~0u;
+    const unsigned same = __match_any_sync(0xFFFFFFFFu, bin);
+    const int lane = threadIdx.x & 31, leader = __ffs(same) - 1;
+    unsigned o = valid && lane == leader ? atomicAdd(cursor + bin, (unsigned)__popc(same)) : 0u;
+    o = __shfl_sync(0xFFFFFFFFu, o, leader) + __popc(same & ((1u << lane) - 1u));
+    if (!valid) return;
     for (int a = 0; a < DIM; ++a) S.pos[to][a][o] = pos[a];
     for (int a = 0; a < 3; ++a) S.vh[to][a][o] = vh[a];
     S.id[to][o] = id;
@@ -3675,7 +3698,7 @@ struct SimND {
         if (MODE == kPushStep) {
             const unsigned g = (S.n + kRunItems * kThreads - 1) / (kRunItems * kThreads);
             const int kind = !boris ? kNoField : (p.prof_rows ? kProfileField : kUniformField);
-            State64 A{{}, {}, S.alive[b]};
+            State64 A{{}, {}, S.alive[b], S.live_end};
             for (int a = 0; a < 3; ++a) { A.pos[a] = S.pos[b][a]; A.vh[a] = S.vh[b][a]; }
             auto run = [&](auto dim, auto wall) {
                 constexpr int D = decltype(dim)::value;
@@ -3726,7 +3749,7 @@ struct SimND {
         else k_cell_hist<3, false><<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_count);
         k_scan_local<<<nb, kThreads, 0, stream>>>(cell_count, cell_offset, block_sums, nbins);
         k_scan_blocks<<<1, kThreads, 0, stream>>>(block_sums, nb);
-        k_scan_add<<<nb, kThreads, 0, stream>>>(cell_offset, block_sums, nbins);
+        k_scan_add<<<nb, kThreads, 0, stream>>>(cell_offset, block_sums, nbins, walls ? S.live_end : nullptr);
         if (fp32) {
             if (in_tiles) k_tile_count<true><<<items, kThreads, 0, stream>>>(p, S, buf[s], cell_offset, ntiles);
             else k_cell_rank32<<<blocks, kThreads, 0, stream>>>(p, S, buf[s], cell_offset);
@@ -3773,6 +3796,7 @@ struct SimND {
                 APIC_ERR_CAPACITY);
         SpeciesND& S = sp[s];
         if (S.alive[buf[s]] && n) APIC_CUDA(cudaMemsetAsync(S.alive[buf[s]], 1, n, stream));
+        if (S.live_end) APIC_CUDA(cudaMemsetAsync(S.live_end, 0xFF, sizeof(unsigned), stream));  // not sorted yet
         const int b = buf[s];
         const size_t bytes = n * sizeof(double);
         for (int a = 0; a < cfg.dims; ++a)
@@ -3833,6 +3857,10 @@ struct SimND {
         for (int k = 0; k < 2 * dims; ++k) absorbing = absorbing || p.pbc[k] == 1;
         for (int s = 0; s < c.nspecies; ++s)
             for (int b = 0; b < 2; ++b) sp[s].alive[b] = absorbing ? dalloc<uint8_t>(c.species[s].capacity) : nullptr;
+        for (int s = 0; s < c.nspecies; ++s) {
+            sp[s].live_end = absorbing ? dalloc<unsigned>(1) : nullptr;
+            if (absorbing) APIC_CUDA(cudaMemsetAsync(sp[s].live_end, 0xFF, sizeof(unsigned), stream));
+        }
         solver.F.dims = dims;
         solver.F.rho_acc = dalloc<unsigned long long>(N);
         solver.F.rho = dalloc<double>(N);

@@ -314,3 +314,33 @@ def test_periodic_solve_of_every_line_length(n):
     assert rel_max(phi.reshape(shape), np.fft.ifftn(ph).real) < TOL
     for a in range(dims):
         assert rel_max(E[a].reshape(shape), np.fft.ifftn(-1j * k[a] * ph).real) < TOL
+
+
+@pytest.mark.parametrize("dims", [2, 3])
+def test_walls_until_most_particles_are_absorbed(dims):
+    """The push skips the particles that a sort moved behind the living; counts, flags and
+    positions stay those of runs that are never sorted; a second load starts over."""
+    n, length = ((9, 17), (4.0, 2.0)) if dims == 2 else ((9, 9, 17), (4.0, 2.0, 3.0))
+    wall, pb = (1,) * dims, (1,) * (2 * dims)
+    sims = []
+    for sort in (3, 10 ** 6):
+        dev = apic.SimulationND(apic.config_nd(dims=dims, n=n, length=length, dt=0.1, magnetic_field=(0.0, 0.0, 0.2),
+                                               sort_interval=sort, species=[(q, m, w, 3001) for q, m, w in SPECIES],
+                                               walls=(wall, [0.0] * 4 if dims == 2 else None, pb)))
+        sims.append(dev)
+    for attempt in range(2):
+        for dev in sims:
+            for k in range(2):
+                pos, v = _particles(3001, dims, length, 40 + k + 10 * attempt)
+                dev.load(k, pos, v)
+            dev.initialize()
+        for steps in (4, 30, 40):
+            for dev in sims:
+                dev.step(steps)
+            for k in range(2):
+                assert np.array_equal(sims[0].alive(k), sims[1].alive(k))
+                assert np.array_equal(sims[0].boundary_losses(k), sims[1].boundary_losses(k))
+                for x, y in zip(sims[0].particles(k)[::2], sims[1].particles(k)[::2]):
+                    assert np.array_equal(x, y)
+            assert np.array_equal(sims[0].fields()[0], sims[1].fields()[0])
+        assert sims[0].alive(0).mean() < 0.5

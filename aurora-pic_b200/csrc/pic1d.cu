@@ -225,7 +225,8 @@ __device__ __forceinline__ Cic cic_periodic(double x, const Params1D& p) {
     const double xp = wrap_periodic(x, p.L);
     const double g = cells_of(xp, p.dx, p.rdx);
     const int i = (int)floor(g);
-    // i % nx and (i + 1) % nx; 0 <= i <= nx after the wrap (a NaN converts to 0)
+    // i % nx and (i + 1) % nx; 0 <= i <= nx after the wrap (a NaN converts to
+    // INT_MIN and lands in cell 0 through the unsigned compare)
     Cic c;
     const double f = g - (double)i;
     c.i0 = (unsigned)i < (unsigned)p.nx ? i : 0;

@@ -166,8 +166,8 @@ struct Axis {
 
 // One axis of the periodic CIC stencil, src/Mesh2D.cpp:96-114, src/FieldSolver.cpp:936-960.
 // The wrap leaves 0 <= x <= L, so the cell is at most n and i % n is a
-// compare (a NaN converts to cell 0); 64-bit remainders here were most of the
-// FP64 push's instructions.
+// compare (a NaN, which converts to INT_MIN, lands in cell 0 through it); 64-bit
+// remainders here were most of the FP64 push's instructions.
 __device__ __forceinline__ Axis axis(double x, double L, double d, double rd, int n) {
     const double xp = wrap_periodic(x, L);
     const double g = cells_of(xp, d, rd);
@@ -181,12 +181,13 @@ __device__ __forceinline__ Axis axis(double x, double L, double d, double rd, in
 
 // One axis of the CIC stencil on a wall axis: clamp into [0, L], cell
 // min(floor, n - 2), fraction clamped to [0, 1], src/Mesh2D.cpp:96-129,
-// src/FieldSolver.cpp:926-960
+// src/FieldSolver.cpp:926-960.  A NaN position lands on the lower wall: the
+// conversion of a NaN to int is INT_MIN, which no index may come from.
 __device__ __forceinline__ Axis axis_wall(double x, double L, double d, double rd, int n) {
-    const double c = x < 0.0 ? 0.0 : (L < x ? L : x);
+    const double c = !(x >= 0.0) ? 0.0 : (L < x ? L : x);
     const double g = cells_of(c, d, rd);
-    int i = (int)floor(g);  // (a NaN converts to cell 0)
-    if (i > n - 2) i = n - 2;
+    int i = (int)floor(g);
+    if ((unsigned)i > (unsigned)(n - 2)) i = n - 2;
     double f = g - (double)i;
     f = f < 0.0 ? 0.0 : (f > 1.0 ? 1.0 : f);
     Axis a;

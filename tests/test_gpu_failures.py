@@ -74,6 +74,42 @@ def test_non_finite_velocity_loaded_from_the_host(precision):
     dev.close()
 
 
+@pytest.mark.parametrize("what", ["position", "velocity"])
+@pytest.mark.parametrize("n,wall", [((9, 8), (1, 0)), ((8, 9), (0, 1)), ((9, 17), (1, 1)), ((5, 9, 17), (1, 1, 1))])
+def test_non_finite_coordinate_between_walls(n, wall, what):
+    """A NaN on a wall axis (reflecting on both sides, so that nothing absorbs it)
+    counts at the lower wall: every index stays inside the mesh, the charge stays whole
+    and the other particles stay finite, sorted every step."""
+    dims, count = len(n), 700
+    length = (4.0, 2.0, 3.0)[:dims]
+    axis = wall.index(1)
+    rng = np.random.default_rng(5)
+    dev = apic.SimulationND(apic.config_nd(
+        dims=dims, n=n, length=length, dt=0.1, sort_interval=1, species=[(-1.0, 1.0, 0.05, count)],
+        walls=(wall, [0.0] * 4 if dims == 2 else None, [2 if wall[k // 2] else 3 for k in range(2 * dims)])))
+    pos = np.stack([rng.uniform(0.0, L, count) for L in length])
+    v = rng.standard_normal((3, count))
+    (pos if what == "position" else v)[axis, 17] = np.nan
+    dev.load(0, pos, v)
+    dev.initialize()
+    # node volumes: half cells at the walls
+    volume = np.ones(())
+    for a in range(dims):
+        w = np.full(n[a], length[a] / (n[a] - wall[a]))
+        if wall[a]:
+            w[[0, -1]] *= 0.5
+        volume = np.multiply.outer(w, volume)
+    for _ in range(4):
+        charge = np.sum(dev.fields()[0] * volume.ravel())
+        assert abs(charge + 0.05 * count) < 1e-9 * 0.05 * count
+        dev.step(1)
+    x, _, vh = dev.particles(0)
+    others = np.arange(count) != 17
+    assert np.isfinite(x[:dims, others]).all() and np.isfinite(vh[:, others]).all()
+    assert np.isnan(x[axis, 17])
+    dev.close()
+
+
 def test_bounded_wait_gives_up_and_a_later_wait_completes():
     """A wait limit far below the time of the enqueued steps ends the
     synchronising call with APIC_ERR_TIMEOUT; the work itself runs on, and a

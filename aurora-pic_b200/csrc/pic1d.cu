@@ -195,7 +195,9 @@ struct Params1D {
 // Programmatic launches: a step's kernels are launched while the one before them
 // is finishing (grid_release, at its tail), set up what does not depend on it, and wait
 // for its completion and its writes (grid_wait) before they read anything
-// of the run.
+// of the run.  So a kernel here is resident while another one writes: what the
+// kernels of a step write is read by ordinary loads, never by non-coherent ones (__ldg,
+// const __restrict__), which may be moved above the wait.
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
@@ -287,7 +289,7 @@ __device__ __forceinline__ unsigned range_of(const unsigned* lstart, unsigned nr
     unsigned lo = 0, hi = nr;
     while (hi - lo > 1) {
         const unsigned mid = (lo + hi) >> 1;
-        if (__ldg(lstart + mid) <= idx) lo = mid; else hi = mid;
+        if (lstart[mid] <= idx) lo = mid; else hi = mid;
     }
     return lo;
 }
@@ -297,12 +299,12 @@ __device__ __forceinline__ unsigned range_of(const unsigned* lstart, unsigned nr
 __device__ __forceinline__ unsigned physical_slot_from(const unsigned* lstart, const unsigned* start, unsigned nr,
                                                        unsigned r0, unsigned idx) {
     unsigned r = r0;
-    while (r + 1 < nr && __ldg(lstart + r + 1) <= idx) ++r;
-    return __ldg(start + r) + (idx - __ldg(lstart + r));
+    while (r + 1 < nr && lstart[r + 1] <= idx) ++r;
+    return start[r] + (idx - lstart[r]);
 }
 
-// The 32 ranges a warp needs for a tile, one per lane.  A range holds at most
-// kTile particles (or is the only one), so range r starts at or before particle
+// The 32 ranges a warp needs for a tile, one per lane.  Every range but the
+// last holds at most kTile particles, so range r starts at or before particle
 // r kTile and the tile's first range is at or after base / kTile: usually that
 // one or the next, since a step's losses are few.  One coalesced load and a
 // ballot replace the binary search's chain of dependent loads (1 M particles: ten
@@ -329,8 +331,8 @@ struct RangeWindow {
     }
     __device__ __forceinline__ void load(const unsigned* lstart, const unsigned* rstart, unsigned nr, int lane) {
         const bool in = r0 + lane < nr;
-        start = in ? __ldg(lstart + r0 + lane) : 0xFFFFFFFFu;
-        delta = in ? __ldg(rstart + r0 + lane) - start : 0u;
+        start = in ? lstart[r0 + lane] : 0xFFFFFFFFu;
+        delta = in ? rstart[r0 + lane] - start : 0u;
     }
     // slot of particle idx of the tile (all lanes call; `live`: this lane's particle exists)
     __device__ __forceinline__ unsigned slot(const unsigned* lstart, const unsigned* rstart, unsigned nr, unsigned idx,

@@ -378,7 +378,7 @@ __global__ void __launch_bounds__(kCollideThreads) k_collide1d_c32(Params1D p) {
 #pragma unroll
         for (int k = 0; k < PER; ++k) {
             const unsigned r = tid * PER + k;
-            c[k] = r < regions ? __ldg(p.cand_count + r) : 0u;
+            c[k] = r < regions ? p.cand_count[r] : 0u;
         }
         unsigned total;
         Scan(tmp).ExclusiveSum(c, o, total);

@@ -31,6 +31,19 @@ def test_library_exports_every_declared_symbol():
     assert not missing, missing
 
 
+def test_overlapping_1d_kernels_load_coherently():
+    """The kernels of a 1D step are resident while the one before them still writes
+    (programmatic launches), so the sources that hold them use no non-coherent load:
+    none by intrinsic or PTX, and no kernel of a step has a const __restrict__ argument."""
+    for name in ("pic1d.cu", "pic1d_c32.cuh"):
+        text = open(os.path.join(ROOT, "aurora-pic_b200", "csrc", name)).read()
+        code = re.sub(r"//[^\n]*|/\*.*?\*/", "", text, flags=re.S)
+        assert "grid_wait" in code
+        assert not re.findall(r"__ldg|ld\.global\.nc", code), name
+        for args in re.findall(r"__global__[^(]*(?:__launch_bounds__\([^{;]*?\)\s*)?k_\w+\(([^)]*)\)", code):
+            assert not (args.startswith("Params1D") and "__restrict__" in args), args
+
+
 def test_status_strings_and_version():
     lib = apic.lib()
     assert b"sm_100a" in lib.apic_version()

@@ -922,6 +922,14 @@ __global__ void __launch_bounds__(kThreads) k_push32_step(ParamsND p, SpeciesND 
     }
 }
 
+// A particle with an infinite or NaN velocity keeps its cell and has a NaN
+// offset: it deposits nothing (the rounding by an added 2^23 would turn a NaN weight
+// into 106 particles' charge, and break the bounds of the box sums' carries).
+template <int DIM>
+__device__ __forceinline__ bool offsets_finite(const float f[3]) {
+    return (DIM == 3 ? f[0] + f[1] + f[2] : f[0] + f[1]) < 4.0f;  // each in [0, 1), or NaN
+}
+
 // The step push of the FP32 form with ITEMS consecutive particles per thread
 // (loaded and stored as vectors).  Particles are sorted by cell, so a thread's
 // particles mostly share a cell: the field at the cell's nodes is fetched once
@@ -1144,6 +1152,7 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         }
         // (units of 2^-23 to nearest even: adding 2^23 leaves the integer in the low
         // bits of the float; the scale, a power of two, is exact on any factor)
+        if (!offsets_finite<DIM>(f)) continue;
         const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale}, uy[2] = {1.0f - f[1], f[1]};
         const float uz[2] = {DIM == 3 ? 1.0f - f[2] : 1.0f, DIM == 3 ? f[2] : 0.0f};
 #pragma unroll
@@ -1433,6 +1442,7 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks) k_push32_tile(ParamsND 
 #pragma unroll
                 for (int j = 0; j < 8; ++j) w[j] = 0u;
             }
+            if (!offsets_finite<3>(f)) continue;
             // the weights in units of 2^-23, to nearest even: adding 2^23 leaves the
             // integer in the low bits of the float (a weight is at most 2^23 units);
             // the scale, a power of two, is exact on any factor

@@ -110,6 +110,32 @@ def test_non_finite_coordinate_between_walls(n, wall, what):
     dev.close()
 
 
+@pytest.mark.parametrize("bad", [np.inf, np.nan])
+@pytest.mark.parametrize("n,items", [((16, 32), 1), ((16, 32), 2), ((16, 32), 4), ((8, 8, 4), 1), ((8, 8, 4), 2),
+                                     ((8, 8, 4), 4), ((8, 16, 8), 0)])
+def test_non_finite_particle_of_the_fp32_form(n, items, bad):
+    """A particle of non-finite velocity deposits nothing from its first step on, in every
+    kernel of the FP32 push (the last mesh goes through its tiles); the others go on."""
+    dims, count = len(n), 8 * int(np.prod(n)) + 1
+    rng = np.random.default_rng(3)
+    dev = apic.SimulationND(apic.config_nd(
+        dims=dims, n=n, length=[float(k) for k in n], dt=0.1, magnetic_field=(0.1, 0.0, 0.2), precision=apic.FP32,
+        sort_interval=2, push_items=items, species=[(-1.0, 1.0, 0.01, count)]))
+    pos = np.stack([rng.uniform(0.0, k, count) for k in n])
+    v = rng.standard_normal((3, count))
+    v[0, 100] = bad
+    dev.load(0, pos, v)
+    dev.initialize()
+    for _ in range(4):
+        dev.step(1)
+        charge = dev.fields()[0].sum() / -0.01  # in particles; 2^dims weights of 2^-23 units each
+        assert abs(charge - (count - 1)) < count * 2 ** dims * 2.0 ** -22
+    x, _, vh = dev.particles(0)
+    others = np.arange(count) != 100
+    assert np.isfinite(x[:dims, others]).all() and np.isfinite(vh[:, others]).all()
+    dev.close()
+
+
 def test_bounded_wait_gives_up_and_a_later_wait_completes():
     """A wait limit far below the time of the enqueued steps ends the
     synchronising call with APIC_ERR_TIMEOUT; the work itself runs on, and a

@@ -76,9 +76,9 @@ __device__ inline int upper_bound_indexed(const MccChannelDev& c, double energy)
     const TableIndex& ix = c.index;
     int lo = 0, hi = c.rows;
     if (ix.nbins > 0) {
-        // the single-precision log is good to 1e-5 bins' widths inside float's
-        // range; one more bin of slack on each side covers it, and the search
-        // below ends at the same row
+        // the single-precision log is good to 2e-5 inside float's range, a fifth of
+        // the narrowest bin (build_index); one more bin of slack on each side
+        // covers it, and the search below ends at the same row
         const bool in_float = energy > 1e-36 && energy < 1e36;
         const double l2 = in_float ? (double)__log2f((float)energy) : log2(energy);
         const double t = (l2 - ix.lmin) * ix.inv_width;

@@ -85,7 +85,7 @@ __device__ inline int upper_bound32(const MccChannel32& c, float energy) {
     if (c.nbins > 0) {
         const float t = (__log2f(energy) - c.lmin) * c.inv_width;
         const int b = !(t >= -1.0f) ? -1 : (t > (float)c.nbins ? c.nbins : (int)floorf(t));
-        // one bin of slack on each side covers the fast log's error
+        // one bin of slack on each side covers the fast log's error (build_index)
         lo = b >= 2 ? (int)__ldg(c.first_gt + (b - 2)) : 0;
         hi = b + 3 <= c.nbins ? (int)__ldg(c.first_gt + (b + 3)) : c.rows;
     }

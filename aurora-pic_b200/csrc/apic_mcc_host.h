@@ -117,7 +117,12 @@ inline double safe_speed(const apic_mcc_model& m, double particle_mass, double n
 }
 
 
-// Bracket index over log2(energy) for a strictly increasing table.
+// Bracket index over log2(energy) for a strictly increasing table.  The device
+// finds the bin with a single-precision log2, whose error is absolute: 2 ulp of values
+// up to 120 and the roundings of its argument and of lmin, below 2e-5 in all.  Bins at least
+// kMinBinWidth wide keep that within a fifth of a bin (the lookup allows one);
+// a table that spans less has no index and is searched whole.
+constexpr double kMinBinWidth = 1e-4;
 inline TableIndex build_index(const double* e, size_t rows, DeviceArena& arena) {
     TableIndex ix{};
     size_t first_pos = 0;
@@ -126,7 +131,9 @@ inline TableIndex build_index(const double* e, size_t rows, DeviceArena& arena) 
     const double lmin = std::log2(e[first_pos]);
     const double lmax = std::log2(e[rows - 1]);
     if (!(lmax > lmin)) return ix;
-    const int nbins = (int)std::min<size_t>(std::max<size_t>(rows, 256), 8192);
+    const int nbins = (int)std::min<double>(std::min<size_t>(std::max<size_t>(rows, 256), 8192),
+                                            (lmax - lmin) / kMinBinWidth);
+    if (nbins < 1) return ix;
     std::vector<unsigned> first(nbins + 1);
     for (int b = 0; b <= nbins; ++b) {
         const double edge = std::exp2(lmin + (lmax - lmin) * (double)b / (double)nbins);

@@ -344,3 +344,70 @@ def test_walls_until_most_particles_are_absorbed(dims):
                     assert np.array_equal(x, y)
             assert np.array_equal(sims[0].fields()[0], sims[1].fields()[0])
         assert sims[0].alive(0).mean() < 0.5
+
+
+def _narrow_table(centre_ev, span, rows, seed):
+    """Cross sections that jump between 0 and 1 from row to row of a narrow table."""
+    from apic import workloads as W
+    e = centre_ev * W.E_CHARGE * np.linspace(1.0, 1.0 + span, rows)
+    sigma = 1e-20 * np.random.default_rng(seed).integers(0, 2, rows)
+    density, vmax = 1e21, np.sqrt(2.0 * e[-1] / W.M_E)
+    return e, sigma, density, 1.001 * density * 1e-20 * vmax
+
+
+@pytest.mark.parametrize("centre_ev,span,rows", [(11.5, 4.3e-4, 256), (11.5, 4.3e-4, 8192), (1000.0, 0.01, 8192),
+                                                 (11.5, 1e-6, 3), (1.0, 5.0, 64)])
+def test_collisions_on_a_narrow_table(centre_ev, span, rows):
+    """A resonance of a few meV: the bracket of every energy is the oracle's, however fine the
+    rows are against the single-precision log of the bracket index."""
+    from apic import workloads as W
+    e, sigma, density, numax = _narrow_table(centre_ev, span, rows, 5)
+    rng = np.random.default_rng(6)
+    n, dt = 3000, 1.5 / numax
+    speed = np.sqrt(2.0 * (e[0] + (e[-1] - e[0]) * rng.uniform(0.0, 1.0, n)) / W.M_E)
+    v = rng.standard_normal((n, 3))
+    v *= (speed / np.linalg.norm(v, axis=1))[:, None]
+    tabs, keep = apic.Tables(), po.TableSet()
+    model = apic.mcc_model(0, [tabs.channel(W.ELASTIC, e, sigma)], density, numax)
+    got, stats = apic.collide3(model, W.M_E, v, dt, seed=(7 << 32) | 9, step=3, stream=0)
+    col = (po.C.c_byte * 8192)()
+    om = po.make_model(0, [keep.channel(W.ELASTIC, e, sigma)], density, numax)
+    assert po.oracle().ora_collider_init(col, po.C.byref(om), W.M_E) == 0
+    hits = 0
+    for i in range(n):
+        r, st = po.Rng(), po.CollideStats()
+        r.kind, r.key[0], r.key[1] = 1, 9, 7
+        r.ctr[0], r.ctr[1], r.ctr[2] = i, 3, 0
+        w = np.ascontiguousarray(v[i])
+        assert po.oracle().ora_collide3(col, po.dptr(w), dt, po.C.byref(r), po.C.byref(st)) == 0
+        assert stats[i].candidates == st.candidates and stats[i].null_collisions == st.null_collisions
+        assert stats[i].channel_collisions[0] == st.channel_collisions[0]
+        assert rel_max(got[i], w) < TOL
+        hits += st.channel_collisions[0]
+    assert hits > n // 4
+
+
+def test_fp32_collisions_on_a_narrow_table():
+    """The FP32 form on 8192 rows within 1 %: no rate above the majorant (a wrong row
+    extrapolates past it), and the accepted collisions of the table's mean."""
+    from apic import workloads as W
+    e, sigma, density, numax = _narrow_table(1000.0, 0.01, 8192, 5)
+    rng = np.random.default_rng(6)
+    n, p = 200_000, 0.1
+    energy = e[0] + (e[-1] - e[0]) * rng.uniform(0.0, 1.0, n)
+    v = rng.standard_normal((3, n))
+    v *= np.sqrt(2.0 * energy / W.M_E) / np.linalg.norm(v, axis=0)
+    tabs = apic.Tables()
+    model = apic.mcc_model(0, [tabs.channel(W.ELASTIC, e, sigma)], density, numax)
+    dev = apic.Simulation1D(apic.config1d(boundary=apic.DIRICHLET, velocity_dimensions=3, units=apic.SI, nx=65, length=1.0,
+                                          dt=p / numax, species=[(-W.E_CHARGE, W.M_E, 1e-3, n)], models=[model],
+                                          precision=apic.FP32), tabs)
+    dev.load(0, rng.uniform(0.4, 0.6, n), v[0], None, v[1], v[2])
+    dev.initialize()
+    dev.step(1)
+    dev.synchronize()
+    t = dev.collision_totals()
+    rate = p * np.interp(energy, e, sigma) * np.sqrt(2.0 * energy / W.M_E) * density / numax
+    assert abs(t.candidates - n * p) < 5 * np.sqrt(n * p)
+    assert abs(t.channel_collisions[0][0] - rate.sum()) < 5 * np.sqrt(rate.sum())
+    dev.close()

@@ -3808,15 +3808,21 @@ struct SimND {
         APIC_CUDA(cudaGetLastError());
     }
 
+    // a species' n particles are about to be loaded: none absorbed, not sorted yet
+    void all_alive(int s, size_t n) {
+        const SpeciesND& S = sp[s];
+        if (S.alive[buf[s]] && n) APIC_CUDA(cudaMemsetAsync(S.alive[buf[s]], 1, n, stream));
+        if (S.live_end) APIC_CUDA(cudaMemsetAsync(S.live_end, 0xFF, sizeof(unsigned), stream));
+    }
+
     void load(int s, size_t n, const double* pos, const double* v, const double* vh) {
         require(s >= 0 && s < cfg.nspecies, "species index out of range");
         require(pos && v, "positions and velocities are required");
         require(n <= cfg.species[s].capacity, "initial particle count exceeds max_particles_per_species",
                 APIC_ERR_CAPACITY);
         SpeciesND& S = sp[s];
-        if (S.alive[buf[s]] && n) APIC_CUDA(cudaMemsetAsync(S.alive[buf[s]], 1, n, stream));
-        if (S.live_end) APIC_CUDA(cudaMemsetAsync(S.live_end, 0xFF, sizeof(unsigned), stream));  // not sorted yet
         const int b = buf[s];
+        all_alive(s, n);
         const size_t bytes = n * sizeof(double);
         for (int a = 0; a < cfg.dims; ++a)
             APIC_CUDA(cudaMemcpyAsync(S.pos[b][a], pos + a * n, bytes, cudaMemcpyHostToDevice, stream));
@@ -3842,7 +3848,7 @@ struct SimND {
         require(std::isfinite(vt) && vt >= 0 && std::isfinite(drift) && std::isfinite(amp), "invalid loading parameters");
         SpeciesND& S = sp[s];
         const unsigned blocks = (unsigned)((n + kThreads - 1) / kThreads);
-        if (S.live_end) APIC_CUDA(cudaMemsetAsync(S.live_end, 0xFF, sizeof(unsigned), stream));  // not sorted yet
+        all_alive(s, n);
         if (n) k_load_maxwellian<<<blocks, kThreads, 0, stream>>>(S, buf[s], cfg.dims, (unsigned)n, seed, p.L[0],
                                                                    p.L[1], p.L[2], vt, drift, axis, amp);
         APIC_CUDA(cudaGetLastError());

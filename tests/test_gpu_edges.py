@@ -346,6 +346,39 @@ def test_walls_until_most_particles_are_absorbed(dims):
         assert sims[0].alive(0).mean() < 0.5
 
 
+@pytest.mark.parametrize("dims", [2, 3])
+def test_walls_loaded_on_the_device(dims):
+    """A species loaded on the device between absorbing walls is alive, also when it replaces
+    one that was sorted and absorbed: the same run as its read-back loaded from the host."""
+    n, length = ((9, 17), (4.0, 2.0)) if dims == 2 else ((9, 9, 17), (4.0, 2.0, 3.0))
+    count = 3001
+    cfg = lambda: apic.config_nd(dims=dims, n=n, length=length, dt=0.1, sort_interval=3,
+                                 species=[(q, m, w, count) for q, m, w in SPECIES],
+                                 walls=((1,) * dims, [0.0] * 4 if dims == 2 else None, (1,) * (2 * dims)))
+    dev = apic.SimulationND(cfg())
+    before = np.zeros((2, 2 * dims), np.int64)
+    for attempt in range(2):
+        host = apic.SimulationND(cfg())
+        for k in range(2):
+            dev.load_maxwellian(k, count, 11 + k + 10 * attempt, 1.0)
+            assert dev.alive(k).all()
+            pos, v, vh = dev.particles(k)
+            host.load(k, pos, v, vh)
+        for sim in (dev, host):
+            sim.initialize()
+        for steps in (0, 1, 40):
+            for sim in (dev, host):
+                sim.step(steps)
+            for k in range(2):
+                assert np.array_equal(dev.alive(k), host.alive(k))
+                assert np.array_equal(dev.boundary_losses(k).astype(np.int64) - before[k], host.boundary_losses(k))
+                for x, y in zip(dev.particles(k)[::2], host.particles(k)[::2]):
+                    assert np.array_equal(x, y)
+            assert np.array_equal(dev.fields()[0], host.fields()[0])
+        assert 0.0 < dev.alive(0).mean() < 0.7
+        before = np.array([dev.boundary_losses(k) for k in range(2)], np.int64)
+
+
 def _narrow_table(centre_ev, span, rows, seed):
     """Cross sections that jump between 0 and 1 from row to row of a narrow table."""
     from apic import workloads as W

@@ -51,7 +51,7 @@ struct SpeciesND {
     double* pos[2][3];
     double* vh[2][3];
     unsigned* id[2];
-    double* v[3];
+    double* v[3];  // runs with walls: in load order (an absorbed particle keeps its last v through sorts)
     // FP32 form: packed cell (10 bits per axis), in-cell offsets in [0, 1) and
     // float velocities; the FP64 arrays above then only stage loads/read-backs
     unsigned* cell[2];
@@ -404,8 +404,9 @@ __global__ void __launch_bounds__(kThreads) k_push(ParamsND p, SpeciesND S, int 
     }
     double e[3];
     gather<DIM, WALLS>(p, pos, e);
+    const unsigned vi = WALLS && (MODE == kPushInitHalf || MODE == kPushSync) ? S.id[buf][j] : j;
     if (MODE == kPushInitHalf) {
-        double v[3] = {S.v[0][i], S.v[1][i], S.v[2][i]};
+        double v[3] = {S.v[0][vi], S.v[1][vi], S.v[2][vi]};
         if (BORIS) {
             double Bp[3];
             field_b(p, pos, Bp);
@@ -427,7 +428,7 @@ __global__ void __launch_bounds__(kThreads) k_push(ParamsND p, SpeciesND S, int 
             // synchronize_leapfrog, src/Pusher.cpp:131-135, :176-180
             for (int a = 0; a < DIM; ++a) vh[a] = vh[a] + 0.5 * S.qm * e[a] * p.dt;
         }
-        for (int a = 0; a < 3; ++a) S.v[a][i] = vh[a];
+        for (int a = 0; a < 3; ++a) S.v[a][vi] = vh[a];
         return;
     }
 }
@@ -2346,8 +2347,8 @@ constexpr size_t reg_smem(int mode) {
 // kinetic energy of v per species and field energy / charge_l1 of the grid;
 // per-block partials, the last block adds them in block order.
 constexpr int kSampleBlocks = 148;
-__global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, const uint8_t* alive, int dims, double* partial, unsigned* done,
-                                                   double* out, const double* E, const double* rho,
+__global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, const uint8_t* alive, const unsigned* id, int dims,
+                                                   double* partial, unsigned* done, double* out, const double* E, const double* rho,
                                                    long long N, double half_eps_vol, double vol, int species,
                                                    int last_species, int wall_x, int wall_y, int wall_z, int nx,
                                                    int ny, int nz) {
@@ -2356,8 +2357,10 @@ __global__ void __launch_bounds__(256) k_sample_nd(SpeciesND S, const uint8_t* a
     const int tid = threadIdx.x;
     double ke = 0.0, fe = 0.0, l1 = 0.0;
     for (unsigned i = blockIdx.x * 256 + tid; i < S.n; i += gridDim.x * 256)
-        if (!alive || alive[i])
-            ke += S.hmw * (S.v[0][i] * S.v[0][i] + S.v[1][i] * S.v[1][i] + S.v[2][i] * S.v[2][i]);
+        if (!alive || alive[i]) {
+            const unsigned k = id ? id[i] : i;
+            ke += S.hmw * (S.v[0][k] * S.v[0][k] + S.v[1][k] * S.v[1][k] + S.v[2][k] * S.v[2][k]);
+        }
     if (last_species) {
         for (long long g = blockIdx.x * 256 + tid; g < N; g += gridDim.x * 256) {
             double e2;
@@ -4084,7 +4087,12 @@ struct SimND {
         for (int a = 0; a < cfg.dims; ++a) fetch(S.pos[b][a], pos ? pos + a * n : nullptr, scratch[0]);
         if (pos && cfg.dims == 2) std::memset(pos + 2 * n, 0, n * sizeof(double));
         for (int a = 0; a < 3; ++a) fetch(S.vh[b][a], vh ? vh + a * n : nullptr, scratch[0]);
-        for (int a = 0; a < 3; ++a) fetch(S.v[a], v ? v + a * n : nullptr, scratch[0]);
+        if (walls && v) {  // in load order already
+            for (int a = 0; a < 3 && n; ++a)
+                APIC_CUDA(cudaMemcpyAsync(v + a * n, S.v[a], n * sizeof(double), cudaMemcpyDeviceToHost, stream));
+        } else {
+            for (int a = 0; a < 3; ++a) fetch(S.v[a], v ? v + a * n : nullptr, scratch[0]);
+        }
         sync();
         return n;
     }
@@ -4146,8 +4154,8 @@ struct SimND {
         if (cfg.dims == 2) vol *= (cfg.out_of_plane_depth == 0.0 ? 1.0 : cfg.out_of_plane_depth);
         for (int s = 0; s < cfg.nspecies; ++s) {
             if (initialized) launch_push<kPushSync>(s);
-            k_sample_nd<<<kSampleBlocks, 256, 0, stream>>>(sp[s], sp[s].alive[buf[s]], cfg.dims, sample_partial, sample_done, sample_out,
-                                                           solver.F.E, solver.F.rho, (long long)ncells,
+            k_sample_nd<<<kSampleBlocks, 256, 0, stream>>>(sp[s], sp[s].alive[buf[s]], walls ? sp[s].id[buf[s]] : nullptr,
+                                                           cfg.dims, sample_partial, sample_done, sample_out, solver.F.E, solver.F.rho, (long long)ncells,
                                                            0.5 * p.eps * vol, vol, s, s == cfg.nspecies - 1,
                                                            p.wall[0], p.wall[1], p.wall[2], p.n[0], p.n[1], p.n[2]);
             APIC_CUDA(cudaGetLastError());

@@ -379,6 +379,40 @@ def test_walls_loaded_on_the_device(dims):
         before = np.array([dev.boundary_losses(k) for k in range(2)], np.int64)
 
 
+@pytest.mark.parametrize("n,wall", [((9, 8), (1, 0)), ((9, 17), (1, 1)), ((9, 9, 17), (1, 1, 1))])
+def test_velocities_of_absorbed_particles(n, wall):
+    """v is read in load order: an absorbed particle keeps the v of the last read before its loss
+    and nobody else's, however often the run was sorted; kinetic energy and a second
+    initialize() take the same v."""
+    dims, count = len(n), 2001
+    length = (4.0, 2.0, 3.0)[:dims]
+    sims = [apic.SimulationND(apic.config_nd(
+        dims=dims, n=n, length=length, dt=0.1, magnetic_field=(0.0, 0.1, 0.2), sort_interval=sort,
+        species=[(q, m, w, count) for q, m, w in SPECIES],
+        walls=(wall, [0.0] * 4 if dims == 2 else None, [1 if wall[k // 2] else 3 for k in range(2 * dims)])))
+        for sort in (2, 10 ** 6)]
+    for dev in sims:
+        for k in range(2):
+            dev.load(k, *_particles(count, dims, length, 60 + k))
+        dev.initialize()
+    last = [None, None]
+    for steps in (1, 5, 5, -1, 7, 20):
+        for dev in sims:
+            dev.step(steps) if steps > 0 else dev.initialize()
+        for k in range(2):
+            a, b = (dev.particles(k) for dev in sims)
+            for x, y in zip(a, b):
+                assert np.array_equal(x, y)
+            if last[k] is not None:
+                dead = last[k][0] == 0
+                assert np.array_equal(a[1][:, dead], last[k][1][:, dead])
+            last[k] = sims[0].alive(k), a[1]
+        assert 0 < (last[0][0] == 0).sum() < count
+        e = [dev.sample() for dev in sims]
+        for k in range(2):
+            assert abs(e[0].kinetic_by_species[k] - e[1].kinetic_by_species[k]) < TOL * e[1].kinetic_by_species[k]
+
+
 def _narrow_table(centre_ev, span, rows, seed):
     """Cross sections that jump between 0 and 1 from row to row of a narrow table."""
     from apic import workloads as W

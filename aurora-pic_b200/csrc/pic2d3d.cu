@@ -3990,10 +3990,13 @@ struct SimND {
             }
     }
 
-    // Runs with walls of this many particles a node stay in load order: their mesh is small
-    // enough for the caches, and sorted warps commit to the same few nodes at once (60 x 64
-    // nodes: 515 a node, 415 -> 398 us a step; 286 a node, 189 -> 157;
-    // 104 a node, sorted is faster, 64 against 74 without the sort and its push).
+    // 2D runs with walls of this many particles a node stay in load order: a sorted warp's
+    // particles, and its neighbours', commit to the same few nodes, and the more of them share a
+    // node the longer its atomics queue, while particles in load order spread over the mesh,
+    // which L2 holds.  us a step, load order against sorted every 16 steps, both species: 260 a
+    // node on 100 x 128 nodes 341 / 430, 129 x 129 406 / 529, 250 x 256 1225 / 1660, 500 x 512
+    // 4649 / 5608; 520 a node on 60 x 64 407 / 445, 250 x 256 2383 / 4152.  Sorted is faster on
+    // 60 x 64 at 260 a node (214 / 174) and at 104 (74 / 64).
     bool crowded(int s) const { return walls && cfg.dims == 2 && sp[s].n / ncells >= (size_t)kCrowdedPpc; }
     static constexpr int kCrowdedPpc = 256;
 
@@ -4004,10 +4007,9 @@ struct SimND {
             for (int s = 0; s < cfg.nspecies; ++s)
                 if (since_sort[s] >= species_interval[s] && sp[s].n && !crowded(s)) sort_mask |= 1u << s;
             for (int s = 0; s < cfg.nspecies; ++s) {
-                if (since_sort[s] < species_interval[s]) continue;
-                since_sort[s] = 0;
+                if (since_sort[s] >= species_interval[s]) since_sort[s] = 0;
                 // histogram, three scan passes, scatter (FP32: rank + gather; tiles: their items)
-                if (sp[s].n) launches += (fp32 ? 6 : 5) + (sp[s].tiled ? 1 : 0);
+                if (sort_mask >> s & 1u) launches += (fp32 ? 6 : 5) + (sp[s].tiled ? 1 : 0);
             }
             if (sort_mask) steps_since_sort = 0;
             for (int s = 0; s < cfg.nspecies; ++s)

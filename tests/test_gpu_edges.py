@@ -379,6 +379,22 @@ def test_walls_loaded_on_the_device(dims):
         before = np.array([dev.boundary_losses(k) for k in range(2)], np.int64)
 
 
+@pytest.mark.parametrize("ppc,sorts", [(255, 2), (256, 0)])
+def test_crowded_walls_are_counted_as_they_run(ppc, sorts):
+    """2D runs with walls of 256 particles a node and more are not sorted, and no sort is counted."""
+    n = (8, 9)
+    count = ppc * n[0] * n[1]
+    dev = apic.SimulationND(apic.config_nd(dims=2, n=n, length=(4.0, 2.0), dt=1e-3, sort_interval=2,
+                                           species=[(q, m, w, count) for q, m, w in SPECIES],
+                                           walls=((0, 1), [0.0] * 4, (3, 3, 2, 2))))
+    for k in range(2):
+        dev.load_maxwellian(k, count, 3 + k, 1.0)
+    dev.initialize()
+    dev.step(4)
+    # density, forward, sweep, inverse, field; a push per species; five launches per sorted species
+    assert dev.launch_count() == 4 * (5 + 2) + sorts * 2 * 5
+
+
 @pytest.mark.parametrize("n,wall", [((9, 8), (1, 0)), ((9, 17), (1, 1)), ((9, 9, 17), (1, 1, 1))])
 def test_velocities_of_absorbed_particles(n, wall):
     """v is read in load order: an absorbed particle keeps the v of the last read before its loss

@@ -6,7 +6,8 @@ fastest, with the table of timings.  Results can be cached in a JSON file keyed
 by the workload shape and the device name, so a service tunes once per shape.
 
 * ``tune_plasma``: 2D3V/3D3V decks - cell-sort interval x particles per thread
-  of the FP32 step push (``apic_config_nd.sort_interval``, ``push_items``).
+  of the FP32 step push (``apic_config_nd.sort_interval``, ``push_items``; 3D
+  decks that are pushed by tiles have no such setting).
 * ``tune_swarm_server``: steps per graph launch of the swarm server (the
   convergence-check cadence trades latency against launch overhead).
 * ``tune_group``: how many 1D runs to step together on one GPU.
@@ -48,17 +49,24 @@ def _cache_put(path, key, value):
         json.dump(data, f, indent=1, sort_keys=True)
 
 
+def by_tiles(plan):
+    """True when every species of the FP32 deck is pushed by tiles: 3D, extents that are
+    multiples of 8, at least 2 particles a cell (push_items is not used then)."""
+    cells = int(np.prod(plan.n))
+    return plan.dims == 3 and all(k % 8 == 0 for k in plan.n) and all(s[3] >= 2 * cells for s in plan.species)
+
+
 def tune_plasma(plan, precision, sort_intervals=(2, 3, 4, 6, 8, 16), push_items=(1, 2, 4, 8), steps=None, cache=None):
     """Fastest (sort_interval, push_items) for a workloads.PlasmaPlan deck:
     each candidate runs one full sort period (at least `steps` steps) after a
-    warm-up and is timed per step, sort included."""
+    warm-up and is timed per step, sort included.  push_items is 0 where it is not used."""
     import torch
     import apic
     key = f"plasma/{plan.dims}/{'x'.join(map(str, plan.n))}/{plan.particles}/{precision}/{_device_name()}"
     hit = _cache_get(cache, key)
     if hit:
         return hit
-    items = push_items if precision == apic.FP32 else (0,)
+    items = push_items if precision == apic.FP32 and not by_tiles(plan) else (0,)
     table = []
     for si in sort_intervals:
         for it in items:

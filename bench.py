@@ -667,11 +667,13 @@ def bench_plasma(args, rank, dist):
     traffic, traffic_note = None, None
     items = push_items or (4 if dims == 2 else 2)
     # consecutive particles per thread (2D, k_push32_run) or whole tiles (3D, k_push32_tile)
-    run_kernel = prec == apic.FP32 and (dims == 3 or items in (2, 4))
+    from apic import autotune
+    by_tiles = prec == apic.FP32 and autotune.by_tiles(plan)
+    run_kernel = prec == apic.FP32 and items in (2, 4)
     if prec == apic.FP32:
         captured = {2: 4194304, 3: 16777216}[dims]
-        name = ("k_push32_tile_plasma3d_fp32.md" if dims == 3 else
-                "k_push32_run_plasma2d_fp32.md" if run_kernel else "k_push32_plasma2d_fp32.md")
+        name = ("k_push32_tile_plasma3d_fp32.md" if by_tiles else
+                f"k_push32_run_plasma{dims}d_fp32.md" if run_kernel else f"k_push32_plasma{dims}d_fp32.md")
         t = _profiled_traffic(name)
         if t:
             traffic = t * (P / 2) / captured
@@ -684,16 +686,16 @@ def bench_plasma(args, rank, dist):
     return {
         "value": value, "ms_per_step": ms_max / args.steps, "dtype": "f32" if prec == apic.FP32 else "f64",
         "config": {"workload": WORKLOAD_2D if dims == 2 else WORKLOAD_3D, "particles": P, "form": form,
-                   "sort_interval": sort_interval, "push_items": push_items or ("4" if dims == 2 else "2"),
+                   "sort_interval": sort_interval,
+                   "push_items": "none (by tiles)" if by_tiles else items if prec == apic.FP32 else "none (FP64)",
                    "autotuned": tuned["table"] if tuned else None,
                    "l2": f"inputs larger than L2 ({bpp // 2 * P / 1e9:.1f} GB of particle state)"},
         "e2e": {"value": e_total / (e_ms * 1e-3), "unit": "particle-steps/s", "h2d_bytes_per_step": h2d,
                 "d2h_bytes_per_step": d2h},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                      "traffic": traffic, "traffic_note": traffic_note, "peak_kind": peak_kind,
-                     "kernel": (("k_push32_tile" if dims == 3 else "k_push32_run" if run_kernel else "k_push32_step")
-                                if prec == apic.FP32 else "k_push_run")
-                     + f"<{dims}, boris, items={items}>",
+                     "kernel": (f"k_push_run<{dims}, boris>" if prec != apic.FP32 else "k_push32_tile<boris>" if by_tiles
+                                else f"k_push32_{'run' if run_kernel else 'step'}<{dims}, boris, items={items}>"),
                      "bytes_per_particle_step": bpp, "push_ms": per_step_push,
                      "solve_ms": solve_ms / max(nsteps, 1), "sort_ms_per_step": sort_ms / max(nsteps, 1)},
         "gpu_launches": launches,
@@ -941,7 +943,7 @@ def bench_swarm(args, rank, dist):
 # stays within a few minutes.
 OTHER_CONFIGS = {
     "plasma2d": {"sort_interval": 8, "push_items": 4, "e2e_steps": 2},
-    "plasma3d": {"sort_interval": 3, "push_items": 2, "e2e_steps": 1},
+    "plasma3d": {"sort_interval": 3, "push_items": 0, "e2e_steps": 1},
     "swarm": {"steps_per_launch": 100, "requests": 48, "mixed_requests": 16},
 }
 

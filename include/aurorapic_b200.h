@@ -382,7 +382,9 @@ typedef struct {
     int nspecies;
     apic_species species[APIC_MAX_SPECIES];
     int push_items;             /* FP32 form: particles per thread of the step push, 1, 2, 4 or 8
-                                   (0 = default: 4 in 2D, 2 in 3D); a tuning knob, no effect on results */
+                                   (0 = default: 4 in 2D, 2 in 3D); a tuning knob, no effect on results.
+                                   Not used by 3D species that are pushed by tiles: every extent a
+                                   multiple of 8 and at least 2 particles a cell */
     size_t species_sort_interval[APIC_MAX_SPECIES];  /* per species (0 = sort_interval): slow heavy
                                    species keep their cell order far longer; no effect on results */
     /* magnetic_field_profile (TabulatedVectorField1D, src/PrescribedField.cpp:89-113): B piecewise

@@ -162,13 +162,15 @@ def test_fp32_energy_conservation_2d():
 
 
 @pytest.mark.parametrize("dims,cells,ppc,sort_interval,steps", [
-    (2, (64, 64), 16, 4, 9), (3, (16, 16, 16), 8, 4, 9), (3, (32, 32, 32), 8, 1000, 30)])
+    (2, (64, 64), 16, 4, 9), (3, (16, 16, 16), 8, 4, 9), (3, (32, 32, 32), 8, 1000, 30),
+    (3, (16, 16, 4), 8, 4, 9), (3, (32, 4, 32), 8, 1000, 30), (3, (32, 32, 32), 1, 4, 9)])
 def test_push_items_leave_results_unchanged(dims, cells, ppc, sort_interval, steps):
     """The FP32 push's particles-per-thread knob changes only speed: every
     setting (one particle per thread, the shared-memory box pushes at 2 and 4,
     8 per thread) gives the same particles and fields, also when the particles
     have drifted far from their sorted order (sorted once, 30 steps: many
-    gather and deposit outside their CTA's box)."""
+    gather and deposit outside their CTA's box).  The first two 3D decks are pushed by
+    tiles, whatever the knob; an extent of 4, or one particle a cell, is not."""
     plan = W.plasma_plan(dims, cells=cells, ppc=ppc, seed=4)
     ref = None
     for items in (1, 2, 4, 8):
@@ -193,6 +195,15 @@ def test_autotuner_returns_a_candidate():
     out = autotune.tune_plasma(plan, apic.FP32, sort_intervals=(4, 8), push_items=(1, 4), steps=8)
     assert out["sort_interval"] in (4, 8) and out["push_items"] in (1, 4)
     assert len(out["table"]) == 4 and all(r["ms_per_step"] > 0 for r in out["table"])
+
+
+@pytest.mark.parametrize("cells,ppc,candidates", [((16, 16, 16), 2, 1), ((16, 16, 16), 1, 2), ((16, 4, 16), 2, 2)])
+def test_autotuner_times_each_3d_kernel_once(cells, ppc, candidates):
+    """A deck pushed by tiles has no particles-per-thread setting to time."""
+    from apic import autotune
+    plan = W.plasma_plan(3, cells=cells, ppc=ppc, seed=4)
+    out = autotune.tune_plasma(plan, apic.FP32, sort_intervals=(4,), push_items=(1, 4), steps=4)
+    assert [r["push_items"] for r in out["table"]] == ([0] if candidates == 1 else [1, 4])
 
 
 def _with_profile(cfg, axis, coords, values):

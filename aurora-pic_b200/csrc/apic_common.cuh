@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
@@ -54,9 +55,10 @@ __device__ __forceinline__ unsigned long long join64(unsigned lo, unsigned hi) {
 // one Newton correction of the quotient through its exact remainder (Markstein,
 // IBM J. Res. Dev. 34 (1990) 111): three operations where the division takes
 // about nine and a slow path.  The corrected quotient is the rounding of a
-// value within 2^-52 ulp of x / d.  rd = 0 asks for the division (spacings
-// whose reciprocal or remainder would leave the normal range).
-__device__ __forceinline__ double cells_of(double x, double d, double rd) {
+// value within 2^-52 ulp of x / d, for x from 2^-960 on (below, the remainder leaves
+// the normal range and the last bits of a quotient near 0 may differ).  rd = 0
+// asks for the division (spacings whose reciprocal would leave it).
+__host__ __device__ __forceinline__ double cells_of(double x, double d, double rd) {
     if (rd == 0.0) return x / d;
     const double q = x * rd;
     return fma(fma(-q, d, x), rd, q);

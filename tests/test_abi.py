@@ -157,3 +157,63 @@ def test_bgk_configuration_checks(bgk, models, msg):
     with pytest.raises(apic.ApicError) as e:
         apic.Simulation1D(cfg, tabs)
     assert msg in str(e.value)
+
+
+CELLS_CHECK = r"""
+#include <cstdio>
+#include <random>
+#include "apic_common.cuh"
+int main() {
+    std::mt19937_64 rng(7);
+    std::uniform_real_distribution<double> u(0.0, 1.0);
+    long long bad = 0, n = 0;
+    auto check = [&](double x, double d, double rd) {
+        ++n;
+        if (!(x >= 0.0)) return;
+        const double q = apic::cells_of(x, d, rd), want = x / d;
+        // below 2^-960 the remainder leaves the normal range: the cell is the same
+        const bool same = x < 0x1p-960 ? std::floor(q) == std::floor(want) && std::fabs(q - want) <= 0x1p-900 : q == want;
+        if (!same && bad++ < 5) std::printf("%a / %a\\n", x, d);
+    };
+    for (int c = 0; c < 4000; ++c) {
+        const int cells = 2 + (int)(rng() % 4096);
+        // lengths of every size, some of them exact multiples of the cells
+        const double L = c % 3 == 0 ? cells * std::ldexp(1.0, (int)(rng() % 60) - 50) : std::exp2(60.0 * u(rng) - 50.0);
+        const double d = L / cells, rd = apic::reciprocal_spacing(d);
+        for (int k = 0; k < 400; ++k) {
+            const int i = (int)(rng() % (unsigned)(cells + 1));
+            double edge[2] = {i * d, L * ((double)i / cells)};
+            for (double e : edge) {
+                check(e, d, rd);
+                double lo = e, hi = e;
+                for (int s = 0; s < 3; ++s) {
+                    check(lo = std::nextafter(lo, 0.0), d, rd);
+                    check(hi = std::nextafter(hi, 2.0 * L), d, rd);
+                }
+            }
+            check(L * u(rng), d, rd);
+        }
+    }
+    for (double d : {1e-300, 1e300, 1e-310}) check(0.7 * d, d, apic::reciprocal_spacing(d));
+    std::printf("%lld of %lld quotients differ\\n", bad, n);
+    return bad != 0;
+}
+"""
+
+
+def test_cell_quotients_are_the_division(tmp_path):
+    """cells_of (a product and a correction in place of the division) gives the bits of x / d at
+    the multiples of the spacing, next to them and anywhere in the domain: cell indices and
+    fractions are the reference's (the fraction of a position below 2^-960 within 2^-900)."""
+    import shutil
+    import subprocess
+    nvcc = shutil.which("nvcc") or "/usr/local/cuda/bin/nvcc"
+    if not os.path.exists(nvcc):
+        pytest.skip("no nvcc on this host")
+    src, exe = tmp_path / "cells.cu", tmp_path / "cells"
+    src.write_text(CELLS_CHECK)
+    subprocess.run([nvcc, "-std=c++17", "-O2", "-Xcompiler", "-ffp-contract=off", "-I", os.path.join(ROOT, "include"),
+                    "-I", os.path.join(ROOT, "aurora-pic_b200", "csrc"), "-gencode", "arch=compute_100a,code=sm_100a",
+                    str(src), "-o", str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True)
+    assert out.returncode == 0, out.stdout

@@ -3296,11 +3296,15 @@ __global__ void k_split_field(const double* __restrict__ E, double* __restrict__
 // take 1 MB pieces in turn, each with two pinned buffers and a stream of its own, so
 // the transfers overlap the host copies and the page faults of fresh
 // destinations, which one thread would take one after another.  Small reads take the driver's
-// own path.  The buffers (16 MB pinned) belong to the run and are made at its
-// first large read.
+// own path, and so do page-locked destinations, which the GPU writes itself (256^3, one
+// array: 2.4 ms, through the pieces 3.8).  The buffers (16 MB pinned) and streams belong
+// to the run.  They take 10 to 20 ms to make, as long as the driver's path takes for 100 MB of
+// fresh destinations, so a read makes them from kHuge bytes on or, with the field, when the
+// run has read its field before (rho and phi of 128^3, read once: 1.8 ms, with the set-up 13;
+// a one-off 1024 x 1024 solve: 20, with the set-up 28).
 struct HostCopier {
     static constexpr int kWorkers = 8;
-    static constexpr size_t kPiece = 1 << 20, kLarge = 16 << 20;
+    static constexpr size_t kPiece = 1 << 20, kLarge = 16 << 20, kHuge = 256 << 20;
     struct Job {
         double* dst;
         const double* src;
@@ -3308,6 +3312,7 @@ struct HostCopier {
     };
     unsigned char* pinned = nullptr;
     cudaStream_t streams[kWorkers] = {};
+    bool field_read = false;
 
     ~HostCopier() {
         for (auto& s : streams)
@@ -3315,15 +3320,24 @@ struct HostCopier {
         if (pinned) cudaFreeHost(pinned);
     }
 
-    // the sources must be complete: the workers' streams do not wait for `stream`
-    void run(const std::vector<Job>& jobs, cudaStream_t stream) {
+    static bool page_locked(const void* p) {
+        cudaPointerAttributes a{};
+        APIC_CUDA(cudaPointerGetAttributes(&a, p));
+        return a.type != cudaMemoryTypeUnregistered;
+    }
+
+    // the sources must be complete: the workers' streams do not wait for `stream`.
+    void run(std::vector<Job> jobs, cudaStream_t stream, bool field) {
+        const auto direct = std::partition(jobs.begin(), jobs.end(), [](const Job& j) { return !page_locked(j.dst); });
         size_t total = 0;
-        for (const Job& j : jobs) total += j.bytes;
-        if (total < kLarge) {
-            for (const Job& j : jobs) APIC_CUDA(cudaMemcpyAsync(j.dst, j.src, j.bytes, cudaMemcpyDeviceToHost, stream));
-            APIC_CUDA(cudaStreamSynchronize(stream));
-            return;
-        }
+        for (auto j = jobs.begin(); j != direct; ++j) total += j->bytes;
+        const bool plain = total < kLarge || !(pinned || total >= kHuge || (field && field_read));
+        field_read = field_read || field;
+        for (auto j = plain ? jobs.begin() : direct; j != jobs.end(); ++j)
+            APIC_CUDA(cudaMemcpyAsync(j->dst, j->src, j->bytes, cudaMemcpyDeviceToHost, stream));
+        APIC_CUDA(cudaStreamSynchronize(stream));
+        if (plain) return;
+        jobs.erase(direct, jobs.end());
         if (!pinned) APIC_CUDA(cudaHostAlloc(&pinned, 2 * kWorkers * kPiece, cudaHostAllocDefault));
         for (auto& s : streams)
             if (!s) APIC_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -4146,7 +4160,7 @@ struct SimND {
             for (int c = 0; c < cfg.dims; ++c) jobs.push_back({E + c * N, plane[c], N * sizeof(double)});
         }
         sync();
-        copier.run(jobs, stream);
+        copier.run(jobs, stream, E != nullptr);
     }
 
     void sample(apic_sample_nd* out) {

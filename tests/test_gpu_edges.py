@@ -210,6 +210,34 @@ def test_fields_read_back(n):
         assert rel_max(E, E2) < TOL
 
 
+def test_fields_into_any_destination():
+    """Large reads of some or all fields, into pageable and page-locked memory, before and after
+    the run's first read of the field."""
+    import torch
+    n = (128, 128, 128)
+    N = int(np.prod(n))
+    dev = apic.SimulationND(apic.config_nd(dims=3, n=n, length=(1.0, 2.0, 3.0), dt=0.1,
+                                           species=[(q, m, w, 5000) for q, m, w in SPECIES]))
+    for k in range(2):
+        dev.load(k, *_particles(5000, 3, (1.0, 2.0, 3.0), 5 + k))
+    dev.initialize()
+    L, sizes = apic._bind_nd(), (N, N, 3 * N)
+
+    def read(which, locked):
+        out = [torch.full((s,), np.nan, dtype=torch.float64, pin_memory=k in locked).numpy() if k in which else None
+               for k, s in enumerate(sizes)]
+        apic._check_nd(L.apic_simnd_read_fields(dev.h, *[apic.dptr(a) for a in out]), dev.h)
+        return out
+
+    first = [read((0, 1), ()), read((0, 1, 2), ())]
+    want = [a.ravel() for a in dev.fields()]
+    calls = first + [read(w, l) for w, l in (((0, 1), ()), ((0, 1, 2), ()), ((0, 1, 2), (0, 1, 2)), ((0, 2), (2,)),
+                                               ((1, 2), (1,)), ((2,), ()), ((1,), (1,)))]
+    for out in calls:
+        for a, b in zip(out, want):
+            assert a is None or np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("precision", [apic.FP64, apic.FP32])
 @pytest.mark.parametrize("particles,steps_per_launch", [(1, 7), (1023, 1), (1025, 60), (2500, 129), (2500, 300)])
 def test_fixed_swarm_alone_and_beside_a_branching_run(precision, particles, steps_per_launch):

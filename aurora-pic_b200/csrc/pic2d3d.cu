@@ -26,7 +26,6 @@
 #include <memory>
 #include <mutex>
 #include <string>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -3375,11 +3374,12 @@ struct HostCopier {
             if (e != cudaSuccess) failed.store((int)e);
         };
         std::vector<std::thread> threads;
+        threads.reserve(kWorkers);
         for (int t = 1; t < kWorkers; ++t) {
             try {
                 threads.emplace_back(work, t);
-            } catch (const std::system_error&) {
-                break;  // fewer workers: those that run take every piece
+            } catch (...) {  // no thread, or no memory for one (a joinable thread must not be unwound)
+                break;       // fewer workers: those that run take every piece
             }
         }
         work(0);

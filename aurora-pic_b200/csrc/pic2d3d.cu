@@ -25,6 +25,7 @@
 #include <functional>
 #include <memory>
 #include <mutex>
+#include <set>
 #include <string>
 #include <thread>
 #include <vector>
@@ -2420,7 +2421,23 @@ static int ilog2(size_t v) { int k = 0; while ((size_t(1) << k) < v) ++k; return
 // limit is a property of the kernel function shared by every simulation and
 // solve in the process, so it is never lowered to one mesh's need (a later
 // small mesh would otherwise make an earlier large mesh's launches fail).
-void ensure_solver_attributes();
+// Raises a kernel's limit of dynamic shared memory, once per device.  Called where a run is set
+// up, for the kernels it will launch and no others: the call loads the kernel, and all of
+// the field solves' together took 11 ms of a process's first run.
+static void allow_smem(const void* kernel, size_t bytes) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    APIC_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(mu);
+    if (done.count({dev, kernel})) return;
+    APIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    done.insert({dev, kernel});
+}
+template <class... Args>
+static void allow_smem(void (*kernel)(Args...), size_t bytes) {
+    allow_smem(reinterpret_cast<const void*>(kernel), bytes);
+}
 
 struct Solver {
     FieldsND F{};
@@ -2537,7 +2554,34 @@ struct Solver {
         smem_pair = std::max(smem_of(px, kFwdMulInv), smem_of(py, kFwdMulInv));
         if (dims == 3) smem_pair = std::max(smem_pair, smem_of(pz, kFwdMulInv));
         require(smem_pair <= kFftSmemMax, "FFT tile exceeds the shared-memory bound", APIC_ERR_UNSUPPORTED);
-        ensure_solver_attributes();
+        allow_passes();
+    }
+
+    // the shared memory of the passes of solve()
+    void allow_passes() {
+        if (F.dims == 2) {
+            allow_pass<kFwdFromRho>(0);
+            allow_pass<kFwdMulInv>(1);
+        } else {
+            allow_pass<kFwdFromRho>(0);
+            allow_pass<kFwdInPlace>(1);
+            allow_pass<kFwdMulInv>(2);
+            allow_pass<kInvInPlace>(1);
+        }
+        allow_pass<kInvToFields>(0);
+    }
+    template <int MODE, int R1, int R2>
+    static void allow_reg(int axis) {
+        if (axis == 0) allow_smem(k_fft_reg<MODE, true, R1, R2>, reg_smem<R1, R2, true>(MODE));
+        else allow_smem(k_fft_reg<MODE, false, R1, R2>, reg_smem<R1, R2, false>(MODE));
+    }
+    template <int MODE>
+    void allow_pass(int axis) {
+        if (!in_regs[axis]) allow_smem(k_fft<MODE>, kFftSmemMax);
+        else if (reg[axis].n == 256) allow_reg<MODE, 16, 16>(axis);
+        else if (reg[axis].n == 128) allow_reg<MODE, 16, 8>(axis);
+        else if (reg[axis].n == 64) allow_reg<MODE, 8, 8>(axis);
+        else allow_reg<MODE, 8, 4>(axis);
     }
 
     size_t smem_of(const FftPass& f, int mode) const {
@@ -2582,8 +2626,6 @@ struct Solver {
         APIC_CUDA(cudaGetLastError());
     }
 };
-
-void ensure_solver_attributes();
 
 // ---- field solves with walls --------------------------------------------------------
 //
@@ -3103,7 +3145,6 @@ struct WallSolver {
             w.rd[1][a] = reciprocal_spacing(2.0 * w.d[a]);
         }
         for (int k = 0; k < 4; ++k) w.side[k] = dims == 2 ? pot[k] : 0.0;
-        ensure_solver_attributes();
         mixed = dims == 2 && !(wall[0] && wall[1]);
         if (mixed) {
             pa = wall[0] ? 1 : 0;
@@ -3116,6 +3157,9 @@ struct WallSolver {
             inv = static_cast<double*>(alloc(modes * ni * sizeof(double)));
             hat = static_cast<Cplx*>(alloc(modes * ni * sizeof(Cplx)));
             tw = twiddles(np);
+            allow_smem(k_mixed_forward, kWallSmemMax);
+            allow_smem(k_mixed_inverse, kWallSmemMax);
+            if (ni <= kMixedSweepMaxRows) allow_smem(k_mixed_sweep<true>, mixed_sweep_smem(kMixedSweepMaxRows));
             k_mixed_coeffs<<<(unsigned)((modes + 127) / 128), 128, 0, stream>>>(mu, inv, ni + 2, np, 1.0 / (hd * hd),
                                                                                 1.0 / (hp * hp));
             APIC_CUDA(cudaGetLastError());
@@ -3151,6 +3195,15 @@ struct WallSolver {
             f.tw = twiddles(2 * (M[a] + 1));
             f.scale = scale;
             for (int b = 0; b < 3; ++b) f.eig[b] = eig[b];
+            if (f.log2N >= 6 && f.log2N <= 8) continue;  // in registers: within the default limit
+            if (a == 0) {
+                allow_smem(k_dst_pass<kDstFromRho>, kWallSmemMax);
+                allow_smem(k_dst_pass<kDstToPhi>, kWallSmemMax);
+            } else if (a == dims - 1) {
+                allow_smem(k_dst_pass<kDstSolve>, kWallSmemMax);
+            } else {
+                allow_smem(k_dst_pass<kDstInPlace>, kWallSmemMax);
+            }
         }
     }
 
@@ -3214,64 +3267,6 @@ struct WallSolver {
         APIC_CUDA(cudaGetLastError());
     }
 };
-
-namespace {
-std::mutex g_attr_mu;
-bool g_attr_done[64] = {};
-}  // namespace
-
-template <int MODE, int R1, int R2>
-static void set_reg_mode() {
-    APIC_CUDA(cudaFuncSetAttribute(k_fft_reg<MODE, true, R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)reg_smem<R1, R2, true>(MODE)));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft_reg<MODE, false, R1, R2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)reg_smem<R1, R2, false>(MODE)));
-}
-template <int R1, int R2>
-static void set_reg_attributes() {
-    set_reg_mode<kFwdFromRho, R1, R2>();
-    set_reg_mode<kFwdInPlace, R1, R2>();
-    set_reg_mode<kFwdMulInv, R1, R2>();
-    set_reg_mode<kInvInPlace, R1, R2>();
-    set_reg_mode<kInvToFields, R1, R2>();
-}
-
-void ensure_solver_attributes() {
-    int dev = 0;
-    APIC_CUDA(cudaGetDevice(&dev));
-    require(dev >= 0 && dev < 64, "device index out of range");
-    std::lock_guard<std::mutex> lock(g_attr_mu);
-    if (g_attr_done[dev]) return;
-    const int fft = (int)kFftSmemMax;
-    APIC_CUDA(cudaFuncSetAttribute(k_fft<kFwdFromRho>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft<kFwdInPlace>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft<kFwdMulInv>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft<kInvInPlace>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    APIC_CUDA(cudaFuncSetAttribute(k_fft<kInvToFields>, cudaFuncAttributeMaxDynamicSharedMemorySize, fft));
-    set_reg_attributes<16, 16>();
-    set_reg_attributes<16, 8>();
-    set_reg_attributes<8, 8>();
-    set_reg_attributes<8, 4>();
-    auto set_box = [](auto kernel, size_t bytes) {
-        APIC_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    };
-    set_box(k_push32_tile<true, true, 1>, tile32_smem<1>());
-    set_box(k_push32_tile<true, false, 1>, tile32_smem<1>());
-    set_box(k_push32_tile<false, false, 1>, tile32_smem<1>());
-    set_box(k_push32_tile<true, true, 2>, tile32_smem<2>());
-    set_box(k_push32_tile<true, false, 2>, tile32_smem<2>());
-    set_box(k_push32_tile<false, false, 2>, tile32_smem<2>());
-    const int tile = (int)kWallSmemMax;
-    APIC_CUDA(cudaFuncSetAttribute(k_dst_pass<kDstFromRho>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_dst_pass<kDstInPlace>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_dst_pass<kDstSolve>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_dst_pass<kDstToPhi>, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_mixed_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_mixed_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, tile));
-    APIC_CUDA(cudaFuncSetAttribute(k_mixed_sweep<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)mixed_sweep_smem(kMixedSweepMaxRows)));
-    g_attr_done[dev] = true;
-}
 
 // the interleaved field as planes
 template <int DIM>
@@ -3626,7 +3621,13 @@ struct SimND {
                 sp[s].chunk = dalloc<uint4>(ntiles + 2 * (c.species[s].capacity / 2048) + 1);
                 sp[s].extra = dalloc<unsigned>(1);
             }
-            ensure_solver_attributes();
+            const auto allow = [](auto one, auto two) {
+                allow_smem(one, tile32_smem<1>());
+                allow_smem(two, tile32_smem<2>());
+            };
+            if (boris && p.prof_rows) allow(k_push32_tile<true, true, 1>, k_push32_tile<true, true, 2>);
+            else if (boris) allow(k_push32_tile<true, false, 1>, k_push32_tile<true, false, 2>);
+            else allow(k_push32_tile<false, false, 1>, k_push32_tile<false, false, 2>);
         }
         sample_partial = dalloc<double>(3 * kSampleBlocks);
         sample_done = dalloc<unsigned>(1);
@@ -4589,11 +4590,9 @@ extern "C" int apic_field_solve_periodic_nd_noalloc(int dims, const size_t* n, c
         require_device_buffer(d_phi, "d_phi");
         require_device_buffer(d_electric, "d_electric");
         // the scratch array's address in the current device's context, looked
-        // up on every call (cheap), so it stays valid after a device reset; and
-        // the FFT kernels' fixed shared-memory limit (set once per device)
+        // up on every call (cheap), so it stays valid after a device reset
         void* base = nullptr;
         APIC_CUDA(cudaGetSymbolAddress(&base, g_solve_scratch));
-        ensure_solver_attributes();
         unsigned char* bytes = static_cast<unsigned char*>(base);
         Cplx* W = reinterpret_cast<Cplx*>(bytes);
         Cplx* A = W + kNoAllocMaxPoints;
@@ -4644,6 +4643,7 @@ extern "C" int apic_field_solve_periodic_nd_noalloc(int dims, const size_t* n, c
         S.py.tw = S.pys.tw = tw + kNoAllocMaxLine;
         if (dims == 3) S.pz.tw = tw + 2 * kNoAllocMaxLine;
         APIC_CUDA(cudaGetLastError());
+        S.allow_passes();  // the FFT kernels' fixed shared-memory limit (set once per device)
         S.solve();
         k_noalloc_deinterleave<<<(unsigned)((N + 255) / 256), 256, 0, s>>>(E, dims, (long long)N, d_electric);
         APIC_CUDA(cudaGetLastError());

@@ -105,11 +105,11 @@ struct ParamsND {
 };
 
 // TabulatedVectorField1D::evaluate, src/PrescribedField.cpp:89-113, at coordinate
-// q inside the table (create checks that the table covers the domain).
+// q inside the table (create checks that the table covers the domain).  A particle
+// loaded outside the domain, or at a NaN, takes the nearest (the last) bracket.
 __device__ __forceinline__ void profile_b(const ParamsND& p, double q, double B[3]) {
     const double* c = p.prof_c;
     const int n = p.prof_rows;
-    int right;
     if (q == __ldg(c)) {
         for (int a = 0; a < 3; ++a) B[a] = __ldg(p.prof_v + a);
         return;
@@ -123,7 +123,7 @@ __device__ __forceinline__ void profile_b(const ParamsND& p, double q, double B[
         const int mid = (lo + hi) >> 1;
         if (q < __ldg(c + mid)) hi = mid; else lo = mid + 1;
     }
-    right = lo;
+    const int right = min(max(lo, 1), n - 1);
     const int left = right - 1;
     const double f = (q - __ldg(c + left)) / (__ldg(c + right) - __ldg(c + left));
     for (int a = 0; a < 3; ++a) {

@@ -136,6 +136,33 @@ def test_non_finite_particle_of_the_fp32_form(n, items, bad):
     dev.close()
 
 
+@pytest.mark.parametrize("precision", [apic.FP64, apic.FP32])
+@pytest.mark.parametrize("dims,axis", [(2, 0), (2, 1), (3, 2)])
+def test_positions_outside_the_table_of_a_field_profile(dims, axis, precision):
+    """B tabulated along an axis, particles loaded outside the domain: the table's end brackets
+    (a uniform B here) hold there, and a NaN position (FP32: it deposits nothing) reads none
+    past them."""
+    n, length, B, count = (8, 16, 8)[:dims], (4.0, 2.0, 3.0)[:dims], (0.1, 0.2, 0.3), 900
+    rng = np.random.default_rng(8)
+    pos = np.stack([rng.uniform(-0.9 * L, 1.9 * L, count) for L in length])
+    v = rng.standard_normal((3, count))
+    if precision == apic.FP32:
+        pos[axis, 17] = np.nan
+    got = []
+    for profile in (None, (axis, [0.0, 0.4, length[axis]], [B] * 3)):
+        dev = apic.SimulationND(apic.config_nd(
+            dims=dims, n=n, length=length, dt=0.05, precision=precision, species=[(-1.0, 1.0, 0.01, count)],
+            magnetic_field=(0.0, 0.0, 0.0) if profile else B, magnetic_field_profile=profile))
+        dev.load(0, pos, v)
+        dev.initialize()
+        dev.step(3)
+        got.append([a[:, np.arange(count) != 17] for a in dev.particles(0)])
+        dev.close()
+    for a, b in zip(*got):
+        assert np.isfinite(b).all()
+        assert np.max(np.abs(a - b)) < (1e-12 if precision == apic.FP64 else 1e-6) * np.max(np.abs(a))
+
+
 def test_bounded_wait_gives_up_and_a_later_wait_completes():
     """A wait limit far below the time of the enqueued steps ends the
     synchronising call with APIC_ERR_TIMEOUT; the work itself runs on, and a

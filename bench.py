@@ -843,11 +843,6 @@ def bench_swarm(args, rank, dist):
     batch = [_swarm_draw(rng, spec, W, k, 20_000_000 + 1000 * rank) for k in range(args.steps)]
     _, ps0, _ = srv.stats()
     ids = [srv.submit(r) for r in batch]
-    srv.set_kernel_timing(True)  # the first two advances time the push kernel one launch at a time
-    srv.advance()
-    srv.advance()
-    push_ms, collide_ms, push_launches, push_bytes = srv.kernel_times()
-    srv.set_kernel_timing(False)
     e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
     if dist:
         dist.barrier()
@@ -862,7 +857,6 @@ def bench_swarm(args, rank, dist):
     t_sat = e0.elapsed_time(e1) * 1e-3
     g1, ps1, _ = srv.stats()
     sat_psteps = ps1 - ps0
-    # the two timed advances ran before e0: count only the work inside the region
     ms_max, total = _reduce(dist, t_sat * 1e3, float(sat_psteps))
     value = total / (ms_max * 1e-3)
     capacity = len(batch) / t_sat
@@ -901,7 +895,10 @@ def bench_swarm(args, rank, dist):
     srv.close()
     lat = np.array(lat)
     hbm, peak_kind = peaks()
-    achieved = push_bytes / (push_ms * 1e-3) / 1e9 if push_ms > 0 else None
+    # the state's bytes of every particle-step: velocities, and displacements while sampling
+    size = 4 if prec == apic.FP32 else 8
+    sampled = sum(q.particles * max(0, res[i].steps_done - 2000) for i, q in zip(ids, batch))  # after the burn-in
+    achieved = 6 * size * (sat_psteps + sampled) / t_sat / 1e9
     steps_done = np.array([r.steps_done for r in results])
     return {
         "value": value, "ms_per_step": 1e3 * t_sat / max(1, (g1 - g0) * spl), "dtype": "f32" if prec == apic.FP32 else "f64",
@@ -925,12 +922,12 @@ def bench_swarm(args, rank, dist):
                   "mean_steps": float(steps_done.mean()), "serving_particle_steps_per_s": serve_value,
                   "mixed": mixed},
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s",
-                     "frac": achieved / hbm if achieved else None, "traffic": None,
-                     "traffic_note": "no ncu capture at the saturation size: the pool there spans tens of GB",
-                     "peak_kind": peak_kind, "kernel": "k_swarm_push<float>",
-                     "bytes_per_particle_step": "24 (burn-in) / 48 (sampling)",
-                     "push_ms_per_launch": push_ms / max(push_launches, 1),
-                     "collide_ms_per_launch": collide_ms / max(push_launches, 1)},
+                     "frac": achieved / hbm, "traffic": None,
+                     "traffic_note": "the electrons stay on the SM over the steps of a launch: the state's bytes cross "
+                                     "memory once a launch, not once a step",
+                     "peak_kind": peak_kind, "kernel": "k_swarm_steps<float>" if size == 4 else "k_swarm_steps<double>",
+                     "bytes_per_particle_step": f"{6 * size} (burn-in) / {12 * size} (sampling)",
+                     "ms_per_launch": 1e3 * t_sat / max(1, g1 - g0)},
         "gpu_launches": int(k1 - k0),
         "clocks": clk.summary(),
     }

@@ -931,14 +931,6 @@ __device__ __forceinline__ bool offsets_finite(const float f[3]) {
     return (DIM == 3 ? f[0] + f[1] + f[2] : f[0] + f[1]) < 4.0f;  // each in [0, 1), or NaN
 }
 
-// The step push of the FP32 form with ITEMS consecutive particles per thread
-// (loaded and stored as vectors).  Particles are sorted by cell, so a thread's
-// particles mostly share a cell: the field at the cell's nodes is fetched once
-// per run of equal cells, and the CIC weights of a run are summed in registers
-// (the deposit of src/Mesh2D.cpp:90-144 / src/Mesh3D.cpp:62-126 at the pushed
-// positions).  A run that ends inside the thread is committed with one 64-bit
-// atomic per node; each lane's last run joins a warp-segmented sum over the
-// lanes holding the same cell, whose last lane commits it.
 // One buffer of the FP32 state, by kernel argument (an index into the species'
 // arrays costs every access its pointer's load).
 struct State32 {
@@ -967,6 +959,14 @@ struct DepositBox {
     int x0, y0;
 };
 
+// The step push of the FP32 form with ITEMS consecutive particles per thread
+// (loaded and stored as vectors).  Particles are sorted by cell, so a thread's
+// particles mostly share a cell: the field at the cell's nodes is fetched once
+// per run of equal cells, and the CIC weights of a run are summed in registers
+// (the deposit of src/Mesh2D.cpp:90-144 / src/Mesh3D.cpp:62-126 at the pushed
+// positions).  A run that ends inside the thread is committed with one 64-bit
+// atomic per node; each lane's last run joins a warp-segmented sum over the
+// lanes holding the same cell, whose last lane commits it.
 template <int DIM, bool BORIS, int ITEMS, bool PROF>
 __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, const State32& A,
                                          unsigned long long* acc, const DepositBox& box) {
@@ -3691,7 +3691,8 @@ struct SimND {
             const State32 A = state32(S, b);
             // one cell around the tile when few particles leave it between sorts, else two
             // (a thermal electron moves about 0.1 cell a step, a heavier species at the same
-            // temperature less; 256^3, electrons sorted every 3 steps: one 4.6, two 4.8 ms)
+            // temperature less; push of 256^3, one against two cells, electrons sorted every 3
+            // steps 4.06 / 4.27 ms, 4: 4.10 / 4.30, 6: 4.24 / 4.36, 8: 4.53 / 4.40, 16: 5.23 / 4.94)
             double lightest = cfg.species[0].mass;
             for (int k = 1; k < cfg.nspecies; ++k) lightest = std::min(lightest, cfg.species[k].mass);
             const double reach = (double)species_interval[s] * std::sqrt(lightest / cfg.species[s].mass);

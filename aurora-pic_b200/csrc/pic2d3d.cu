@@ -923,14 +923,6 @@ __global__ void __launch_bounds__(kThreads) k_push32_step(ParamsND p, SpeciesND 
     }
 }
 
-// A particle with an infinite or NaN velocity keeps its cell and has a NaN
-// offset: it deposits nothing (the rounding by an added 2^23 would turn a NaN weight
-// into 106 particles' charge, and break the bounds of the box sums' carries).
-template <int DIM>
-__device__ __forceinline__ bool offsets_finite(const float f[3]) {
-    return (DIM == 3 ? f[0] + f[1] + f[2] : f[0] + f[1]) < 4.0f;  // each in [0, 1), or NaN
-}
-
 // One buffer of the FP32 state, by kernel argument (an index into the species'
 // arrays costs every access its pointer's load).
 struct State32 {
@@ -1153,9 +1145,12 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         }
         // (units of 2^-23 to nearest even: adding 2^23 leaves the integer in the low
         // bits of the float; the scale, a power of two, is exact on any factor)
-        if (!offsets_finite<DIM>(f)) continue;
         const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale}, uy[2] = {1.0f - f[1], f[1]};
         const float uz[2] = {DIM == 3 ? 1.0f - f[2] : 1.0f, DIM == 3 ? f[2] : 0.0f};
+        // a particle of infinite or NaN velocity keeps its cell, has a NaN offset and deposits
+        // nothing (its weights would become 106 particles' charge, and break the bounds
+        // of the box sums' carries)
+        if (!((DIM == 3 ? ux[1] * uy[1] * uz[1] : ux[1] * uy[1]) >= 0.0f)) continue;
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
             const float w = DIM == 3 ? ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1] : ux[j & 1] * uy[(j >> 1) & 1];
@@ -1443,12 +1438,14 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks) k_push32_tile(ParamsND 
 #pragma unroll
                 for (int j = 0; j < 8; ++j) w[j] = 0u;
             }
-            if (!offsets_finite<3>(f)) continue;
             // the weights in units of 2^-23, to nearest even: adding 2^23 leaves the
             // integer in the low bits of the float (a weight is at most 2^23 units);
             // the scale, a power of two, is exact on any factor
             const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale};
             const float uy[2] = {1.0f - f[1], f[1]}, uz[2] = {1.0f - f[2], f[2]};
+            // a NaN offset (see k_push32_run) deposits nothing: tested on the last weight, which
+            // is formed anyway (256^3: 4.05 ms a step, with a sum of the offsets 4.08)
+            if (!(ux[1] * uy[1] * uz[1] >= 0.0f)) continue;
 #pragma unroll
             for (int j = 0; j < 8; ++j)
                 w[j] += __float_as_uint(ux[j & 1] * uy[(j >> 1) & 1] * uz[j >> 2] + kWeightScale) - 0x4B000000u;

@@ -924,11 +924,23 @@ __global__ void __launch_bounds__(kThreads) k_push32_step(ParamsND p, SpeciesND 
 }
 
 // One buffer of the FP32 state, by kernel argument (an index into the species'
-// arrays costs every access its pointer's load).
+// arrays costs every access its pointer's load) ...
 struct State32 {
     unsigned* cell;
     float* off[3];
     float* vel[3];
+    __device__ __forceinline__ unsigned* cells() const { return cell; }
+    __device__ __forceinline__ float* offs(int a) const { return off[a]; }
+    __device__ __forceinline__ float* vels(int a) const { return vel[a]; }
+};
+// ... or by that index, for the 3D run push, where the pointers' registers cost more: 64 registers
+// and no spills against 80 (128^3, 2 x 3.1 M particles: push 214 against 227 us a step)
+struct Buffer32 {
+    const SpeciesND& S;
+    int buf;
+    __device__ __forceinline__ unsigned* cells() const { return S.cell[buf]; }
+    __device__ __forceinline__ float* offs(int a) const { return S.off[buf][a]; }
+    __device__ __forceinline__ float* vels(int a) const { return S.vel[buf][a]; }
 };
 
 // 2D: the CTA's deposit into a box of nodes in shared memory (kDBoxX cells
@@ -959,8 +971,8 @@ struct DepositBox {
 // positions).  A run that ends inside the thread is committed with one 64-bit
 // atomic per node; each lane's last run joins a warp-segmented sum over the
 // lanes holding the same cell, whose last lane commits it.
-template <int DIM, bool BORIS, int ITEMS, bool PROF>
-__device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, const State32& A,
+template <int DIM, bool BORIS, int ITEMS, bool PROF, class State>
+__device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, const State& A,
                                          unsigned long long* acc, const DepositBox& box) {
     constexpr int NN = DIM == 2 ? 4 : 8;  // nodes of a cell
     const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * ITEMS;
@@ -975,32 +987,32 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
     const bool full = first + ITEMS <= S.n;
     if (full) {
         if (ITEMS == 4) {
-            const uint4 c = __ldcs(reinterpret_cast<const uint4*>(A.cell + first));
+            const uint4 c = __ldcs(reinterpret_cast<const uint4*>(A.cells() + first));
             cl[0] = c.x; cl[1] = c.y; cl[2 % ITEMS] = c.z; cl[3 % ITEMS] = c.w;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM) {
-                    const float4 f = __ldcs(reinterpret_cast<const float4*>(A.off[a] + first));
+                    const float4 f = __ldcs(reinterpret_cast<const float4*>(A.offs(a) + first));
                     fo[0][a] = f.x; fo[1][a] = f.y; fo[2 % ITEMS][a] = f.z; fo[3 % ITEMS][a] = f.w;
                 } else {
 #pragma unroll
                     for (int k = 0; k < ITEMS; ++k) fo[k][a] = 0.0f;
                 }
-                const float4 v = __ldcs(reinterpret_cast<const float4*>(A.vel[a] + first));
+                const float4 v = __ldcs(reinterpret_cast<const float4*>(A.vels(a) + first));
                 vv[0][a] = v.x; vv[1][a] = v.y; vv[2 % ITEMS][a] = v.z; vv[3 % ITEMS][a] = v.w;
             }
         } else {
-            const uint2 c = __ldcs(reinterpret_cast<const uint2*>(A.cell + first));
+            const uint2 c = __ldcs(reinterpret_cast<const uint2*>(A.cells() + first));
             cl[0] = c.x; cl[1 % ITEMS] = c.y;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM) {
-                    const float2 f = __ldcs(reinterpret_cast<const float2*>(A.off[a] + first));
+                    const float2 f = __ldcs(reinterpret_cast<const float2*>(A.offs(a) + first));
                     fo[0][a] = f.x; fo[1 % ITEMS][a] = f.y;
                 } else {
                     fo[0][a] = 0.0f; fo[1 % ITEMS][a] = 0.0f;
                 }
-                const float2 v = __ldcs(reinterpret_cast<const float2*>(A.vel[a] + first));
+                const float2 v = __ldcs(reinterpret_cast<const float2*>(A.vels(a) + first));
                 vv[0][a] = v.x; vv[1 % ITEMS][a] = v.y;
             }
         }
@@ -1009,11 +1021,11 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         for (int k = 0; k < ITEMS; ++k) {
             const unsigned i = first + k;
             const bool ok = i < S.n;
-            cl[k] = ok ? A.cell[i] : 0u;
+            cl[k] = ok ? A.cells()[i] : 0u;
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                fo[k][a] = (ok && a < DIM) ? A.off[a][i] : 0.0f;
-                vv[k][a] = ok ? A.vel[a][i] : 0.0f;
+                fo[k][a] = (ok && a < DIM) ? A.offs(a)[i] : 0.0f;
+                vv[k][a] = ok ? A.vels(a)[i] : 0.0f;
             }
         }
     }
@@ -1147,35 +1159,33 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         // bits of the float; the scale, a power of two, is exact on any factor)
         const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale}, uy[2] = {1.0f - f[1], f[1]};
         const float uz[2] = {DIM == 3 ? 1.0f - f[2] : 1.0f, DIM == 3 ? f[2] : 0.0f};
-        // a particle of infinite or NaN velocity keeps its cell, has a NaN offset and deposits
-        // nothing (its weights would become 106 particles' charge, and break the bounds
-        // of the box sums' carries)
-        if (!((DIM == 3 ? ux[1] * uy[1] * uz[1] : ux[1] * uy[1]) >= 0.0f)) continue;
 #pragma unroll
         for (int j = 0; j < NN; ++j) {
             const float w = DIM == 3 ? ux[j & 1] * uy[(j >> 1) & 1] * uz[(j >> 2) & 1] : ux[j & 1] * uy[(j >> 1) & 1];
-            racc[j] += __float_as_uint(w + kWeightScale) - 0x4B000000u;
+            // (a particle of infinite or NaN velocity keeps its cell and has a NaN offset: the
+            // maximum makes its weights 0 instead of 106 particles' charge)
+            racc[j] += __float_as_uint(fmaxf(w + kWeightScale, kWeightScale)) - 0x4B000000u;
         }
     }
     // the state back, in place
     if (full) {
         if (ITEMS == 4) {
-            __stcs(reinterpret_cast<uint4*>(A.cell + first), make_uint4(cl[0], cl[1], cl[2 % ITEMS], cl[3 % ITEMS]));
+            __stcs(reinterpret_cast<uint4*>(A.cells() + first), make_uint4(cl[0], cl[1], cl[2 % ITEMS], cl[3 % ITEMS]));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM)
-                    __stcs(reinterpret_cast<float4*>(A.off[a] + first),
+                    __stcs(reinterpret_cast<float4*>(A.offs(a) + first),
                            make_float4(fo[0][a], fo[1][a], fo[2 % ITEMS][a], fo[3 % ITEMS][a]));
-                __stcs(reinterpret_cast<float4*>(A.vel[a] + first),
+                __stcs(reinterpret_cast<float4*>(A.vels(a) + first),
                        make_float4(vv[0][a], vv[1][a], vv[2 % ITEMS][a], vv[3 % ITEMS][a]));
             }
         } else {
-            __stcs(reinterpret_cast<uint2*>(A.cell + first), make_uint2(cl[0], cl[1 % ITEMS]));
+            __stcs(reinterpret_cast<uint2*>(A.cells() + first), make_uint2(cl[0], cl[1 % ITEMS]));
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
                 if (a < DIM)
-                    __stcs(reinterpret_cast<float2*>(A.off[a] + first), make_float2(fo[0][a], fo[1 % ITEMS][a]));
-                __stcs(reinterpret_cast<float2*>(A.vel[a] + first), make_float2(vv[0][a], vv[1 % ITEMS][a]));
+                    __stcs(reinterpret_cast<float2*>(A.offs(a) + first), make_float2(fo[0][a], fo[1 % ITEMS][a]));
+                __stcs(reinterpret_cast<float2*>(A.vels(a) + first), make_float2(vv[0][a], vv[1 % ITEMS][a]));
             }
         }
     } else {
@@ -1183,11 +1193,11 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
         for (int k = 0; k < ITEMS; ++k) {
             const unsigned i = first + k;
             if (i >= S.n) continue;
-            A.cell[i] = cl[k];
+            A.cells()[i] = cl[k];
 #pragma unroll
             for (int a = 0; a < 3; ++a) {
-                if (a < DIM) A.off[a][i] = fo[k][a];
-                A.vel[a][i] = vv[k][a];
+                if (a < DIM) A.offs(a)[i] = fo[k][a];
+                A.vels(a)[i] = vv[k][a];
             }
         }
     }
@@ -1216,9 +1226,10 @@ __device__ __forceinline__ void push_run(const ParamsND& p, const SpeciesND& S, 
     if (tail && key != kNoCell) commit(key, racc);
 }
 
+// (3D states no CTAs per SM: 4 spilled, 128^3 with 4 particles a thread 272 -> 394 us a step)
 template <int DIM, bool BORIS, int ITEMS, bool PROF>
-__global__ void __launch_bounds__(kThreads, 4) k_push32_run(ParamsND p, SpeciesND S, State32 A,
-                                                         unsigned long long* acc) {
+__global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 0)
+    k_push32_run(ParamsND p, SpeciesND S, State32 A, int buf, unsigned long long* acc) {
     if constexpr (DIM == 2) {
         __shared__ unsigned s_sum[kDBoxNodes];
         const int nx = p.n[0], ny = p.n[1];
@@ -1238,7 +1249,7 @@ __global__ void __launch_bounds__(kThreads, 4) k_push32_run(ParamsND p, SpeciesN
             atomicAdd(acc + (size_t)((box.y0 + qy) & (ny - 1)) * nx + ((box.x0 + qx) & (nx - 1)), v);
         }
     } else {
-        push_run<DIM, BORIS, ITEMS, PROF>(p, S, A, acc, DepositBox{nullptr, 0, 0});
+        push_run<DIM, BORIS, ITEMS, PROF>(p, S, Buffer32{S, buf}, acc, DepositBox{nullptr, 0, 0});
     }
 }
 
@@ -1443,7 +1454,7 @@ __global__ void __launch_bounds__(kThreads, kTileBlocks) k_push32_tile(ParamsND 
             // the scale, a power of two, is exact on any factor
             const float ux[2] = {(1.0f - f[0]) * kWeightScale, f[0] * kWeightScale};
             const float uy[2] = {1.0f - f[1], f[1]}, uz[2] = {1.0f - f[2], f[2]};
-            // a NaN offset (see k_push32_run) deposits nothing: tested on the last weight, which
+            // a NaN offset (see push_run) deposits nothing: tested on the last weight, which
             // is formed anyway (256^3: 4.05 ms a step, with a sum of the offsets 4.08)
             if (!(ux[1] * uy[1] * uz[1] >= 0.0f)) continue;
 #pragma unroll
@@ -3671,8 +3682,8 @@ struct SimND {
         }
         switch (items) {
             case 1: k_push32_step<DIM, BORIS, 1, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
-            case 2: k_push32_run<DIM, BORIS, 2, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), acc); break;
-            case 4: k_push32_run<DIM, BORIS, 4, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), acc); break;
+            case 2: k_push32_run<DIM, BORIS, 2, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), b, acc); break;
+            case 4: k_push32_run<DIM, BORIS, 4, false><<<g, kThreads, 0, stream>>>(p, S, state32(S, b), b, acc); break;
             default: k_push32_step<DIM, BORIS, 8, false><<<g, kThreads, 0, stream>>>(p, S, b, acc); break;
         }
     }

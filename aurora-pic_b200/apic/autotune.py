@@ -51,9 +51,11 @@ def _cache_put(path, key, value):
 
 def by_tiles(plan):
     """True when every species of the FP32 deck is pushed by tiles: 3D, extents that are
-    multiples of 8, at least 2 particles a cell (push_items is not used then)."""
+    multiples of 8, at least 2 particles a cell, and 256 tiles, 256 x 2048 particles or 64
+    particles a cell (push_items is not used then)."""
     cells = int(np.prod(plan.n))
-    return plan.dims == 3 and all(k % 8 == 0 for k in plan.n) and all(s[3] >= 2 * cells for s in plan.species)
+    return plan.dims == 3 and all(k % 8 == 0 for k in plan.n) and all(
+        s[3] >= 2 * cells and (max(cells // 512, s[3] // 2048) >= 256 or s[3] >= 64 * cells) for s in plan.species)
 
 
 def tune_plasma(plan, precision, sort_intervals=(2, 3, 4, 6, 8, 16), push_items=(1, 2, 4, 8), steps=None, cache=None):

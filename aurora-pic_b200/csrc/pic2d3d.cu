@@ -80,6 +80,14 @@ constexpr int kTileCells = 8, kTileLog = 3;
 constexpr unsigned kTileVolume = kTileCells * kTileCells * kTileCells;
 // from 2 particles a cell: 128^3 x 2, 258 -> 243 us; 128^3 x 4, 525 -> 404; 64^3 x 12, 192 -> 150
 constexpr double kTileMinPpc = 2.0;
+// and from as many work items (one per tile, or per 2048 particles) as keep the chip busy, or
+// with so many particles a cell that the untiled push's atomics queue at the few nodes.  Step in us
+// of both species, by tiles against without: 128 items, 32^3 x 8 59 / 51, 64 x 32 x 32 x 4 62 / 51;
+// 256 items, 32^3 x 16 67 / 74, 64 x 32 x 32 x 8 69 / 70, 64 x 64 x 32 x 4 74 / 73; 512, 64^3 x 4
+// 106 / 113.  8^3 x 40 41 / 35, 16^3 x 16 54 / 37, 16^3 x 64 56 / 76, 8^3 x 200 47 / 94.
+constexpr size_t kTileMinItems = 256;
+constexpr double kTileCrowdedPpc = 64.0;
+constexpr size_t kTileMinTarget = 2048;  // particles of a work item, at least
 
 struct ParamsND {
     int dims;
@@ -3625,8 +3633,8 @@ struct SimND {
         if (tileable) {
             ntiles = (unsigned)(N / kTileVolume);
             for (int s = 0; s < c.nspecies; ++s) {
-                // at most 2 n / target + 1 items past the first of every tile, target >= 2048
-                sp[s].chunk = dalloc<uint4>(ntiles + 2 * (c.species[s].capacity / 2048) + 1);
+                // at most 2 n / target + 1 items past the first of every tile
+                sp[s].chunk = dalloc<uint4>(ntiles + 2 * (c.species[s].capacity / kTileMinTarget) + 1);
                 sp[s].extra = dalloc<unsigned>(1);
             }
             const auto allow = [](auto one, auto two) {
@@ -3647,17 +3655,19 @@ struct SimND {
 
     // Tiles: 3D meshes whose every extent holds a tile, from kTileMinPpc particles a
     // cell on average (below, filling and flushing a tile's box costs more than its
-    // particles save).
+    // particles save) and enough work items.
     unsigned ntiles = 0;
     bool tileable = false;
     bool tiles_ready[APIC_MAX_SPECIES] = {};  // sorted in tiles since its particles were loaded
     unsigned tile_target(int s) const {  // particles per work item: enough items for four waves of CTAs
-        return (unsigned)std::min<size_t>(8192, std::max<size_t>(2048, sp[s].n / (148 * 16)));
+        return (unsigned)std::min<size_t>(8192, std::max<size_t>(kTileMinTarget, sp[s].n / (148 * 16)));
     }
     unsigned tile_extra_max(int s) const { return 2 * (sp[s].n / tile_target(s)) + 1; }
     void choose_tiles(int s) {
         SpeciesND& S = sp[s];
-        S.tiled = tileable && (double)S.n >= kTileMinPpc * (double)ncells;
+        const double ppc = (double)S.n / (double)ncells;
+        const size_t items = std::max<size_t>(ntiles, S.n / kTileMinTarget);
+        S.tiled = tileable && ppc >= kTileMinPpc && (items >= kTileMinItems || ppc >= kTileCrowdedPpc);
         tiles_ready[s] = false;
     }
 

@@ -384,7 +384,8 @@ typedef struct {
     int push_items;             /* FP32 form: particles per thread of the step push, 1, 2, 4 or 8
                                    (0 = default: 4 in 2D, 2 in 3D); a tuning knob, no effect on results.
                                    Not used by 3D species that are pushed by tiles: every extent a
-                                   multiple of 8 and at least 2 particles a cell */
+                                   multiple of 8, at least 2 particles a cell, and 256 tiles of 8^3
+                                   cells, 256 x 2048 particles or 64 particles a cell */
     size_t species_sort_interval[APIC_MAX_SPECIES];  /* per species (0 = sort_interval): slow heavy
                                    species keep their cell order far longer; no effect on results */
     /* magnetic_field_profile (TabulatedVectorField1D, src/PrescribedField.cpp:89-113): B piecewise

@@ -75,13 +75,16 @@ def test_full_two_stream_deck():
 def _scaled(dims):
     if dims == 2:
         return W.plasma_2d(cells=(64, 64), ppc=64, seed=21), 8, 4
+    if dims == "3 by tiles":  # the full deck's push: 256 tiles and more, or 64 particles a cell
+        return W.plasma_3d(cells=(16, 16, 16), ppc=64, seed=23), 8, 2
     return W.plasma_3d(cells=(32, 32, 32), ppc=8, seed=23), 8, 2
 
 
-@pytest.mark.parametrize("dims", [2, 3])
+@pytest.mark.parametrize("dims", [2, 3, "3 by tiles"])
 @pytest.mark.parametrize("precision", ["fp64", "fp32"])
 def test_plasma_decks_at_benchmark_particles_per_cell(dims, precision):
     wl, sort_interval, items = _scaled(dims)
+    dims = wl.dims
     prec = apic.FP64 if precision == "fp64" else apic.FP32
     cfg = W.to_device_config_nd(wl, precision=prec, sort_interval=sort_interval)
     cfg.push_items = items

@@ -267,8 +267,8 @@ def test_fixed_swarm_alone_and_beside_a_branching_run(precision, particles, step
 
 
 def _plasma3d_run(n, count, pos, v, split, B=(0.005, 0.1, 0.2), steps=1, sort=2, weight=0.01):
-    """One electron species (tiled push), or the same particles as `split` species of
-    fewer than two a cell each (the untiled push)."""
+    """One electron species of at least 64 particles a cell (tiled push), or the same
+    particles as `split` species of fewer each (few tiles: the untiled push)."""
     length = tuple(float(k) for k in n)
     parts = np.array_split(np.arange(count), split)
     dev = apic.SimulationND(apic.config_nd(dims=3, n=n, length=length, dt=0.2, magnetic_field=B, precision=apic.FP32,
@@ -282,8 +282,8 @@ def _plasma3d_run(n, count, pos, v, split, B=(0.005, 0.1, 0.2), steps=1, sort=2,
 
 
 @pytest.mark.parametrize("steps", [1, 5])
-@pytest.mark.parametrize("n,ppc,spread", [((8, 8, 8), 4.1, 1.0), ((16, 8, 32), 7.3, 1.0), ((32, 16, 8), 5.9, 4.0),
-                                          ((8, 16, 8), 6.0, 30.0)])
+@pytest.mark.parametrize("n,ppc,spread", [((8, 8, 8), 64.1, 1.0), ((16, 8, 32), 77.3, 1.0), ((32, 16, 8), 65.9, 4.0),
+                                          ((8, 16, 8), 96.0, 30.0)])
 def test_tiled_push_gives_the_untiled_bits(n, ppc, spread, steps):
     """Gather, push and deposit through a tile's shared memory against the kernels
     without it, from thermal particles to ones that cross several tiles a step."""
@@ -303,7 +303,7 @@ def test_tiled_push_gives_the_untiled_bits(n, ppc, spread, steps):
 def test_tiled_push_with_crowded_nodes():
     """More weight on a node than one 32-bit word of a tile's box holds (and several work items
     of one tile): the charge stays exact."""
-    n, count = (16, 8, 8), 40000
+    n, count = (16, 8, 8), 70000
     rng = np.random.default_rng(3)
     pos = np.stack([rng.uniform(0.0, k, count) for k in n])
     crowd = rng.random(count) < 0.8

@@ -116,7 +116,7 @@ def test_non_finite_coordinate_between_walls(n, wall, what):
 def test_non_finite_particle_of_the_fp32_form(n, items, bad):
     """A particle of non-finite velocity deposits nothing from its first step on, in every
     kernel of the FP32 push (the last mesh goes through its tiles); the others go on."""
-    dims, count = len(n), 8 * int(np.prod(n)) + 1
+    dims, count = len(n), (8 if items else 64) * int(np.prod(n)) + 1
     rng = np.random.default_rng(3)
     dev = apic.SimulationND(apic.config_nd(
         dims=dims, n=n, length=[float(k) for k in n], dt=0.1, magnetic_field=(0.1, 0.0, 0.2), precision=apic.FP32,

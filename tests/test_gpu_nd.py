@@ -163,14 +163,15 @@ def test_fp32_energy_conservation_2d():
 
 @pytest.mark.parametrize("dims,cells,ppc,sort_interval,steps", [
     (2, (64, 64), 16, 4, 9), (3, (16, 16, 16), 8, 4, 9), (3, (32, 32, 32), 8, 1000, 30),
-    (3, (16, 16, 4), 8, 4, 9), (3, (32, 4, 32), 8, 1000, 30), (3, (32, 32, 32), 1, 4, 9)])
+    (3, (16, 16, 4), 8, 4, 9), (3, (32, 4, 32), 8, 1000, 30), (3, (32, 32, 32), 1, 4, 9),
+    (3, (8, 16, 8), 64, 4, 9), (3, (64, 64, 32), 2, 1000, 30)])
 def test_push_items_leave_results_unchanged(dims, cells, ppc, sort_interval, steps):
     """The FP32 push's particles-per-thread knob changes only speed: every
     setting (one particle per thread, the shared-memory box pushes at 2 and 4,
     8 per thread) gives the same particles and fields, also when the particles
     have drifted far from their sorted order (sorted once, 30 steps: many
-    gather and deposit outside their CTA's box).  The first two 3D decks are pushed by
-    tiles, whatever the knob; an extent of 4, or one particle a cell, is not."""
+    gather and deposit outside their CTA's box).  The last two decks are pushed by
+    tiles, whatever the knob; few tiles, an extent of 4 or one particle a cell are not."""
     plan = W.plasma_plan(dims, cells=cells, ppc=ppc, seed=4)
     ref = None
     for items in (1, 2, 4, 8):
@@ -197,7 +198,8 @@ def test_autotuner_returns_a_candidate():
     assert len(out["table"]) == 4 and all(r["ms_per_step"] > 0 for r in out["table"])
 
 
-@pytest.mark.parametrize("cells,ppc,candidates", [((16, 16, 16), 2, 1), ((16, 16, 16), 1, 2), ((16, 4, 16), 2, 2)])
+@pytest.mark.parametrize("cells,ppc,candidates", [((16, 16, 16), 64, 1), ((64, 64, 32), 2, 1), ((16, 16, 16), 2, 2),
+                                                  ((64, 64, 32), 1, 2), ((16, 4, 16), 64, 2)])
 def test_autotuner_times_each_3d_kernel_once(cells, ppc, candidates):
     """A deck pushed by tiles has no particles-per-thread setting to time."""
     from apic import autotune

@@ -2690,7 +2690,13 @@ struct DstPass {
     const Cplx* tw;                // exp(-2 pi i k / N)
     const double* eig[3];          // eigenvalues per axis and interior index
     double scale;                  // inverse normalisation (kDstSolve)
+    bool in_regs;                  // k_dst_reg
 };
+// Lines from which the register passes are taken: a CTA holds 16 of them and each thread a chain of
+// 16-point transforms, so few lines are few CTAs of long latency, where k_dst_pass spreads a line pair
+// over a CTA.  Step of runs with 2 particles a node, registers against tiles, us: 63 lines
+// (65^2) 35 / 28, 225 (129 x 17 x 17) 60 / 58, 511 (513 x 65) 41.2 / 39.5, 961 (33^3) 50 / 60.
+constexpr int kDstRegLines = 512;
 
 struct WallMesh {
     int dims, n[3];
@@ -2795,7 +2801,8 @@ __global__ void __launch_bounds__(kFftThreads) k_dst_pass(double* __restrict__ u
     }
 }
 
-// The same passes for N = R1 R2 = 64 .. 256 (33 to 129 nodes) in registers: eight
+// The same passes for N = R1 R2 = 64 .. 256 (33 to 129 nodes) in registers, for the many
+// lines of a 3D mesh (kDstRegLines; 2D meshes have at most 511): eight
 // line pairs per CTA, laid out as in k_fft_reg.  Both halves of the odd extension are read
 // from the interior values, and the transform of an odd sequence is odd, so
 // the second transform of kDstSolve starts from the first one's own positions.
@@ -2826,7 +2833,7 @@ __global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_dst_reg(double* __r
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
         if (MODE == kDstFromRho) {
-            src[c] = rho + ((size_t)(w.dims == 3 ? lb[c] + 1 : 0) * w.n[1] + (la[c] + 1)) * w.n[0] + 1;
+            src[c] = rho + ((size_t)(lb[c] + 1) * w.n[1] + (la[c] + 1)) * w.n[0] + 1;
         } else {
             src[c] = u + la[c] * f.stride_a + lb[c] * f.stride_b;
             stride = f.stride;
@@ -2847,16 +2854,7 @@ __global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_dst_reg(double* __r
         double x[2] = {a[0][j].re, a[0][j].im};
 #pragma unroll
         for (int c = 0; c < 2; ++c) {
-            if (MODE == kDstFromRho) {
-                x[c] = cells_of(x[c], w.eps, w.reps);
-                if (w.dims == 2) {  // 2D walls at their potentials; 3D walls are grounded
-                    const int e = k <= M ? k - 1 : N - k - 1;
-                    if (e == 0) x[c] += w.side[0] * w.ih2[0];
-                    if (e == M - 1) x[c] += w.side[1] * w.ih2[0];
-                    if (la[c] == 0) x[c] += w.side[2] * w.ih2[1];
-                    if (la[c] == w.n[1] - 3) x[c] += w.side[3] * w.ih2[1];
-                }
-            }
+            if (MODE == kDstFromRho) x[c] = cells_of(x[c], w.eps, w.reps);  // (3D walls are grounded)
             x[c] = zero || !in[c] ? 0.0 : (k <= M ? x[c] : -x[c]);
         }
         a[0][j] = {x[0], x[1]};
@@ -2872,9 +2870,8 @@ __global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_dst_reg(double* __r
             double g[2];
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
-                // (the last axis: la is the x index, lb the y index in 3D)
-                const double lam = __ldg(f.eig[0] + la[c]) + (w.dims == 3 ? __ldg(f.eig[1] + lb[c]) + __ldg(f.eig[2] + e)
-                                                                         : __ldg(f.eig[1] + e));
+                // (the last axis: la is the x index, lb the y index)
+                const double lam = __ldg(f.eig[0] + la[c]) + (__ldg(f.eig[1] + lb[c]) + __ldg(f.eig[2] + e));
                 g[c] = zero ? 0.0 : f.scale * __drcp_rn(lam);
             }
             a[0][j] = {-0.5 * a[0][j].im * g[0], 0.5 * a[0][j].re * g[1]};
@@ -2890,7 +2887,7 @@ __global__ void __launch_bounds__(kRegLines * R2, 48 / R2) k_dst_reg(double* __r
             if (!in[c]) continue;
             const double v = c ? 0.5 * a[0][j].re : -0.5 * a[0][j].im;
             if (MODE == kDstToPhi)
-                phi[((size_t)(w.dims == 3 ? lb[c] + 1 : 0) * w.n[1] + (la[c] + 1)) * w.n[0] + k] = v;
+                phi[((size_t)(lb[c] + 1) * w.n[1] + (la[c] + 1)) * w.n[0] + k] = v;
             else
                 u[la[c] * f.stride_a + lb[c] * f.stride_b + (k - 1) * f.stride] = v;
         }
@@ -3211,7 +3208,8 @@ struct WallSolver {
             f.tw = twiddles(2 * (M[a] + 1));
             f.scale = scale;
             for (int b = 0; b < 3; ++b) f.eig[b] = eig[b];
-            if (f.log2N >= 6 && f.log2N <= 8) continue;  // in registers: within the default limit
+            f.in_regs = dims == 3 && f.log2N >= 6 && f.log2N <= 8 && f.lines >= kDstRegLines;
+            if (f.in_regs) continue;  // within the default limit
             if (a == 0) {
                 allow_smem(k_dst_pass<kDstFromRho>, kWallSmemMax);
                 allow_smem(k_dst_pass<kDstToPhi>, kWallSmemMax);
@@ -3242,11 +3240,11 @@ struct WallSolver {
         };
         using I8 = std::integral_constant<int, 8>;
         using I16 = std::integral_constant<int, 16>;
-        switch (f.log2N) {
-            case 6: in_regs(I8{}, I8{}); return;
-            case 7: in_regs(I16{}, I8{}); return;
-            case 8: in_regs(I16{}, I16{}); return;
-            default: break;
+        if (f.in_regs) {
+            if (f.log2N == 6) in_regs(I8{}, I8{});
+            else if (f.log2N == 7) in_regs(I16{}, I8{});
+            else in_regs(I16{}, I16{});
+            return;
         }
         const unsigned g = (unsigned)((f.lines + 2 * f.T - 1) / (2 * f.T));
         k_dst_pass<MODE><<<g, kFftThreads, wall_smem(2 * (f.M + 1), f.T), stream>>>(u, w, f, rho, phi);

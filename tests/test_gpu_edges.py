@@ -158,7 +158,8 @@ def test_mixed_solve_sizes(n, axis):
     assert rel_max(E, Er) < 10 * tol
 
 
-@pytest.mark.parametrize("n", [(3, 3), (5, 3), (3, 513), (513, 9), (3, 5, 9), (17, 3, 3), (33, 65, 17), (129, 33), (9, 129, 65)])
+@pytest.mark.parametrize("n", [(3, 3), (5, 3), (3, 513), (513, 9), (3, 5, 9), (17, 3, 3), (33, 65, 17), (129, 33), (9, 129, 65),
+                               (129, 33, 65), (65, 129, 33), (33, 65, 129), (33, 33, 17)])
 def test_dirichlet_solve_sizes(n):
     """The discrete equation at every interior node: eps Laplacian(phi) = -rho."""
     rng = np.random.default_rng(sum(n))

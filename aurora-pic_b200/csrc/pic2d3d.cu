@@ -460,7 +460,7 @@ __device__ __forceinline__ void boris_uniform(double v[3], const double E[3], co
 enum : int { kNoField = 0, kUniformField = 1, kProfileField = 2 };
 
 // The FP64 step push: kick, drift, particle boundaries and CIC deposit of
-// kRunItems consecutive particles per thread.  Particles are sorted by cell,
+// ITEMS consecutive particles per thread (1, or kRunItems).  Particles are sorted by cell,
 // so the fixed-point contributions of a run of equal cells are summed in registers,
 // a run that ends inside the thread is committed with one atomic per node, and each lane's
 // last run joins a segmented sum over the lanes that end in the same cell.  The
@@ -474,6 +474,11 @@ enum : int { kNoField = 0, kUniformField = 1, kProfileField = 2 };
 // deposit's global atomics); walls, 2 x 2 M on 512 x 513, 161 -> 113 us and
 // 2 x 4.2 M on 129^3, 680 -> 490 us (these also sorted by cell now).
 constexpr int kRunItems = 2;
+// Up to this many particles each has its own thread: all of them are resident at once, and
+// two particles in a thread only lengthen its chain.  Push of both species, us a step, one
+// against two a thread: 16^3 x 4 16.5 / 21.1, 256 x 128 x 8 on the line's far side 23.0 / 23.6,
+// walls 9 x 8 x 10 15.2 / 18.3, 17^3 x 2 19.7 / 28.5, 33^3 x 2 23.3 / 29.9, 33^3 x 4 38.0 / 36.1.
+constexpr unsigned kOneItemMax = 148 * 3 * kThreads;
 
 // One buffer of the FP64 state, by kernel argument (an index into the species'
 // arrays costs every access its pointer's load).
@@ -484,18 +489,18 @@ struct State64 {
     const unsigned* live_end;
 };
 
-template <int DIM, int BKIND, bool WALLS>
+template <int DIM, int BKIND, bool WALLS, int ITEMS>
 __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsND p, SpeciesND S, State64 A) {
     constexpr int NN = DIM == 2 ? 4 : 8;
-    const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * kRunItems;
+    const unsigned first = (blockIdx.x * kThreads + threadIdx.x) * ITEMS;
     const int lane = threadIdx.x & 31;
     // whole warp past the end, or past the particles that were alive at the last sort
-    const unsigned warp_first = (blockIdx.x * kThreads + (threadIdx.x & ~31u)) * kRunItems;
+    const unsigned warp_first = (blockIdx.x * kThreads + (threadIdx.x & ~31u)) * ITEMS;
     if (warp_first >= (WALLS && A.live_end ? min(S.n, *A.live_end) : S.n)) return;
     const int nx = p.n[0], ny = p.n[1];
-    double x[kRunItems][3], v[kRunItems][3];
-    bool live[kRunItems];
-    const bool full = first + kRunItems <= S.n;
+    double x[ITEMS][3], v[ITEMS][3];
+    bool live[ITEMS];
+    const bool full = ITEMS == 2 && first + ITEMS <= S.n;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
         double2 q{0.0, 0.0}, w{0.0, 0.0};
@@ -506,11 +511,12 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsN
             if (a < DIM) q.x = A.pos[a][first];
             w.x = A.vh[a][first];
         }
-        x[0][a] = q.x; x[1][a] = q.y;
-        v[0][a] = w.x; v[1][a] = w.y;
+        x[0][a] = q.x;
+        v[0][a] = w.x;
+        if (ITEMS == 2) { x[ITEMS - 1][a] = q.y; v[ITEMS - 1][a] = w.y; }
     }
 #pragma unroll
-    for (int k = 0; k < kRunItems; ++k)
+    for (int k = 0; k < ITEMS; ++k)
         live[k] = first + k < S.n && (!WALLS || !A.alive || A.alive[first + k]);
     const unsigned kNoCell = 0xFFFFFFFFu;
     unsigned rcell = kNoCell;  // cell of the current deposit run
@@ -526,7 +532,7 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsN
         }
     };
 #pragma unroll
-    for (int k = 0; k < kRunItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         if (!live[k]) continue;
         const Axis gx = axis2<WALLS>(p, 0, x[k][0]), gy = axis2<WALLS>(p, 1, x[k][1]);
         const Axis gz = DIM == 3 ? axis2<WALLS>(p, 2, x[k][DIM - 1]) : Axis{0, 0, 0.0};
@@ -626,10 +632,10 @@ __global__ void __launch_bounds__(kThreads, DIM == 2 ? 4 : 3) k_push_run(ParamsN
     // the state back, in place
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        if (WALLS && !live[0] && !live[1]) break;  // nothing of an absorbed pair changed
+        if (WALLS && !live[0] && !live[ITEMS - 1]) break;  // nothing of absorbed particles changed
         if (full) {
-            if (a < DIM) __stcs(reinterpret_cast<double2*>(A.pos[a] + first), make_double2(x[0][a], x[1][a]));
-            __stcs(reinterpret_cast<double2*>(A.vh[a] + first), make_double2(v[0][a], v[1][a]));
+            if (a < DIM) __stcs(reinterpret_cast<double2*>(A.pos[a] + first), make_double2(x[0][a], x[ITEMS - 1][a]));
+            __stcs(reinterpret_cast<double2*>(A.vh[a] + first), make_double2(v[0][a], v[ITEMS - 1][a]));
         } else if (first < S.n) {
             if (a < DIM) A.pos[a][first] = x[0][a];
             A.vh[a][first] = v[0][a];
@@ -3750,16 +3756,21 @@ struct SimND {
             return;
         }
         if (MODE == kPushStep) {
-            const unsigned g = (S.n + kRunItems * kThreads - 1) / (kRunItems * kThreads);
+            const int items = S.n <= kOneItemMax ? 1 : kRunItems;
+            const unsigned g = (S.n + items * kThreads - 1) / (items * kThreads);
             const int kind = !boris ? kNoField : (p.prof_rows ? kProfileField : kUniformField);
             State64 A{{}, {}, S.alive[b], S.live_end};
             for (int a = 0; a < 3; ++a) { A.pos[a] = S.pos[b][a]; A.vh[a] = S.vh[b][a]; }
-            auto run = [&](auto dim, auto wall) {
-                constexpr int D = decltype(dim)::value;
+            auto launch = [&](auto dim, auto wall, auto per) {
+                constexpr int D = decltype(dim)::value, I = decltype(per)::value;
                 constexpr bool Wl = decltype(wall)::value;
-                if (kind == kNoField) k_push_run<D, kNoField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
-                else if (kind == kUniformField) k_push_run<D, kUniformField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
-                else k_push_run<D, kProfileField, Wl><<<g, kThreads, 0, stream>>>(p, S, A);
+                if (kind == kNoField) k_push_run<D, kNoField, Wl, I><<<g, kThreads, 0, stream>>>(p, S, A);
+                else if (kind == kUniformField) k_push_run<D, kUniformField, Wl, I><<<g, kThreads, 0, stream>>>(p, S, A);
+                else k_push_run<D, kProfileField, Wl, I><<<g, kThreads, 0, stream>>>(p, S, A);
+            };
+            auto run = [&](auto dim, auto wall) {
+                if (items == 1) launch(dim, wall, std::integral_constant<int, 1>{});
+                else launch(dim, wall, std::integral_constant<int, kRunItems>{});
             };
             using D2 = std::integral_constant<int, 2>;
             using D3 = std::integral_constant<int, 3>;

@@ -76,6 +76,39 @@ def test_walls_of_ragged_counts(count, sort):
         assert rel_max(x, y) < TOL
 
 
+@pytest.mark.parametrize("B", [(0.0, 0.0, 0.0), (0.1, 0.2, 0.3), "profile"])
+@pytest.mark.parametrize("n,walls", [((64, 32), None), ((64, 33), (0, 1)), ((33, 65), (1, 1)), ((32, 16, 8), None),
+                                     ((17, 33, 9), (1, 1, 1))])
+@pytest.mark.parametrize("count", [113_665, 113_920, 170_001])
+def test_two_particles_a_thread_give_the_bits_of_one(n, walls, B, count):
+    """A species of more particles than the one-a-thread push takes against the same particles
+    as two species below that (the density is one sum of integers): counts that end inside a
+    thread, a warp and a CTA, periodic and with absorbing and reflecting walls."""
+    dims = len(n)
+    length = (4.0, 2.0, 3.0)[:dims]
+    rng = np.random.default_rng(count)
+    pos, v = _particles(count, dims, length, count)
+    profile = (0, [0.0, 1.0, 4.0], rng.standard_normal((3, 3))) if B == "profile" else None
+    got = []
+    for split in (1, 2):
+        parts = np.array_split(np.arange(count), split)
+        dev = apic.SimulationND(apic.config_nd(
+            dims=dims, n=n, length=length, dt=0.05, magnetic_field=(0.0, 0.0, 0.0) if profile else B,
+            magnetic_field_profile=profile, sort_interval=3, species=[(-1.0, 1.0, 2.0 ** -12, len(i)) for i in parts],
+            walls=(walls, [0.0] * 4 if dims == 2 else None,
+                   [(1 if k % 2 else 2) if walls[k // 2] else 3 for k in range(2 * dims)]) if walls else None))
+        for k, i in enumerate(parts):
+            dev.load(k, pos[:, i], v[:, i])
+        dev.initialize()
+        dev.step(8)
+        out = [dev.particles(k) for k in range(split)]
+        got.append([np.concatenate([o[c] for o in out], axis=1) for c in range(3)] + list(dev.fields()) +
+                   ([np.concatenate([dev.alive(k) for k in range(split)])] if walls else []))
+        dev.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("nx", [3, 4, 5, 12, 37, 64, 97, 100, 127, 255, 256, 1022, 1024, 1999, 2048])
 def test_periodic_1d_solve(nx):
     """Two-step transforms (even and odd extents, squares, primes)."""

@@ -438,7 +438,7 @@ __device__ __noinline__ bool bgk_relax(uint64_t seed, unsigned idx, uint32_t ste
 // and the one that takes them, deposits the spatial collision energy, keeps the
 // electric-work ledger and applies the legacy BGK model (start and read-back
 // passes, campaign-diagnostics windows, the ledger, BGK).
-// The steady step of runs with collision models and none of these is k_pass1d_mcc.
+// The steady step of runs with collision models, many tiles and none of these is k_pass1d_mcc.
 enum : int { kPassPlain = 0, kPassDiag = 1 };
 
 template <int VDIM, bool DIRICHLET, bool F32, int KIND>
@@ -776,7 +776,7 @@ __global__ void __launch_bounds__(kThreads, KIND == kPassPlain ? kPlainBlocks<VD
     }
 }
 
-// The steady step of a run with collision models: k_pass1d's phases (synchronize
+// The steady step of a run with collision models and many tiles (choose_pass): k_pass1d's phases (synchronize
 // and first draw, collision loops of the candidates, the rest of the step) with the
 // same arithmetic.  A candidate's loop is a chain of several thousand
 // dependent instructions (about 30 us), so the pass takes as long as the tiles that
@@ -2544,7 +2544,7 @@ struct Sim1D {
     void launch_kernels(const Params1D& q, int blocks, size_t smem, size_t post_smem, unsigned post, EvPair& ev) {
         if (q.coll_acc || q.ledger || q.bgk)
             launch_dependent(k_pass1d<VDIM, DIR, F32, kPassDiag>, blocks, kThreads, smem, q);
-        else if (cfg.nmodels && q.mode == (kModeSyncMcc | kModeKickDrift | kModeDeposit))
+        else if (many_tiles && q.mode == (kModeSyncMcc | kModeKickDrift | kModeDeposit))
             launch_dependent(k_pass1d_mcc<VDIM, DIR, F32>, wave(kMccBlocks), kMccThreads, smem, q);
         else if (cfg.nmodels)
             launch_dependent(k_pass1d<VDIM, DIR, F32, kPassDiag>, blocks, kThreads, smem, q);
@@ -2743,12 +2743,32 @@ struct Sim1D {
         pending = false;
     }
 
+    // Runs with collision models take k_pass1d_mcc's small CTAs when they have many tiles: few of them
+    // finish sooner in k_pass1d, with twice the threads on each and on the mesh that every CTA
+    // loads and flushes, alone and in groups; so does a mesh of which fewer than three
+    // small CTAs fit an SM.  Step in us, k_pass1d_mcc against k_pass1d, FP64 storage form: 64 tiles (513
+    // nodes) 40 / 35, eight such runs together 53 / 49, 128 tiles (2048 nodes) 50 / 42, four 61 / 53.
+    // The other side: 130 tiles of 513 nodes, eight runs 73 / 83; 256 of 2048, four 73 / 80; 512 of
+    // 513, eight 133 / 157; past three CTAs, 4096 nodes, 1024 tiles, three runs 319 / 262.
+    static constexpr int kMccMaxNx = 3300, kMccWideNx = 1024;
+    static constexpr size_t kMccMinTiles = 81, kMccMinTilesWide = 129;
+    bool many_tiles = false;
+    void choose_pass() {
+        size_t tiles = 0;
+        for (int s = 0; s < cfg.nspecies; ++s) tiles += (range_host[s][1] + kTile - 1) / kTile;
+        const bool many = cfg.nmodels > 0 && cfg.nx <= (size_t)kMccMaxNx &&
+                          tiles >= (cfg.nx > (size_t)kMccWideNx ? kMccMinTilesWide : kMccMinTiles);
+        if (many != many_tiles) drop_graphs();
+        many_tiles = many;
+    }
+
     // The loaded particles are one contiguous range at slot 0.
-    unsigned range_host[kMaxSpecies][4];
+    unsigned range_host[kMaxSpecies][4] = {};
     void set_single_range(int s, unsigned n) {
         SpeciesDev& B = p.sp[s];
         unsigned* h = range_host[s];
         h[0] = 0; h[1] = n; h[2] = 0; h[3] = n ? 1u : 0u;
+        choose_pass();
         APIC_CUDA(cudaMemcpyAsync(B.rstart[parity], &h[0], sizeof(unsigned), cudaMemcpyHostToDevice, stream));
         APIC_CUDA(cudaMemcpyAsync(B.rcount[parity], &h[1], sizeof(unsigned), cudaMemcpyHostToDevice, stream));
         APIC_CUDA(cudaMemcpyAsync(B.rlstart[parity], &h[2], sizeof(unsigned), cudaMemcpyHostToDevice, stream));

@@ -175,6 +175,43 @@ def test_1d_heavy_wall_losses(mcc, count, leaving):
             assert rel_max(x, y) < 1e-11
 
 
+@pytest.mark.parametrize("precision", [apic.FP64, apic.FP32_STORAGE])
+@pytest.mark.parametrize("vdim", [1, 3])
+@pytest.mark.parametrize("cells,count", [(40, 40_960), (40, 41_985), (1500, 66_000), (1500, 66_561), (3299, 70_001)])
+def test_collision_passes_give_the_same_bits(cells, count, vdim, precision):
+    """Around the tiles (81, or 129 of a wide mesh) from which a discharge takes the pass of
+    small CTAs: the same run with the electric-work ledger, which always takes the other pass."""
+    from apic import workloads as W
+    from common import load_device
+    wl = W.ccp_helium(particles_per_cell=1, cells=cells, seed=4, table_rows=256, te_ev=8.0, vdim=vdim)
+    rng = np.random.default_rng(count)
+    for s in wl.species:
+        s.weight *= cells / count
+        s.capacity = count + 20_000
+        s.x = rng.uniform(0.0, wl.length, count)
+        v = s.thermal * rng.standard_normal((3, count))
+        s.v, s.vy, s.vz = v[0], *((v[1], v[2]) if vdim == 3 else (None, None))
+    got = []
+    for ledger in (False, True):
+        cfg, tabs = W.to_device_config(wl, seed=21, precision=precision)
+        dev = apic.Simulation1D(cfg, tabs)
+        load_device(dev, wl)
+        if ledger:
+            dev.enable_power_transfer()
+        dev.initialize()
+        dev.step(7)
+        t = dev.collision_totals()
+        assert t.candidates > count // 20
+        out = [np.array([t.candidates, t.null_collisions] + [c for m in t.channel_collisions for c in m])]
+        for k in range(2):
+            p, b = dev.particles(k), dev.boundary_losses(k)
+            out += [np.array([b.absorbed_left, b.absorbed_right])] + [p[c] for c in ("x", "v", "vh", "vy", "vz")]
+        got.append(out + list(dev.fields()))
+        dev.close()
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
 @pytest.mark.parametrize("n,axis", [((4, 3), 0), ((3, 4), 1), ((8, 34), 0), ((35, 16), 1), ((1024, 40), 0),
                                     ((4, 4002), 0), ((4, 4003), 0), ((4100, 8), 1)])
 def test_mixed_solve_sizes(n, axis):

@@ -4171,9 +4171,24 @@ struct SimND {
 
     // The components are separated on the device (a strided loop over the interleaved
     // field on the host took longer than 48 steps of the 256^3 deck) into
-    // the work arrays of the solve, which are free between steps.
+    // the work arrays of the solve, which are free between steps.  A small field is read in one
+    // piece and separated here: a kernel and more copies take longer (all fields of 16^2 48 against
+    // 66 us, 64^2 83 / 100, 16^3 96 / 115, 32 x 16^2 140 / 150, 128^2 the same).
+    static constexpr size_t kSmallField = 256 << 10;
     void read_fields(double* rho, double* phi, double* E) {
         const size_t N = ncells;
+        const size_t st = cfg.dims == 2 ? 2 : 4;  // doubles of E per node on the device
+        if (E && N * st * sizeof(double) <= kSmallField) {
+            sync();
+            std::vector<double> h(N * st);
+            if (rho) APIC_CUDA(cudaMemcpyAsync(rho, solver.F.rho, N * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            if (phi) APIC_CUDA(cudaMemcpyAsync(phi, solver.F.phi, N * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            APIC_CUDA(cudaMemcpyAsync(h.data(), solver.F.E, N * st * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            APIC_CUDA(cudaStreamSynchronize(stream));
+            for (int c = 0; c < cfg.dims; ++c)
+                for (size_t g = 0; g < N; ++g) E[c * N + g] = h[g * st + c];
+            return;
+        }
         std::vector<HostCopier::Job> jobs;
         if (rho) jobs.push_back({rho, solver.F.rho, N * sizeof(double)});
         if (phi) jobs.push_back({phi, solver.F.phi, N * sizeof(double)});

@@ -2758,7 +2758,9 @@ struct Sim1D {
         for (int s = 0; s < cfg.nspecies; ++s) tiles += (range_host[s][1] + kTile - 1) / kTile;
         const bool many = cfg.nmodels > 0 && cfg.nx <= (size_t)kMccMaxNx &&
                           tiles >= (cfg.nx > (size_t)kMccWideNx ? kMccMinTilesWide : kMccMinTiles);
-        if (many != many_tiles) drop_graphs();
+        if (many == many_tiles) return;
+        APIC_CUDA(cudaStreamSynchronize(stream));  // (steps of the old choice may be under way)
+        drop_graphs();
         many_tiles = many;
     }
 

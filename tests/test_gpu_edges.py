@@ -212,6 +212,42 @@ def test_collision_passes_give_the_same_bits(cells, count, vdim, precision):
         assert np.array_equal(a, b)
 
 
+def test_reloads_across_the_collision_passes():
+    """A run that is loaded again with many, few and many particles, with steps still under way,
+    is each time the run of a new handle."""
+    from apic import workloads as W
+    from common import load_device
+    wl = W.ccp_helium(particles_per_cell=1, cells=40, seed=4, table_rows=256, te_ev=8.0)
+    for s in wl.species:
+        s.capacity = 100_000
+        s.weight *= 40 / 60_000  # the deck's density at the larger counts
+
+    def load(count):
+        rng = np.random.default_rng(count)
+        for s in wl.species:
+            s.x = rng.uniform(0.0, wl.length, count)
+            s.v, s.vy, s.vz = s.thermal * rng.standard_normal((3, count))
+
+    def state(dev):
+        return [dev.particles(k)[c] for k in range(2) for c in ("x", "v", "vh", "vy", "vz")] + list(dev.fields())
+
+    cfg, tabs = W.to_device_config(wl, seed=21)
+    dev = apic.Simulation1D(cfg, tabs)
+    for count in (60_000, 1500, 60_001):
+        load(count)
+        load_device(dev, wl)
+        dev.initialize()
+        dev.step(6)
+        fresh = apic.Simulation1D(*W.to_device_config(wl, seed=21))
+        load_device(fresh, wl)
+        fresh.initialize()
+        fresh.step(6)
+        for a, b in zip(state(dev), state(fresh)):
+            assert np.array_equal(a, b)
+        dev.step(40)  # under way at the next load
+        fresh.close()
+
+
 @pytest.mark.parametrize("n,axis", [((4, 3), 0), ((3, 4), 1), ((8, 34), 0), ((35, 16), 1), ((1024, 40), 0),
                                     ((4, 4002), 0), ((4, 4003), 0), ((4100, 8), 1)])
 def test_mixed_solve_sizes(n, axis):
